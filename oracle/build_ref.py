@@ -19,7 +19,7 @@ repository's on the same inputs.
 
 Usage: python oracle/build_ref.py [reference_root]
 The checkout is the argument, else $ZKPOLY_REFERENCE_DIR, else a directory named `reference`
-beside this repository's own directory; when none exists, nothing is built.
+beside this repository's own directory; when none holds the sources, nothing is built.
 """
 import os
 import subprocess
@@ -101,7 +101,7 @@ def build_poly(failed):
 
 
 def main():
-    if not os.path.isdir(REF):
+    if not os.path.isdir(os.path.join(REF, "core", "src")):
         print("reference checkout absent; oracle/_ref not built")
         return
     os.makedirs(OUT_DIR, exist_ok=True)
