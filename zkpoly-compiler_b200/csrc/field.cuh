@@ -9,9 +9,8 @@
 // subtraction; additions and subtractions fold back into [0, 2m) with one conditional
 // correction.  `canonical()` maps [0, 2m) to [0, m) before a store.
 //
-// The multiply is word-serial CIOS with two carry chains per row (low halves, then high
-// halves) on mad.lo.cc / madc.hi.cc; the low word of the reduction row is replaced by a
-// carry test because it is zero by construction.
+// The multiply is word-serial CIOS on mad.lo.cc / madc.hi.cc pairs, which the hardware issues as
+// one wide multiply-add on an aligned register pair (see Fp::mul for how the chains are laid out).
 #pragma once
 #include <cstdint>
 
@@ -258,87 +257,126 @@ struct Fp {
     // doubling (lazy)
     ZK_DI static Fp dbl(const Fp &a) { return add(a, a); }
 
-    // CIOS Montgomery product: a, b < 2m -> a * b / R mod m in [0, 2m).  Every 32x32 multiply
-    // is emitted as a (low, high) pair on adjacent words: per row, the products of the even
-    // limbs a[0], a[2], a[4], a[6] form one carry chain over t[0..7] (their word pairs do not
-    // overlap) and the odd limbs a second chain over t[1..8]; the reduction row q * m is split
-    // the same way.  Emitting the pairs together runs 28 % faster on B200 than one chain of
-    // low halves followed by one chain of high halves per row (57.0 vs 44.6 G products/s,
-    // bit-identical results).  Bounds: with a, b < 2m < 2^255 the running sum stays below
-    // 2^288 (nine words) inside a row and below 2^256 after each shift.
+    // CIOS Montgomery product: a, b < 2m -> a * b / R mod m in [0, 2m).  The running value is
+    // kept as two accumulators, T = E + O 2^32: the products of the even limbs a[0], a[2],
+    // a[4], a[6] (and m's) land on the word pairs (0,1), (2,3), (4,5), (6,7) of E, those of the
+    // odd limbs on the same pairs of O.  A 32x32 multiply writes an aligned register pair, so
+    // every one of them accumulates in place.  Dropping T's low word after a reduction row swaps
+    // the two: O becomes the even accumulator (plus the word E[1] left over, whose carry enters
+    // the odd chain), and E[2..7] the odd one.  The carry-chain form with one accumulator over
+    // t[0..8] had its odd chain on the other pair alignment, which cost register moves: 57.3 G
+    // products/s on B200 against 68.0 for this form, 97 % of the rate at which the 128 wide and
+    // 8 low multiplies issue (mul(x, x) 57.7, sqr 77.8).  Bounds: T < 2^288 before each shift.
     ZK_DI static Fp mul(const Fp &a, const Fp &b) {
-        u32 t[9];
-        {
-            const u32 bi = b.v[0];
+        u32 e[8], o[8];
 #pragma unroll
-            for (int j = 0; j < 8; j += 2) {
-                t[j] = a.v[j] * bi;
-                t[j + 1] = __umulhi(a.v[j], bi);
-            }
-            t[8] = 0;
-            t[1] = mad_lo_cc(a.v[1], bi, t[1]);
-            t[2] = madc_hi_cc(a.v[1], bi, t[2]);
-            t[3] = madc_lo_cc(a.v[3], bi, t[3]);
-            t[4] = madc_hi_cc(a.v[3], bi, t[4]);
-            t[5] = madc_lo_cc(a.v[5], bi, t[5]);
-            t[6] = madc_hi_cc(a.v[5], bi, t[6]);
-            t[7] = madc_lo_cc(a.v[7], bi, t[7]);
-            t[8] = madc_hi(a.v[7], bi, t[8]);
-            reduce_row(t);
+        for (int j = 0; j < 8; j += 2) {
+            e[j] = a.v[j] * b.v[0];
+            e[j + 1] = __umulhi(a.v[j], b.v[0]);
+            o[j] = a.v[j + 1] * b.v[0];
+            o[j + 1] = __umulhi(a.v[j + 1], b.v[0]);
         }
+        const u32 q0 = e[0] * P::MPRIME;
+        acc_row(e, o, q0);
 #pragma unroll
         for (int i = 1; i < 8; i++) {
-            const u32 bi = b.v[i];
-            t[0] = mad_lo_cc(a.v[0], bi, t[0]);
-            t[1] = madc_hi_cc(a.v[0], bi, t[1]);
-            t[2] = madc_lo_cc(a.v[2], bi, t[2]);
-            t[3] = madc_hi_cc(a.v[2], bi, t[3]);
-            t[4] = madc_lo_cc(a.v[4], bi, t[4]);
-            t[5] = madc_hi_cc(a.v[4], bi, t[5]);
-            t[6] = madc_lo_cc(a.v[6], bi, t[6]);
-            t[7] = madc_hi_cc(a.v[6], bi, t[7]);
-            t[8] = addc(t[8], 0u);
-            t[1] = mad_lo_cc(a.v[1], bi, t[1]);
-            t[2] = madc_hi_cc(a.v[1], bi, t[2]);
-            t[3] = madc_lo_cc(a.v[3], bi, t[3]);
-            t[4] = madc_hi_cc(a.v[3], bi, t[4]);
-            t[5] = madc_lo_cc(a.v[5], bi, t[5]);
-            t[6] = madc_hi_cc(a.v[5], bi, t[6]);
-            t[7] = madc_lo_cc(a.v[7], bi, t[7]);
-            t[8] = madc_hi(a.v[7], bi, t[8]);
-            reduce_row(t);
+            shift_mul_row(e, o, a.v, b.v[i]);
+            const u32 q = e[0] * P::MPRIME;
+            acc_row(e, o, q);
         }
-        Fp r;
+        return shift_join(e, o);
+    }
+
+    // (e, o) += q m; with q = -e[0] m^-1 mod 2^32 the low word becomes zero
+    ZK_DI static void acc_row(u32 *e, u32 *o, u32 q) {
+        e[0] = mad_lo_cc(q, P::m(0), e[0]);
+        e[1] = madc_hi_cc(q, P::m(0), e[1]);
 #pragma unroll
-        for (int i = 0; i < 8; i++) r.v[i] = t[i];
+        for (int j = 2; j < 8; j += 2) {
+            e[j] = madc_lo_cc(q, P::m(j), e[j]);
+            e[j + 1] = madc_hi_cc(q, P::m(j), e[j + 1]);
+        }
+        o[7] = addc(o[7], 0u);
+        o[0] = mad_lo_cc(q, P::m(1), o[0]);
+        o[1] = madc_hi_cc(q, P::m(1), o[1]);
+        o[2] = madc_lo_cc(q, P::m(3), o[2]);
+        o[3] = madc_hi_cc(q, P::m(3), o[3]);
+        o[4] = madc_lo_cc(q, P::m(5), o[4]);
+        o[5] = madc_hi_cc(q, P::m(5), o[5]);
+        o[6] = madc_lo_cc(q, P::m(7), o[6]);
+        o[7] = madc_hi(q, P::m(7), o[7]);
+    }
+
+    // (e, o) <- (e + o 2^32) / 2^32 + a b, for e[0] = 0
+    ZK_DI static void shift_mul_row(u32 *e, u32 *o, const u32 *a, u32 b) {
+        u32 x[8], y[8];
+        x[0] = add_cc(o[0], e[1]);
+        y[0] = madc_lo_cc(a[1], b, e[2]);
+        y[1] = madc_hi_cc(a[1], b, e[3]);
+        y[2] = madc_lo_cc(a[3], b, e[4]);
+        y[3] = madc_hi_cc(a[3], b, e[5]);
+        y[4] = madc_lo_cc(a[5], b, e[6]);
+        y[5] = madc_hi_cc(a[5], b, e[7]);
+        y[6] = madc_lo_cc(a[7], b, 0u);
+        y[7] = madc_hi(a[7], b, 0u);
+        x[0] = mad_lo_cc(a[0], b, x[0]);
+        x[1] = madc_hi_cc(a[0], b, o[1]);
+#pragma unroll
+        for (int j = 2; j < 8; j += 2) {
+            x[j] = madc_lo_cc(a[j], b, o[j]);
+            x[j + 1] = madc_hi_cc(a[j], b, o[j + 1]);
+        }
+        y[7] = addc(y[7], 0u);
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            e[j] = x[j];
+            o[j] = y[j];
+        }
+    }
+
+    // (e + o 2^32) / 2^32 as one value, for e[0] = 0 and a result below 2^256
+    ZK_DI static Fp shift_join(const u32 *e, const u32 *o) {
+        Fp r;
+        r.v[0] = add_cc(o[0], e[1]);
+#pragma unroll
+        for (int j = 1; j < 7; j++) r.v[j] = addc_cc(o[j], e[j + 1]);
+        r.v[7] = addc(o[7], 0u);
         return r;
     }
 
-    // one reduction row: t += q * m with q = t[0] * m' (the low word becomes zero), then
-    // t >>= 32.  The even limbs of m pair up over t[0..7] (the low word of q * m[0] is never
-    // formed: its carry is t[0] != 0), the odd limbs over t[1..8].
-    ZK_DI static void reduce_row(u32 *t) {
-        const u32 q = t[0] * P::MPRIME;
-        add_cc(t[0], 0xffffffffu);
-        t[1] = madc_hi_cc(q, P::m(0), t[1]);
-        t[2] = madc_lo_cc(q, P::m(2), t[2]);
-        t[3] = madc_hi_cc(q, P::m(2), t[3]);
-        t[4] = madc_lo_cc(q, P::m(4), t[4]);
-        t[5] = madc_hi_cc(q, P::m(4), t[5]);
-        t[6] = madc_lo_cc(q, P::m(6), t[6]);
-        t[7] = madc_hi_cc(q, P::m(6), t[7]);
-        t[8] = addc(t[8], 0u);
-        t[1] = mad_lo_cc(q, P::m(1), t[1]);
-        t[2] = madc_hi_cc(q, P::m(1), t[2]);
-        t[3] = madc_lo_cc(q, P::m(3), t[3]);
-        t[4] = madc_hi_cc(q, P::m(3), t[4]);
-        t[5] = madc_lo_cc(q, P::m(5), t[5]);
-        t[6] = madc_hi_cc(q, P::m(5), t[6]);
-        t[7] = madc_lo_cc(q, P::m(7), t[7]);
-        t[8] = madc_hi(q, P::m(7), t[8]);
+    // t / R mod m for a 16-word t < 4m^2: the reduction rows run over the low half alone (its
+    // result is at most m), then the high half is added; below m + 4m^2 / R < 2m
+    ZK_DI static Fp redc(const u32 *t) {
+        u32 e[8], o[8];
+        const u32 q0 = t[0] * P::MPRIME;
+        e[0] = mad_lo_cc(q0, P::m(0), t[0]);
+        e[1] = madc_hi_cc(q0, P::m(0), t[1]);
 #pragma unroll
-        for (int j = 0; j < 8; j++) t[j] = t[j + 1];
-        t[8] = 0;
+        for (int j = 2; j < 8; j += 2) {
+            e[j] = madc_lo_cc(q0, P::m(j), t[j]);
+            e[j + 1] = madc_hi_cc(q0, P::m(j), t[j + 1]);
+        }
+        const u32 c = addc(0u, 0u);
+#pragma unroll
+        for (int j = 0; j < 8; j += 2) {
+            o[j] = q0 * P::m(j + 1);
+            o[j + 1] = __umulhi(q0, P::m(j + 1));
+        }
+        o[7] += c;
+#pragma unroll
+        for (int i = 1; i < 8; i++) {
+            u32 mw[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++) mw[j] = P::m(j);
+            const u32 q = (o[0] + e[1]) * P::MPRIME;
+            shift_mul_row(e, o, mw, q);
+        }
+        Fp r = shift_join(e, o);
+        r.v[0] = add_cc(r.v[0], t[8]);
+#pragma unroll
+        for (int j = 1; j < 7; j++) r.v[j] = addc_cc(r.v[j], t[8 + j]);
+        r.v[7] = addc(r.v[7], t[15]);
+        return r;
     }
 
     // ---- product by a fixed factor (Shoup's method with a truncated quotient estimate)
@@ -401,26 +439,30 @@ struct Fp {
             h[i + 1] = addc(h[i + 1], 0u);
             shoup_high_chain(h, a.v[i], ws.v, i, (i + 1) & 1, false);
         }
-        // q = h[1..8]; r = a * w + q * (2^256 - m) mod 2^256
-        u32 t[8], npv[8];
+        // q = h[1..8]; r = a * w + q * (2^256 - m) mod 2^256, accumulated by the alignment of the
+        // word pair a product lands on (even columns in e, odd in o) and joined at the end
+        u32 e[8], o[8], npv[8];
 #pragma unroll
         for (int k = 0; k < 8; k++) {
-            t[k] = 0;
+            e[k] = o[k] = 0;
             npv[k] = Q::np(k);
         }
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-            shoup_low_chain(t, a.v[i], w.v, i, 0);
-            shoup_low_chain(t, a.v[i], w.v, i, 1);
+            shoup_low_chain((i & 1) ? o : e, a.v[i], w.v, i, 0);
+            shoup_low_chain((i & 1) ? e : o, a.v[i], w.v, i, 1);
         }
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-            shoup_low_chain(t, h[i + 1], npv, i, 0);
-            shoup_low_chain(t, h[i + 1], npv, i, 1);
+            shoup_low_chain((i & 1) ? o : e, h[i + 1], npv, i, 0);
+            shoup_low_chain((i & 1) ? e : o, h[i + 1], npv, i, 1);
         }
         Fp r;
+        r.v[0] = e[0];
+        r.v[1] = add_cc(e[1], o[1]);
 #pragma unroll
-        for (int k = 0; k < 8; k++) r.v[k] = t[k];
+        for (int k = 2; k < 7; k++) r.v[k] = addc_cc(e[k], o[k]);
+        r.v[7] = addc(e[7], o[7]);
         fold<true>(r.v);
         return r;
     }
@@ -447,10 +489,50 @@ struct Fp {
         for (int k = 0; k < 8; k++) ws->v[k] = t[k];
     }
 
-    // Montgomery square.  The product routine with both operands equal: on B200 it runs faster
-    // (58.6 G/s) than a schoolbook square that forms the 28 off-diagonal products once
-    // (52.6 G/s, one low chain and one high chain per row); the results are identical.
-    ZK_DI static Fp sqr(const Fp &a) { return mul(a, a); }
+    // Montgomery square: the 28 products of distinct limbs once, doubled, the 8 squares, then
+    // the reduction rows (100 wide multiplies against mul's 128).  As in mul the products are
+    // accumulated by the alignment of the word pair they land on: a_i a_j with i + j even in e,
+    // odd in o.  77.8 G squares/s on B200, mul(a, a) 57.7 with one accumulator.
+    ZK_DI static Fp sqr(const Fp &a) {
+        u32 e[16], o[16], t[16];
+#pragma unroll
+        for (int k = 0; k < 16; k++) e[k] = o[k] = 0;
+#pragma unroll
+        for (int i = 0; i < 7; i++) {
+#pragma unroll
+            for (int par = 0; par < 2; par++) {
+                u32 *p = par ? o : e;
+                bool first = true;
+                int top = 16;  // the word after the chain, not touched by an earlier row
+#pragma unroll
+                for (int j = 1; j < 8; j++) {
+                    if (j <= i || ((i + j) & 1) != par) continue;
+                    const int c = i + j;
+                    p[c] = first ? mad_lo_cc(a.v[i], a.v[j], p[c]) : madc_lo_cc(a.v[i], a.v[j], p[c]);
+                    p[c + 1] = madc_hi_cc(a.v[i], a.v[j], p[c + 1]);
+                    first = false;
+                    top = c + 2;
+                }
+                if (!first && top < 16) p[top] = addc(p[top], 0u);
+            }
+        }
+        t[1] = o[1];
+        t[2] = add_cc(e[2], o[2]);
+#pragma unroll
+        for (int k = 3; k < 15; k++) t[k] = addc_cc(e[k], o[k]);
+        t[15] = addc(e[15], o[15]);
+#pragma unroll
+        for (int k = 15; k > 1; k--) t[k] = __funnelshift_l(t[k - 1], t[k], 1);
+        t[1] <<= 1;
+        t[0] = mad_lo_cc(a.v[0], a.v[0], 0u);
+        t[1] = madc_hi_cc(a.v[0], a.v[0], t[1]);
+#pragma unroll
+        for (int i = 1; i < 8; i++) {
+            t[2 * i] = madc_lo_cc(a.v[i], a.v[i], t[2 * i]);
+            t[2 * i + 1] = madc_hi_cc(a.v[i], a.v[i], t[2 * i + 1]);
+        }
+        return redc(t);
+    }
 
     // x in [0, 2m) is 0 mod m exactly when x == 0 or x == m
     ZK_DI bool is_zero_mod() const {

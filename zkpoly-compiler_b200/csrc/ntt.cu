@@ -486,7 +486,7 @@ constexpr size_t BR_SMEM = 2 * 8 * BR_TILE * sizeof(u32);  // 64 KiB
 // results into shared memory and writes them back permuted as bitrev_tiled_kernel does.  The
 // vector is read and written once for both steps instead of twice.
 template <u32 D, bool SH>
-__global__ void __launch_bounds__(512) ntt_last_bitrev_kernel(PassArgs a) {
+__global__ void __launch_bounds__(512, 2) ntt_last_bitrev_kernel(PassArgs a) {
     extern __shared__ u32 br_sm[];  // 2 tiles x 8 planes x BR_TILE words
     const u32 L = a.L;
     const u32 M = L - 2 * BR_T;
