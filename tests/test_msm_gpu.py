@@ -288,3 +288,23 @@ def test_msm_stage_block_shapes(zk, orc, threads):
         zk.msm.set_affine_rounds(-1)
         zk.tuner.apply_msm_blocks()
     assert lib.zkp_msm_set_block(3, 128) == 1 and lib.zkp_msm_set_block(0, 96) == 1  # refused
+
+
+@pytest.mark.parametrize("window", [3, 4, 5, 7, 9, 12])
+def test_msm_reduction_small_windows(zk, orc, window):
+    """Bucket reductions of the smallest windows, over bases that are few points repeated (so the
+    reduction adds equal, opposite and identity points) and over distinct ones."""
+    n = 700
+    p = orc.gen_points(400 + window, n)
+    s = orc.gen_fr(401 + window, n)
+    p[: n // 2] = p[np.arange(n // 2) % 3]
+    s[: n // 4] = s[np.arange(n // 4) % 2]
+    s[n // 4] = 0
+    p[n // 4 + 1] = 0
+    bases = zk.msm.ResidentBases(p, window=window)
+    res = torch.zeros(16, dtype=torch.int32, device="cuda")
+    for m in (n, 1):
+        b = bases if m == n else zk.msm.ResidentBases(p[:m], window=window)
+        dev_s = torch.from_numpy(s[:m].view(np.int32).reshape(m, 8).copy()).cuda()
+        b.msm(dev_s, res, b.workspace())
+        assert np.array_equal(res.cpu().numpy().view(np.uint64), orc.best_multiexp(s[:m], p[:m])), m

@@ -172,73 +172,85 @@ ZK_DI G1X g1_add(const G1X &a, const G1X &b) {
     return o;
 }
 
-// ------------------------------------------------------------------ warp-parallel forms
-// For a serial chain of point operations on one point (the window combination of an MSM
-// without precomputed tables: about 240 doublings), one thread pays every Fq product's full
-// latency in turn.  These forms run the same formulas with every lane of a warp holding the
-// same point: the products of one dependency level (at most four) are computed at once, one
-// per lane, and broadcast with shuffles.  A doubling then costs three product latencies
-// instead of nine, an addition four instead of fourteen; the values are the serial forms'.
-ZK_DI Fq lane_pick(u32 lane, const Fq &a0, const Fq &a1, const Fq &a2, const Fq &a3) {
+// ------------------------------------------------------------------ four lanes per point
+// A single thread pays the latency of an addition's fourteen products (a doubling's nine) one
+// after the other, about 0.45 us each when its warp has the scheduler to itself, and the
+// reduction of the buckets is made of chains of such additions on few threads.  Here four
+// neighbouring lanes (a quad) hold one XYZZ point, lane role r = lane & 3 its r-th coordinate
+// (x, y, zz, zzz, the order in memory), and compute the products of one dependency level at
+// the same time: four levels for an addition (fourteen of its sixteen product slots used),
+// three for a doubling.  The values are the serial forms'.  Every lane of the warp takes part in
+// every call.
+ZK_DI u32 quad_role() { return threadIdx.x & 3; }
+ZK_DI Fq quad_xor(const Fq &x, u32 mask) {
     Fq r;
 #pragma unroll
-    for (int w = 0; w < 8; w++) r.v[w] = lane == 1 ? a1.v[w] : lane == 2 ? a2.v[w] : lane == 3 ? a3.v[w] : a0.v[w];
+    for (int w = 0; w < 8; w++) r.v[w] = __shfl_xor_sync(0xffffffffu, x.v[w], mask);
     return r;
 }
-ZK_DI Fq lane_bcast(const Fq &x, int src) {
+// the value of the quad's lane with the given role
+ZK_DI Fq quad_get(const Fq &x, int role) {
     Fq r;
 #pragma unroll
-    for (int w = 0; w < 8; w++) r.v[w] = __shfl_sync(0xffffffffu, x.v[w], src);
+    for (int w = 0; w < 8; w++) r.v[w] = __shfl_sync(0xffffffffu, x.v[w], role, 4);
+    return r;
+}
+ZK_DI bool quad_flag(bool f, int role) { return __shfl_sync(0xffffffffu, f ? 1 : 0, role, 4) != 0; }
+ZK_DI Fq fq_select(bool c, const Fq &a, const Fq &b) {
+    Fq r;
+#pragma unroll
+    for (int w = 0; w < 8; w++) r.v[w] = c ? a.v[w] : b.v[w];
     return r;
 }
 
-// dbl-2008-s-1 with its nine products in three levels; every lane of the warp passes the same p
-ZK_DI G1X g1_dbl_warp(const G1X &p) {
-    if (p.is_identity()) return p;
-    const u32 lane = threadIdx.x & 31;
-    const Fq u = Fq::dbl(p.y);
-    // level 1: v = u^2, x2 = x^2
-    Fq t = fmul(lane_pick(lane, u, p.x, u, p.x), lane_pick(lane, u, p.x, u, p.x));
-    const Fq v = lane_bcast(t, 0), x2 = lane_bcast(t, 1);
+// dbl-2008-s-1: x2 = x^2, v = u^2 | s = x v, w = u v, zz v, m^2 | m (s - x3), w y, w zzz.  The
+// identity (zz = 0) stays the identity.
+ZK_DI Fq g1_dbl_quad(const Fq &a) {
+    const u32 role = quad_role();
+    const Fq op = fq_select(role == 1, Fq::dbl(a), a);  // u = 2y in role 1
+    const Fq t1 = fsqr(op);
+    const Fq x2 = quad_get(t1, 0), v = quad_get(t1, 1);
     const Fq m = Fq::add(Fq::dbl(x2), x2);
-    // level 2: w = u v, s = x v, m^2, zz v
-    t = fmul(lane_pick(lane, u, p.x, m, v), lane_pick(lane, v, v, m, p.zz));
-    const Fq w = lane_bcast(t, 0), sv = lane_bcast(t, 1), m2 = lane_bcast(t, 2);
-    G1X r;
-    r.zz = lane_bcast(t, 3);
-    r.x = Fq::sub(Fq::sub(m2, sv), sv);
-    // level 3: m (s - x3), w y, w zzz
-    t = fmul(lane_pick(lane, m, w, w, w), lane_pick(lane, Fq::sub(sv, r.x), p.y, p.zzz, p.zzz));
-    r.y = Fq::sub(lane_bcast(t, 0), lane_bcast(t, 1));
-    r.zzz = lane_bcast(t, 2);
-    return r;
+    const Fq t2 = fmul(fq_select(role == 3, m, op), fq_select(role == 3, m, v));
+    const Fq s = quad_get(t2, 0), w = quad_get(t2, 1);
+    const Fq x3 = Fq::sub(Fq::sub(quad_get(t2, 3), s), s);
+    const Fq t3 = fmul(fq_select(role == 0, m, a), fq_select(role == 0, Fq::sub(s, x3), w));
+    const Fq y3 = Fq::sub(quad_xor(t3, 1), t3);
+    return fq_select(role < 2, fq_select(role == 0, x3, y3), fq_select(role == 2, t2, t3));
 }
 
-// add-2008-s with its fourteen products in four levels; every lane passes the same a and b
-ZK_DI G1X g1_add_warp(const G1X &a, const G1X &b) {
-    if (a.is_identity()) return b;
-    if (b.is_identity()) return a;
-    const u32 lane = threadIdx.x & 31;
-    // level 1: u1 = x_a zz_b, u2 = x_b zz_a, s1 = y_a zzz_b, s2 = y_b zzz_a
-    Fq t = fmul(lane_pick(lane, a.x, b.x, a.y, b.y), lane_pick(lane, b.zz, a.zz, b.zzz, a.zzz));
-    const Fq u1 = lane_bcast(t, 0), u2 = lane_bcast(t, 1), s1 = lane_bcast(t, 2), s2 = lane_bcast(t, 3);
-    const Fq p = Fq::sub(u2, u1);
-    const Fq r = Fq::sub(s2, s1);
-    if (p.is_zero_mod() && r.is_zero_mod()) return g1_dbl_warp(a);
-    // level 2: pp = p^2, r^2, zz_a zz_b, zzz_a zzz_b
-    t = fmul(lane_pick(lane, p, r, a.zz, a.zzz), lane_pick(lane, p, r, b.zz, b.zzz));
-    const Fq pp = lane_bcast(t, 0), r2 = lane_bcast(t, 1), zzab = lane_bcast(t, 2), zzzab = lane_bcast(t, 3);
-    // level 3: ppp = p pp, q = u1 pp, zz = zz_a zz_b pp
-    t = fmul(lane_pick(lane, p, u1, zzab, zzab), lane_pick(lane, pp, pp, pp, pp));
-    const Fq ppp = lane_bcast(t, 0), q = lane_bcast(t, 1);
-    G1X o;
-    o.zz = lane_bcast(t, 2);
-    o.x = Fq::sub(Fq::sub(Fq::sub(r2, ppp), q), q);
-    // level 4: r (q - x3), s1 ppp, zzz_a zzz_b ppp
-    t = fmul(lane_pick(lane, r, s1, zzzab, zzzab), lane_pick(lane, Fq::sub(q, o.x), ppp, ppp, ppp));
-    o.y = Fq::sub(lane_bcast(t, 0), lane_bcast(t, 1));
-    o.zzz = lane_bcast(t, 2);
-    return o;
+// add-2008-s: u1, s1, u2, s2 | p^2, r^2, zz_a zz_b, zzz_a zzz_b | q, ppp, zz | s1 ppp,
+// r (q - x3), zzz; identities and doubling handled by selects (the doubling is only computed
+// when some quad of the warp adds equal points)
+ZK_DI Fq g1_add_quad(const Fq &a, const Fq &b) {
+    const u32 role = quad_role();
+    const bool hi = role >= 2;
+    const bool id_a = quad_flag(a.is_zero_mod(), 2), id_b = quad_flag(b.is_zero_mod(), 2);
+    const Fq t1 = fmul(a, quad_xor(b, 2));  // u1, s1, u2, s2
+    const Fq o1 = quad_xor(t1, 2);
+    const Fq d = Fq::sub(fq_select(hi, t1, o1), fq_select(hi, o1, t1));  // p, r, p, r
+    const bool dz = d.is_zero_mod();
+    const bool p_zero = quad_flag(dz, 0), r_zero = quad_flag(dz, 1);  // shuffles: outside any short circuit
+    const bool equal = p_zero && r_zero && !id_a && !id_b;
+    const Fq t2 = fmul(fq_select(hi, a, d), fq_select(hi, b, d));  // pp, r^2, zz_ab, zzz_ab
+    // q = u1 pp, ppp = p pp, zz_ab pp
+    const Fq t3 = fmul(fq_select(role == 0, t1, fq_select(role == 1, quad_xor(d, 1), t2)), quad_get(t2, 0));
+    const Fq q = quad_get(t3, 0), ppp = quad_get(t3, 1);
+    const Fq x3 = Fq::sub(Fq::sub(Fq::sub(quad_get(t2, 1), ppp), q), q);
+    // s1 ppp, r (q - x3), -, zzz_ab ppp
+    const Fq t4 = fmul(fq_select(role == 0, quad_xor(t1, 1), fq_select(role == 1, d, t2)),
+                       fq_select(role == 1, Fq::sub(q, x3), ppp));
+    const Fq y3 = Fq::sub(t4, quad_xor(t4, 1));
+    Fq r = fq_select(role < 2, fq_select(role == 0, x3, y3), fq_select(role == 2, t3, t4));
+    if (__any_sync(0xffffffffu, equal)) r = fq_select(equal, g1_dbl_quad(a), r);
+    return fq_select(id_a, b, fq_select(id_b, a, r));
+}
+
+// sum over the warp's eight quads, in quad 0
+ZK_DI Fq g1_sum_quads(Fq v) {
+#pragma unroll 1
+    for (u32 d = 4; d < 32; d <<= 1) v = g1_add_quad(v, quad_xor(v, d));
+    return v;
 }
 
 // k * p by double-and-add over the bits of a 64-bit k
@@ -267,14 +279,19 @@ ZK_DI G1X g1_mul_u64(const G1X &p, u64 k) {
 // 510 steps a = 0 and b = gcd = 1, so y^-1 = v 2^(32 * 17 - 510) = v 2^34.  The iteration counts
 // are fixed and every step is a select, so the threads of a warp never diverge.
 ZK_DI void mul_small9(const u32 *x, u32 c, u32 *r) {
-    u64 carry = 0;
+    u32 e[8], o[8];  // products of the even and odd words
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-        const u64 t = (u64)x[i] * c + carry;
-        r[i] = (u32)t;
-        carry = t >> 32;
+    for (int i = 0; i < 8; i += 2) {
+        e[i] = x[i] * c;
+        e[i + 1] = __umulhi(x[i], c);
+        o[i] = x[i + 1] * c;
+        o[i + 1] = __umulhi(x[i + 1], c);
     }
-    r[8] = (u32)carry;
+    r[0] = e[0];
+    r[1] = add_cc(e[1], o[0]);
+#pragma unroll
+    for (int i = 2; i < 8; i++) r[i] = addc_cc(e[i], o[i - 1]);
+    r[8] = addc(o[7], 0u);
 }
 ZK_DI void neg9_if(u32 *r, bool neg) {
     const u32 mask = neg ? 0xffffffffu : 0u;
@@ -431,6 +448,131 @@ ZK_DI Fp<P> inv_binary(const Fp<P> &a_mont) {
 #pragma unroll
     for (int i = 0; i < 8; i++) k.v[i] = P::invk(i);
     return F::mul(F::from_words(v), k).canonical();
+}
+
+// The same inversion on four lanes, for the places where one value is inverted and its latency is
+// what counts.  The four linear combinations of an outer iteration run one per lane: roles 0 and 1
+// hold (a, b) and form the new a and b, roles 2 and 3 hold (u, v) and form the new u and v.  Every
+// lane of the warp takes part and passes the same value.  A negative u f + v g
+// is made positive by adding m 2^30.
+template <class P>
+ZK_DI Fp<P> inv_binary_quad(const Fp<P> &a_mont) {
+    using F = Fp<P>;
+    const u32 role = threadIdx.x & 3;
+    const bool coef = role >= 2;
+    const F y = a_mont.canonical();
+    u32 x0[8], x1[8];  // a, b or u, v
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        x0[i] = coef ? (i == 0 ? 1u : 0u) : y.v[i];
+        x1[i] = coef ? 0u : P::m(i);
+    }
+#pragma unroll 1
+    for (int it = 0; it < 17; it++) {
+        u32 n = 62;
+#pragma unroll
+        for (u32 i = 0; i < 8; i++) {
+            const u32 o = x0[i] | x1[i];
+            const u32 len = o ? 32 * i + 32 - __clz(o) : 0u;
+            n = len > n ? len : n;
+        }
+        const u64 ha = ((u64)bits32_at(x0, n - 32) << 30) | (x0[0] & 0x3fffffffu);
+        const u64 hb = ((u64)bits32_at(x1, n - 32) << 30) | (x1[0] & 0x3fffffffu);
+        u64 ab = __shfl_sync(0xffffffffu, ha, 0, 4), bb = __shfl_sync(0xffffffffu, hb, 0, 4);
+        // the same 30 steps, a run of halvings at a time (the warp has one value, so nothing diverges)
+        int f0 = 1, g0 = 0, f1 = 0, g1 = 1;
+#pragma unroll 1
+        for (int left = 30;;) {
+            const u32 low = (u32)ab;
+            const int z0 = low ? __ffs(low) - 1 : 30;
+            const int z = z0 < left ? z0 : left;
+            ab >>= z;
+            f1 <<= z;
+            g1 <<= z;
+            left -= z;
+            if (left == 0) break;
+            if (ab < bb) {
+                const u64 x = ab;
+                ab = bb;
+                bb = x;
+                int y = f0;
+                f0 = f1;
+                f1 = y;
+                y = g0;
+                g0 = g1;
+                g1 = y;
+            }
+            ab -= bb;
+            f0 -= f1;
+            g0 -= g1;
+        }
+        const int f = role & 1 ? f1 : f0, g = role & 1 ? g1 : g0;
+        const u32 fa = (u32)(f < 0 ? -f : f), ga = (u32)(g < 0 ? -g : g);
+        // t = |f| x0 + |g| x1 or |f| x0 - |g| x1 by the factors' signs: s = f x0 + g x1 is t or -t
+        u32 p[9], q[9], t[9];
+        mul_small9(x0, fa, p);
+        mul_small9(x1, ga, q);
+        const u32 diff = (f < 0) != (g < 0) ? 0xffffffffu : 0u;
+        add_cc(diff, diff);  // carry in: 1 for a subtraction
+#pragma unroll
+        for (int i = 0; i < 8; i++) t[i] = addc_cc(p[i], q[i] ^ diff);
+        t[8] = addc(p[8], q[8] ^ diff);
+        const bool tneg = (t[8] >> 31) != 0;
+        const bool sneg = tneg != (f < 0);  // the sign of s
+        // rows of a and b keep |s|; rows of u and v change sign with the row of a or b they follow
+        const bool row = __shfl_xor_sync(0xffffffffu, sneg ? 1 : 0, 2) != 0;
+        const u32 flip = (coef ? (f < 0) != row : tneg) ? 0xffffffffu : 0u;
+        add_cc(flip, flip);
+#pragma unroll
+        for (int i = 0; i < 8; i++) t[i] = addc_cc(t[i] ^ flip, 0u);
+        t[8] = addc(t[8] ^ flip, 0u);
+        F r;
+        if (!coef) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) r.v[i] = (t[i] >> 30) | (t[i + 1] << 2);
+        } else {
+            const u32 neg = (t[8] >> 31) != 0 ? 0xffffffffu : 0u;
+            t[0] = add_cc(t[0], (P::m(0) << 30) & neg);
+#pragma unroll
+            for (int i = 1; i < 8; i++) t[i] = addc_cc(t[i], ((P::m(i) << 30) | (P::m(i - 1) >> 2)) & neg);
+            t[8] = addc(t[8], (P::m(7) >> 2) & neg);
+            // 0 <= t < m 2^30: (t + k m) / 2^32 < 2m with k = t (-m^-1) mod 2^32
+            const u32 k = t[0] * P::MPRIME;
+            u32 w[8], km[9];
+#pragma unroll
+            for (int i = 0; i < 8; i++) w[i] = P::m(i);
+            mul_small9(w, k, km);
+            add_cc(t[0], km[0]);
+#pragma unroll
+            for (int i = 1; i < 8; i++) r.v[i - 1] = addc_cc(t[i], km[i]);
+            r.v[7] = addc(t[8], km[8]);
+            r = r.canonical();
+        }
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            x0[i] = __shfl_sync(0xffffffffu, r.v[i], role & 2, 4);
+            x1[i] = __shfl_sync(0xffffffffu, r.v[i], (role & 2) + 1, 4);
+        }
+    }
+    // v = y^-1 2^-34, and x^-1 R = y^-1 R^2 = Montgomery product of v and 2^34 R^3
+    F v, k;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        v.v[i] = __shfl_sync(0xffffffffu, x1[i], 2, 4);
+        k.v[i] = P::invk(i);
+    }
+    const F r = F::mul(v, k).canonical();
+    return y.is_zero() ? F::zero() : r;
+}
+
+// a quad's XYZZ point normalised into out (64 bytes, affine); identity -> (0, 0)
+ZK_DI void g1_to_affine_quad(const Fq &p, u32 *out) {
+    const u32 role = quad_role();
+    const Fq zz = quad_get(p, 2);
+    const Fq a = inv_binary_quad<FqParams>(quad_get(p, 3));  // 0 for the identity
+    const Fq b = fsqr(fmul(zz, a));
+    const Fq r = fmul(p, fq_select(role == 0, b, a)).canonical();
+    if (role < 2) fq_select(zz.is_zero_mod(), Fq::zero(), r).store(out + role * 8);
 }
 
 // XYZZ -> affine (scaling-z, curve_xyzz.cuh:316-322); identity -> (0, 0)

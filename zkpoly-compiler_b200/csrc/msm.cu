@@ -27,7 +27,9 @@
 //                (summation by parts), the segment sums are split by the bits of their
 //                index into classes summed in parallel, and the classes are scaled by
 //                doublings and added.
-//   6. combine:  one thread folds the windows (c doublings each) and normalises to affine.
+//   6. combine:  one warp folds the windows (c doublings each) and normalises to affine.
+// The reduction and the fix-up are chains of dependent additions on few points; they run four lanes
+// per point (curve.cuh), which shortens an addition from fourteen products in a row to four.
 #include <cuda_runtime.h>
 #include <dlfcn.h>
 #include <atomic>
@@ -62,7 +64,7 @@ struct Task {
     u32 B;    // buckets per window = 2^(c-1)
     u32 L;    // buckets per reduction segment
     u32 gbits;  // log2(B / L): bit classes of the segment index
-    u32 parts;  // CTAs per class in the reduction
+    u32 parts;  // CTAs per class in the reduction (finish_batch)
 };
 
 // The whole batch travels as a kernel parameter (no device copy, capturable in a graph).
@@ -92,7 +94,7 @@ ZK_DI u32 find_task(const T *first, u32 ntasks, T x) {
 
 // CTAs per bit class in the bucket reduction (a power of two); scale_kernel and window_kernel
 // fold up to 32 parts and 32 classes, one per lane
-constexpr u32 MAX_PARTS = 32;
+constexpr u32 MAX_PARTS = 32, CLASS_ITEMS = 256, CLASS_CTAS = 4;
 
 inline Task make_task(u64 n, u32 c, u32 n_tables) {
     Task t{};
@@ -109,8 +111,6 @@ inline Task make_task(u64 n, u32 c, u32 n_tables) {
     if (t.B >= (1u << 19)) t.L = t.B >= (1u << 20) ? 16 : 8;
     const u32 G = t.B / t.L;
     t.gbits = 31 - __builtin_clz(G);
-    const u32 half = G / 2, per_cta = 256 * 8;  // about 8 additions per thread
-    t.parts = half / per_cta < 1 ? 1 : (half / per_cta > MAX_PARTS ? MAX_PARTS : half / per_cta);
     return t;
 }
 
@@ -166,9 +166,9 @@ inline u64 next_list_bound(u64 e, u64 nb) {
     return x < e ? x : e;
 }
 
-// fills the prefixes and the chunk size; tasks[] must be set.  rounds < 0: the library
-// setting (itself -1 = by size).
-inline void finish_batch(Batch &b, int rounds = -1) {
+// fills the prefixes and the chunk size (at least min_chunk entries: a chunk costs 280 bytes of
+// workspace); tasks[] must be set.  rounds < 0: the library setting (itself -1 = by size).
+inline void finish_batch(Batch &b, int rounds = -1, u32 min_chunk = 4) {
     b.sc_first[0] = b.key_first[0] = b.seg_first[0] = 0;
     b.win_first[0] = 0;
     b.ncls = b.nparts = 1;
@@ -180,8 +180,19 @@ inline void finish_batch(Batch &b, int rounds = -1) {
         b.seg_first[t + 1] = b.seg_first[t] + (u64)k.Wp * k.B / k.L;
         b.win_first[t + 1] = b.win_first[t] + k.Wp;
         b.ncls = b.ncls > k.gbits + 2 ? b.ncls : k.gbits + 2;
-        b.nparts = b.nparts > k.parts ? b.nparts : k.parts;
         entries += k.n * k.W;
+    }
+    // CTAs per class: as many as keep at least CLASS_ITEMS segment sums each, but about
+    // CLASS_CTAS an SM in all - a single window is bound by the length of its chains, many windows
+    // by the additions that joining more parts adds (2^12 points, one window of 2^14 buckets: 8
+    // parts 32 us, 2 parts 70; 17 such windows: 8 parts 252 us, 2 parts 219)
+    for (u32 t = 0; t < b.ntasks; t++) {
+        Task &k = b.task[t];
+        const u32 half = k.B / k.L / 2;
+        const u64 most = (u64)num_sms() * CLASS_CTAS / ((u64)b.win_first[b.ntasks] * b.ncls);
+        k.parts = 1;
+        while (k.parts < MAX_PARTS && half / (2 * k.parts) >= CLASS_ITEMS && 2 * k.parts <= most) k.parts *= 2;
+        b.nparts = b.nparts > k.parts ? b.nparts : k.parts;
     }
     if (rounds < 0) rounds = affine_rounds_setting();
     b.rounds = rounds < 0 ? auto_rounds(entries) : (u32)(rounds > (int)MAX_ROUNDS ? MAX_ROUNDS : rounds);
@@ -191,15 +202,15 @@ inline void finish_batch(Batch &b, int rounds = -1) {
     // chunk so that roughly 4 waves of 384 threads per SM cover the walk's entries
     const u64 threads = (u64)num_sms() * 384 * 4;
     u64 k = (entries + threads - 1) / threads;
-    if (k < 8) k = 8;
+    if (k < min_chunk) k = min_chunk;
     if (k > 4096) k = 4096;
     b.K = (u32)k;
 }
 
 // ------------------------------------------------------------------ workspace layout
 // Montgomery-trick tree over a round's thread totals: a CTA of TREE_CTA threads folds
-// TREE_CTA * TREE_PER values per level, so two levels and the top cover 2^36 values
-constexpr u32 TREE_CTA = 256, TREE_PER = 16;
+// TREE_CTA * TREE_PER values per level, so two levels and the top cover 2^33 values
+constexpr u32 TREE_CTA = 256, TREE_PER = 8;
 constexpr u64 TREE_SPAN = (u64)TREE_CTA * TREE_PER;
 constexpr u32 TREE_LEVELS = 3;
 
@@ -213,9 +224,9 @@ struct Layout {
     u32 rounds;
     u64 emax[MAX_ROUNDS + 1], thr[MAX_ROUNDS];
     size_t starts[MAX_ROUNDS + 1], lst_bkt[2], lst_pts[2], prefix[MAX_ROUNDS], tvals;
-    // per tree level: member prefixes, per-thread exclusive prefix / suffix products, and the
+    // per tree level: member prefixes, per thread the product of the CTA's other threads, and the
     // next level's values (the CTA products)
-    size_t tree_pre[TREE_LEVELS + 1], tree_ex[TREE_LEVELS + 1], tree_sx[TREE_LEVELS + 1], tree_dat[TREE_LEVELS + 1];
+    size_t tree_pre[TREE_LEVELS + 1], tree_es[TREE_LEVELS + 1], tree_dat[TREE_LEVELS + 1];
 };
 
 inline size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -275,13 +286,12 @@ inline Layout make_layout(const Batch &b) {
         }
         l.tvals = take(l.thr[0] * 32);
         u64 m = l.thr[0];
-        for (u32 k = 0; k <= TREE_LEVELS; k++) l.tree_pre[k] = l.tree_ex[k] = l.tree_sx[k] = l.tree_dat[k] = 0;
+        for (u32 k = 0; k <= TREE_LEVELS; k++) l.tree_pre[k] = l.tree_es[k] = l.tree_dat[k] = 0;
         for (u32 k = 0; k <= TREE_LEVELS; k++) {
             l.tree_pre[k] = take(m * 32);  // the top level uses only this one
             if (m <= TREE_SPAN) break;
             const u64 ctas = (m + TREE_SPAN - 1) / TREE_SPAN;
-            l.tree_ex[k] = take(ctas * TREE_CTA * 32);
-            l.tree_sx[k] = take(ctas * TREE_CTA * 32);
+            l.tree_es[k] = take(ctas * TREE_CTA * 32);
             m = ctas;
             l.tree_dat[k + 1] = take(m * 32);
         }
@@ -293,7 +303,9 @@ inline Layout make_layout(const Batch &b) {
     l.long_list = take((l.chunks + 1) * 4 + 4);  // long chain starts + a counter at the end
     l.chain_list = take((l.chunks + 1) * 4);     // chain starts + a counter at the end
     l.seg = take(2 * l.segs * 128);  // U_g then T_g
-    l.cls = take(l.wins * b.ncls * b.nparts * 128);
+    // class parts: in the cursors' place (last used by the pairing rounds) where they fit
+    const size_t cls_bytes = l.wins * b.ncls * b.nparts * 128;
+    l.cls = cls_bytes <= (l.nb + 1) * 4 ? l.cursor : take(cls_bytes);
     l.win = take(l.wins * 128);
     l.total = off;
     return l;
@@ -484,6 +496,38 @@ __global__ void __launch_bounds__(SCAN_BLOCK) scan_apply_kernel(const u32 *in, u
     }
 }
 
+// the whole scan in one CTA, for few counters: every warp owns a contiguous run of them, adds it up,
+// and after a scan of the warps' sums walks it again 32 counters at a time
+constexpr u32 SCAN_SMALL = 36 * SCAN_BLOCK;
+__global__ void __launch_bounds__(SCAN_BLOCK) scan_small_kernel(const u32 *in, u32 n, u32 *out, u32 *out2) {
+    __shared__ u32 sm[32];
+    const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const u32 run = ((n + 31) / 32 + 31) & ~31u;  // counters a warp
+    const u32 begin = warp * run < n ? warp * run : n, end = n - begin < run ? n : begin + run;
+    u32 s = 0;
+#pragma unroll 4
+    for (u32 i = begin + lane; i < end; i += 32) s += in[i];
+    s = __reduce_add_sync(0xffffffffu, s);
+    if (lane == 0) sm[warp] = s;
+    __syncthreads();
+    u32 carry = __reduce_add_sync(0xffffffffu, lane < warp ? sm[lane] : 0u);
+#pragma unroll 4
+    for (u32 i0 = begin; i0 < end; i0 += 32) {
+        const u32 i = i0 + lane, v = i < end ? in[i] : 0u;
+        u32 x = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const u32 y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= (u32)o) x += y;
+        }
+        if (i < end) {
+            out[i] = carry + x - v;
+            out2[i] = carry + x - v;
+        }
+        carry += __shfl_sync(0xffffffffu, x, 31);
+    }
+}
+
 // ------------------------------------------------------------------ 4: accumulation
 ZK_DI G1A fetch_point(const u32 *points, u32 code) {
     const u32 idx = code & 0x7fffffffu;
@@ -604,31 +648,52 @@ ZK_DI bool chain_member(const u32 *part_bucket, const u32 *part_flag, u64 u, u32
     return (f == 1u || f == 2u) && part_bucket[2 * u] == bucket;
 }
 
-// One thread per chain start recorded by the walk (chain_list, chain_count entries).
+// One quad per chain start recorded by the walk (chain_list, chain_count entries).
 __global__ void __launch_bounds__(256) fixup_kernel(const u32 *live, u32 K, u32 *bucket_sums, const u32 *part_pts,
                                                    const u32 *part_bucket, const u32 *part_flag,
                                                    const u32 *chain_list, const u32 *chain_count, u32 *long_list,
                                                    u32 *long_count) {
     const u64 chunks = ((u64)*live + K - 1) / K;
-    const u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= *chain_count) return;
-    const u64 t = chain_list[i];
+    const u32 count = *chain_count;
+    const u64 i = ((u64)blockIdx.x * blockDim.x + threadIdx.x) >> 2;
+    const u32 role = quad_role();
+    if ((i & ~7ull) >= count) return;  // the whole warp leaves together
+    bool active = i < count;
+    u64 t = active ? chain_list[i] : 0;
     const u64 slot = 2 * t + 1;
-    const u32 bucket = part_bucket[slot];
+    const u32 bucket = active ? part_bucket[slot] : EMPTY;
     // a chain longer than SHORT_CHAIN goes to the CTA-wide pass
     const u64 probe = t + 1 + SHORT_CHAIN;
-    if (probe < chunks && chain_member(part_bucket, part_flag, probe - 1, bucket) &&
+    if (active && probe < chunks && chain_member(part_bucket, part_flag, probe - 1, bucket) &&
         part_flag[2 * (probe - 1)] == 2u) {
-        long_list[atomicAdd(long_count, 1u)] = (u32)t;
-        return;
+        if (role == 0) long_list[atomicAdd(long_count, 1u)] = (u32)t;
+        active = false;
     }
-    G1X acc = G1X::load(part_pts + slot * 32);
-    for (u64 u = t + 1; u < chunks; u++) {
-        if (!chain_member(part_bucket, part_flag, u, bucket)) break;
-        acc = g1_add(acc, G1X::load(part_pts + 2 * u * 32));
-        if (part_flag[2 * u] == 1u) break;
+    const bool owner = active;
+    Fq acc = active ? Fq::load(part_pts + slot * 32 + role * 8) : Fq::zero();
+    for (u64 u = t + 1;; u++) {
+        active = active && u < chunks && chain_member(part_bucket, part_flag, u, bucket);
+        if (!__any_sync(0xffffffffu, active)) break;
+        const Fq v = active ? Fq::load(part_pts + 2 * u * 32 + role * 8) : Fq::zero();
+        acc = g1_add_quad(acc, v);
+        active = active && part_flag[2 * u] != 1u;
     }
-    acc.store(bucket_sums + (u64)bucket * 32);
+    if (owner) acc.store(bucket_sums + (u64)bucket * 32 + role * 8);
+}
+
+// sum over the CTA's quads (at most 8 warps); the result is in quad 0 of warp 0
+ZK_DI Fq g1_sum_cta(u32 *sm, const Fq &mine) {
+    const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    Fq v = g1_sum_quads(mine);
+    if (warps == 1) return v;
+    if (lane < 4) v.store(sm + warp * 32 + lane * 8);
+    __syncthreads();
+    if (warp == 0) {
+        v = (lane >> 2) < warps ? Fq::load(sm + (lane >> 2) * 32 + (lane & 3) * 8) : Fq::zero();
+        v = g1_sum_quads(v);
+    }
+    __syncthreads();
+    return v;
 }
 
 // one CTA per long chain (looping over the recorded list): strided partial sums, then a tree
@@ -636,33 +701,26 @@ __global__ void __launch_bounds__(128) long_chain_kernel(const u32 *live, u32 K,
                                                         const u32 *part_pts, const u32 *part_bucket,
                                                         const u32 *part_flag, const u32 *long_list,
                                                         const u32 *long_count) {
-    __shared__ u32 sm[128 * 32];
+    __shared__ __align__(16) u32 sm[4 * 32];
     const u64 chunks = ((u64)*live + K - 1) / K;
     const u32 nlong = *long_count;
+    const u32 quad = threadIdx.x >> 2, quads = blockDim.x >> 2, role = quad_role();
     for (u32 item = blockIdx.x; item < nlong; item += gridDim.x) {
         const u64 t0 = long_list[item];
         const u32 bucket = part_bucket[2 * t0 + 1];
-        G1X acc = threadIdx.x == 0 ? G1X::load(part_pts + (2 * t0 + 1) * 32) : G1X::identity();
-        // members are the contiguous chunks t0+1 .. t1; each thread takes every blockDim-th
-        for (u64 u = t0 + 1 + threadIdx.x; u < chunks; u += blockDim.x) {
-            if (!chain_member(part_bucket, part_flag, u, bucket)) break;
-            // a flag-1 head ends the chain, but threads strided past it stop at the next
+        Fq acc = quad == 0 ? Fq::load(part_pts + (2 * t0 + 1) * 32 + role * 8) : Fq::zero();
+        // members are the contiguous chunks t0+1 .. t1; each quad takes every quads-th
+        bool active = true;
+        for (u64 u = t0 + 1 + quad;; u += quads) {
+            // a flag-1 head ends the chain, but quads strided past it stop at the next
             // non-member anyway; a member after an earlier flag-1 end cannot share the bucket id
             // because bucket ids are strictly increasing along the sorted array
-            acc = g1_add(acc, G1X::load(part_pts + 2 * u * 32));
+            active = active && u < chunks && chain_member(part_bucket, part_flag, u, bucket);
+            if (!__any_sync(0xffffffffu, active)) break;
+            acc = g1_add_quad(acc, active ? Fq::load(part_pts + 2 * u * 32 + role * 8) : Fq::zero());
         }
-        acc.store(sm + threadIdx.x * 32);
-        __syncthreads();
-        for (u32 stride = blockDim.x / 2; stride > 0; stride >>= 1) {
-            if (threadIdx.x < stride) {
-                G1X a = G1X::load(sm + threadIdx.x * 32);
-                G1X b = G1X::load(sm + (threadIdx.x + stride) * 32);
-                g1_add(a, b).store(sm + threadIdx.x * 32);
-            }
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) G1X::load(sm).store(bucket_sums + (u64)bucket * 32);
-        __syncthreads();
+        const Fq sum = g1_sum_cta(sm, acc);
+        if (threadIdx.x < 4) sum.store(bucket_sums + (u64)bucket * 32 + role * 8);
     }
 }
 
@@ -833,83 +891,118 @@ __global__ void __launch_bounds__(256, 3) pair_down_kernel(const Batch b, const 
 
 // Montgomery's trick over a plain array of non-zero Fq values (the thread totals), in place.
 // A CTA takes TREE_SPAN values: thread j folds the values base + j + TREE_CTA k (k <
-// TREE_PER) into running prefixes and a product p_j; shared-memory scans give every thread the
+// TREE_PER) into running prefixes and a product p_j; shuffle scans give every thread the
 // products E_j of the threads before it and S_j of those after it, so p_j^-1 = P^-1 E_j S_j
 // with P the CTA's product.  tree_up_kernel hands P to the next level; tree_top_kernel (one
 // CTA, at most TREE_SPAN values) inverts its P once and resolves its members; tree_down_kernel
 // resolves a level's members from the inverses of its CTA products.
 
-// exclusive product scan over the CTA's threads, forward (reverse = false) or backward
-ZK_DI Fq cta_exclusive_product(const Fq &v, u32 *sm, bool reverse) {
-    const u32 j = reverse ? TREE_CTA - 1 - threadIdx.x : threadIdx.x;
-    Fq x = v;
-    for (u32 d = 1; d < TREE_CTA; d <<= 1) {
-        x.store(sm + j * 8);
-        __syncthreads();
-        const Fq y = j >= d ? Fq::load(sm + (j - d) * 8) : Fq::one();
-        __syncthreads();
-        x = fmul(x, y);
-    }
-    // x = inclusive product; shift by one
-    x.store(sm + j * 8);
-    __syncthreads();
-    const Fq r = j > 0 ? Fq::load(sm + (j - 1) * 8) : Fq::one();
-    __syncthreads();
+// exclusive product scans over the CTA's threads: e the product of the threads before, f that of
+// the threads after.  The two scans are independent, so each step's two products overlap: five
+// shuffle steps inside the warp, three over the eight warp products (every warp repeats those).
+ZK_DI Fq warp_fq(const Fq &x, u32 src) {
+    Fq r;
+#pragma unroll
+    for (int w = 0; w < 8; w++) r.v[w] = __shfl_sync(0xffffffffu, x.v[w], src);
     return r;
+}
+ZK_DI void lane_scans(Fq &x, Fq &y, u32 lane, u32 width) {
+#pragma unroll 1
+    for (u32 d = 1; d < width; d <<= 1) {
+        const Fq a = warp_fq(x, lane - d), c = warp_fq(y, lane + d);
+        const Fq xa = fmul(x, a), yc = fmul(y, c);
+        x = fq_select(lane >= d, xa, x);
+        y = fq_select(lane + d < width, yc, y);
+    }
+}
+ZK_DI void cta_exclusive_products(const Fq &v, u32 *sm, Fq &e, Fq &f) {
+    constexpr u32 W = TREE_CTA / 32;
+    const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    Fq x = v, y = v;
+    lane_scans(x, y, lane, 32);
+    if (lane == 31) x.store(sm + warp * 8);
+    __syncthreads();
+    Fq wx = lane < W ? Fq::load(sm + lane * 8) : Fq::one(), wy = wx;
+    lane_scans(wx, wy, lane, W);
+    const Fq bx = warp_fq(wx, warp - 1), by = warp_fq(wy, warp + 1);
+    const Fq px = warp_fq(x, lane - 1), py = warp_fq(y, lane + 1);
+    e = fq_select(lane > 0, px, Fq::one());
+    f = fq_select(lane < 31, py, Fq::one());
+    if (warp > 0) e = fmul(e, bx);
+    if (warp + 1 < W) f = fmul(f, by);
+    __syncthreads();
+}
+
+// thread's members base + j + TREE_CTA k (ones past the end), all loads in flight at once
+ZK_DI void tree_load(Fq *v, const u32 *vals, u64 n, u64 base) {
+#pragma unroll
+    for (u32 k = 0; k < TREE_PER; k++) {
+        const u64 i = base + threadIdx.x + (u64)k * TREE_CTA;
+        v[k] = i < n ? Fq::load(vals + i * 8) : Fq::one();
+    }
 }
 
 // thread's member fold: pre[i] = product of its earlier members, returns the product
 ZK_DI Fq tree_fold(const u32 *vals, u64 n, u64 base, u32 *pre) {
-    Fq acc = Fq::one();
-    for (u32 k = 0; k < TREE_PER; k++) {
+    Fq v[TREE_PER];
+    tree_load(v, vals, n, base);
+    Fq acc = v[0];
+#pragma unroll
+    for (u32 k = 1; k < TREE_PER; k++) {
         const u64 i = base + threadIdx.x + (u64)k * TREE_CTA;
         if (i >= n) break;
         acc.canonical().store(pre + i * 8);
-        acc = fmul(acc, Fq::load(vals + i * 8));
+        acc = fmul(acc, v[k]);
     }
     return acc;
 }
 
 // members from the inverse of the thread's product, walking backwards
 ZK_DI void tree_resolve(u32 *vals, u64 n, u64 base, const u32 *pre, Fq inv) {
-    for (u32 k = TREE_PER; k-- > 0;) {
+    Fq v[TREE_PER], p[TREE_PER];
+    tree_load(v, vals, n, base);
+    tree_load(p, pre, n, base);
+#pragma unroll
+    for (int k = (int)TREE_PER - 1; k >= 0; k--) {
         const u64 i = base + threadIdx.x + (u64)k * TREE_CTA;
         if (i >= n) continue;
-        const Fq v = Fq::load(vals + i * 8);
-        fmul(inv, Fq::load(pre + i * 8)).canonical().store(vals + i * 8);
-        inv = fmul(inv, v);
+        const Fq r = k ? fmul(inv, p[k]) : inv;
+        r.canonical().store(vals + i * 8);
+        if (k) inv = fmul(inv, v[k]);
     }
 }
 
-__global__ void __launch_bounds__(TREE_CTA) tree_up_kernel(const u32 *vals, u64 n, u32 *pre, u32 *ex, u32 *sx,
+__global__ void __launch_bounds__(TREE_CTA) tree_up_kernel(const u32 *vals, u64 n, u32 *pre, u32 *es,
                                                           u32 *tot) {
-    __shared__ __align__(16) u32 sm[TREE_CTA * 8];
+    __shared__ __align__(16) u32 sm[TREE_CTA / 32 * 8];
     const u64 base = (u64)blockIdx.x * TREE_SPAN;
     const Fq p = tree_fold(vals, n, base, pre);
-    const Fq e = cta_exclusive_product(p, sm, false);
-    const Fq f = cta_exclusive_product(p, sm, true);
+    Fq e, f;
+    cta_exclusive_products(p, sm, e, f);
     const u64 slot = (u64)blockIdx.x * TREE_CTA + threadIdx.x;
-    e.canonical().store(ex + slot * 8);
-    f.canonical().store(sx + slot * 8);
+    fmul(e, f).canonical().store(es + slot * 8);
     if (threadIdx.x == TREE_CTA - 1) fmul(e, p).canonical().store(tot + (u64)blockIdx.x * 8);
 }
 
 __global__ void __launch_bounds__(TREE_CTA) tree_top_kernel(u32 *vals, u64 n, u32 *pre) {
-    __shared__ __align__(16) u32 sm[TREE_CTA * 8];
+    __shared__ __align__(16) u32 sm[TREE_CTA / 32 * 8];
     const Fq p = tree_fold(vals, n, 0, pre);
-    const Fq e = cta_exclusive_product(p, sm, false);
-    const Fq f = cta_exclusive_product(p, sm, true);
-    if (threadIdx.x == TREE_CTA - 1) inv_binary<FqParams>(fmul(e, p)).store(sm);
+    Fq e, f;
+    cta_exclusive_products(p, sm, e, f);
+    if (threadIdx.x >= TREE_CTA - 32) {  // the last warp: its last lane has the whole product
+        const Fq inv = inv_binary_quad<FqParams>(warp_fq(fmul(e, p), 31));
+        if (threadIdx.x == TREE_CTA - 1) inv.store(sm);
+    }
     __syncthreads();
     const Fq inv_all = Fq::load(sm);
     tree_resolve(vals, n, 0, pre, fmul(inv_all, fmul(e, f)));
 }
 
-__global__ void __launch_bounds__(TREE_CTA) tree_down_kernel(u32 *vals, u64 n, const u32 *pre, const u32 *ex,
-                                                            const u32 *sx, const u32 *inv_tot) {
+__global__ void __launch_bounds__(TREE_CTA) tree_down_kernel(u32 *vals, u64 n, const u32 *pre, const u32 *es,
+                                                            const u32 *inv_tot) {
     const u64 base = (u64)blockIdx.x * TREE_SPAN;
     const u64 slot = (u64)blockIdx.x * TREE_CTA + threadIdx.x;
-    const Fq inv = fmul(Fq::load(inv_tot + (u64)blockIdx.x * 8), fmul(Fq::load(ex + slot * 8), Fq::load(sx + slot * 8)));
+    const Fq inv = fmul(Fq::load(inv_tot + (u64)blockIdx.x * 8), Fq::load(es + slot * 8));
     tree_resolve(vals, n, base, pre, inv);
 }
 
@@ -939,120 +1032,119 @@ __global__ void __launch_bounds__(128) segment_kernel(const Batch b, const u32 *
     acc.store(seg_t + s * 32);
 }
 
-// sum of the CTA's per-thread points (256 threads) into sm[0]
-ZK_DI void cta_tree_sum(u32 *sm, const G1X &mine) {
-    mine.store(sm + threadIdx.x * 32);
-    __syncthreads();
-    for (u32 stride = blockDim.x / 2; stride > 0; stride >>= 1) {
-        if (threadIdx.x < stride) {
-            G1X x = G1X::load(sm + threadIdx.x * 32);
-            G1X y = G1X::load(sm + (threadIdx.x + stride) * 32);
-            g1_add(x, y).store(sm + threadIdx.x * 32);
-        }
-        __syncthreads();
+constexpr u64 SEG_QUAD_MAX = 8192;
+// The same with two quads a segment: the even quad adds the buckets up (the running sum), the
+// odd one adds up the running sums one step behind, so a segment takes L steps of one addition
+// each instead of 2 L additions of one thread.
+__global__ void __launch_bounds__(128) segment_quad_kernel(const Batch b, const u32 *bucket_sums, u32 *seg_u,
+                                                          u32 *seg_t) {
+    const u64 total = b.seg_first[b.ntasks];
+    const u64 i = ((u64)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+    if ((i & ~3ull) >= total) return;  // the whole warp leaves together
+    const u64 s = i < total ? i : total - 1;
+    const u32 t = find_task(b.seg_first, b.ntasks, s);
+    const Task &k = b.task[t];
+    const u32 L = k.L, role = quad_role();
+    const bool odd = (threadIdx.x & 4) != 0;
+    const u32 *base = bucket_sums + (b.key_first[t] + (s - b.seg_first[t]) * L) * 32 + role * 8;
+    // segments of one warp may belong to tasks with different L
+    u32 steps = L;
+#pragma unroll
+    for (u32 d = 8; d < 32; d <<= 1) steps = max(steps, __shfl_xor_sync(0xffffffffu, steps, d));
+    Fq v = Fq::load(base + (u64)(L - 1) * 32);  // both quads start from the last bucket
+    for (u32 j = 1; j <= steps; j++) {
+        const Fq run = quad_xor(v, 4);  // the odd quad's operand: the running sum so far
+        const bool take = odd ? (j > 1 && j <= L) : j < L;
+        Fq x = Fq::zero();
+        if (take) x = odd ? run : Fq::load(base + (u64)(L - 1 - j) * 32);
+        v = g1_add_quad(v, x);
     }
+    if (i < total) v.store((odd ? seg_t : seg_u) + s * 32 + role * 8);
 }
 
 // grid (windows, classes, parts): class k < gbits sums U_g over the g with bit k set; classes
 // gbits and gbits + 1 sum T_g over the lower and upper half of g.  Each class has G/2 items,
-// split into `parts` equal ranges, one CTA each.
+// split into `parts` equal ranges, one CTA of 64 quads each.
 __global__ void __launch_bounds__(256) class_kernel(const Batch b, const u32 *seg_u, const u32 *seg_t,
                                                    u32 *cls_out) {
-    __shared__ u32 sm[256 * 32];
+    __shared__ __align__(16) u32 sm[8 * 32];
     const u32 wg = blockIdx.x, cls = blockIdx.y, part = blockIdx.z;
     const u32 t = find_task(b.win_first, b.ntasks, wg);
     const Task &k = b.task[t];
     if (cls >= k.gbits + 2 || part >= k.parts) return;  // the whole CTA leaves together
+    const u32 quad = threadIdx.x >> 2, quads = blockDim.x >> 2, role = quad_role();
     const u64 G = k.B / k.L, half = G / 2;
     const u64 seg0 = b.seg_first[t] + (u64)(wg - b.win_first[t]) * G;
     const u64 per = half / k.parts;
     const u64 m0 = (u64)part * per;
     const bool is_t = cls >= k.gbits;
-    const u32 *src = is_t ? seg_t : seg_u;
-    G1X acc = G1X::identity();
-    for (u64 m = m0 + threadIdx.x; m < m0 + per; m += blockDim.x) {
+    const u32 *src = (is_t ? seg_t : seg_u) + role * 8;
+    auto item = [&](u64 j) {
+        const u64 m = m0 + j;
         const u64 g = is_t ? m + (u64)(cls - k.gbits) * half
                            : ((m >> cls) << (cls + 1)) | (1ull << cls) | (m & ((1ull << cls) - 1));
-        acc = g1_add(acc, G1X::load(src + (seg0 + g) * 32));
-    }
-    cta_tree_sum(sm, acc);
-    if (threadIdx.x == 0) G1X::load(sm).store(cls_out + (((u64)wg * b.ncls + cls) * b.nparts + part) * 32);
+        return j < per ? Fq::load(src + (seg0 + g) * 32) : Fq::zero();
+    };
+    Fq acc = item(quad);
+    for (u64 j = quads; j < per; j += quads) acc = g1_add_quad(acc, item(j + quad));
+    acc = g1_sum_cta(sm, acc);
+    if (threadIdx.x < 4) acc.store(cls_out + (((u64)wg * b.ncls + cls) * b.nparts + part) * 32 + role * 8);
 }
 
 // Classes to window values in two launches of single warps, so that the work spreads over as
-// many SMs as there are classes.  scale_kernel, one warp per (window, class): one part per lane
-// (at most 32 parts, a power of two) summed by a shuffle tree of additions; every lane then
-// holds the class sum X_k and the warp scales it by 2^k L with warp-wide doublings (each
-// doubling's independent products side by side, g1_dbl_warp), the longest dependent chain of
-// the reduction (up to 18 doublings); the result replaces part 0 of the class.  window_kernel,
-// one warp per window: one class per lane (at most 32), summed by a shuffle tree.
-ZK_DI G1X g1x_shfl_down(const G1X &p, u32 d) {
-    G1X r;
-#pragma unroll
-    for (int w = 0; w < 8; w++) {
-        r.x.v[w] = __shfl_down_sync(0xffffffffu, p.x.v[w], d);
-        r.y.v[w] = __shfl_down_sync(0xffffffffu, p.y.v[w], d);
-        r.zz.v[w] = __shfl_down_sync(0xffffffffu, p.zz.v[w], d);
-        r.zzz.v[w] = __shfl_down_sync(0xffffffffu, p.zzz.v[w], d);
-    }
-    return r;
-}
-ZK_DI G1X g1x_bcast(const G1X &p, int src) {
-    G1X r;
-    r.x = lane_bcast(p.x, src);
-    r.y = lane_bcast(p.y, src);
-    r.zz = lane_bcast(p.zz, src);
-    r.zzz = lane_bcast(p.zzz, src);
-    return r;
-}
-
-// grid (windows, classes), 32 threads
+// many SMs as there are classes.  scale_kernel, one warp per (window, class): the parts (at most
+// 32) are summed by the warp's eight quads, then the class sum X_k is scaled by 2^k L, the
+// longest dependent chain of the reduction (up to 18 doublings); the result replaces part 0 of
+// the class.  window_kernel, one warp per window: the sum of its classes (at most 32).
 __global__ void __launch_bounds__(32) scale_kernel(const Batch b, u32 *cls_out) {
-    const u32 wg = blockIdx.x, cl = blockIdx.y, lane = threadIdx.x;
+    const u32 wg = blockIdx.x, cl = blockIdx.y, quad = threadIdx.x >> 2, role = quad_role();
     const u32 t = find_task(b.win_first, b.ntasks, wg);
     const Task &k = b.task[t];
     if (cl >= k.gbits + 2) return;  // the whole warp leaves together
     const u32 P = k.parts;
-    u32 *base = cls_out + ((u64)wg * b.ncls + cl) * b.nparts * 32;
-    G1X v = lane < P ? G1X::load(base + (u64)lane * 32) : G1X::identity();
-    for (u32 d = P >> 1; d > 0; d >>= 1) v = g1_add(v, g1x_shfl_down(v, d));
+    u32 *base = cls_out + ((u64)wg * b.ncls + cl) * b.nparts * 32 + role * 8;
+    Fq v = quad < P ? Fq::load(base + (u64)quad * 32) : Fq::zero();
+    for (u32 p = 8; p < P; p += 8) v = g1_add_quad(v, p + quad < P ? Fq::load(base + (u64)(p + quad) * 32) : Fq::zero());
+    if (P > 1) v = g1_sum_quads(v);
     if (cl < k.gbits) {
-        v = g1x_bcast(v, 0);
         const u32 dbls = cl + (31 - __clz(k.L));  // 2^cl * L
-        for (u32 i = 0; i < dbls; i++) v = g1_dbl_warp(v);
+#pragma unroll 1
+        for (u32 i = 0; i < dbls; i++) v = g1_dbl_quad(v);
     }
-    if (lane == 0) v.store(base);
+    if (quad == 0) v.store(base);
 }
 
 // one warp per physical window: the sum of its classes' scaled values
 __global__ void __launch_bounds__(32) window_kernel(const Batch b, const u32 *cls_out, u32 *win_out) {
-    const u32 wg = blockIdx.x, lane = threadIdx.x;
+    const u32 wg = blockIdx.x, quad = threadIdx.x >> 2, role = quad_role();
     const u32 t = find_task(b.win_first, b.ntasks, wg);
     const Task &k = b.task[t];
     const u32 ncls = k.gbits + 2;
-    G1X v = lane < ncls ? G1X::load(cls_out + ((u64)wg * b.ncls + lane) * b.nparts * 32) : G1X::identity();
-    const u32 span = 1u << (32 - __clz(ncls - 1));  // ncls >= 2 rounded up to a power of two
-    for (u32 d = span >> 1; d > 0; d >>= 1) v = g1_add(v, g1x_shfl_down(v, d));
-    if (lane == 0) v.store(win_out + (u64)wg * 32);
+    auto cls = [&](u32 i) {
+        return i < ncls ? Fq::load(cls_out + ((u64)wg * b.ncls + i) * b.nparts * 32 + role * 8) : Fq::zero();
+    };
+    Fq v = cls(quad);
+    for (u32 i = 8; i < ncls; i += 8) v = g1_add_quad(v, cls(i + quad));
+    v = g1_sum_quads(v);
+    if (quad == 0) v.store(win_out + (u64)wg * 32 + role * 8);
 }
 
 // ------------------------------------------------------------------ 6: window combination
 // one warp per task (one CTA of 32 threads): Horner over the physical windows (c doublings
-// each).  Without precomputed tables that is a serial chain of (Wp - 1) c doublings (240 at
-// c = 15, 17 windows), so the warp computes each doubling's and addition's independent
-// products side by side (g1_dbl_warp / g1_add_warp: 1.2 ms -> 0.4 ms at 2^22); lane 0 then
-// normalises to affine.
+// each), every quad the same point.  Without precomputed tables that is a serial chain of
+// (Wp - 1) c doublings (240 at c = 15, 17 windows).
 __global__ void __launch_bounds__(32) combine_kernel(const Batch b, const u32 *win_out) {
     const u32 t = blockIdx.x;
     if (t >= b.ntasks) return;
     const Task &k = b.task[t];
-    const u32 *w = win_out + (u64)b.win_first[t] * 32;
-    G1X acc = G1X::load(w + (u64)(k.Wp - 1) * 32);
+    const u32 *w = win_out + (u64)b.win_first[t] * 32 + quad_role() * 8;
+    Fq acc = Fq::load(w + (u64)(k.Wp - 1) * 32);
     for (int i = (int)k.Wp - 2; i >= 0; i--) {
-        for (u32 d = 0; d < k.c; d++) acc = g1_dbl_warp(acc);
-        acc = g1_add_warp(acc, G1X::load(w + (u64)i * 32));
+#pragma unroll 1
+        for (u32 d = 0; d < k.c; d++) acc = g1_dbl_quad(acc);
+        acc = g1_add_quad(acc, Fq::load(w + (u64)i * 32));
     }
-    if (threadIdx.x == 0) g1_to_affine(acc).store(k.result);
+    g1_to_affine_quad(acc, k.result);
 }
 
 __global__ void zero_results_kernel(const Batch b) {
@@ -1085,6 +1177,25 @@ inline u32 grid_for(u64 items, u32 block, u32 per_sm = 8) {
     return (u32)(b < cap ? (b == 0 ? 1 : b) : cap);
 }
 
+// Up to three 256-byte aligned regions cleared in 16-byte words (each region's last partial
+// word reaches into the padding that align_up leaves after it), and two counters.
+struct ClearList {
+    struct Region {
+        uint4 *p;
+        u64 n;
+    } r[3];
+    u32 *c0, *c1;
+};
+inline u64 clear_words(u64 u32s) { return (u32s + 3) / 4; }
+__global__ void __launch_bounds__(256) clear_kernel(const ClearList z) {
+    const u64 stride = (u64)gridDim.x * blockDim.x, t = (u64)blockIdx.x * blockDim.x + threadIdx.x;
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+        for (u64 i = t; i < z.r[k].n; i += stride) z.r[k].p[i] = make_uint4(0, 0, 0, 0);
+    if (t == 0) *z.c0 = 0;
+    if (t == 1) *z.c1 = 0;
+}
+
 // Runs a batch of MSMs whose points / scalars are on the device; `ws` holds the layout
 // regions.  Launches only: no allocation, no host copy.
 // points_ready (optional): the first kernel that reads the points (the first pairing round, or
@@ -1112,6 +1223,10 @@ cudaError_t run_batch(const Batch &b, const Layout &l, char *ws, cudaStream_t st
     auto at = [&](size_t off) { return reinterpret_cast<u32 *>(ws + off); };
     // exclusive scan of items counters in[] into out[] (and out2[])
     auto scan = [&](const u32 *in, u64 items, u32 *out, u32 *out2) -> cudaError_t {
+        if (items <= SCAN_SMALL) {
+            scan_small_kernel<<<1, SCAN_BLOCK, 0, stream>>>(in, (u32)items, out, out2);
+            return cudaGetLastError();
+        }
         const u32 nblocks = (u32)((items + SCAN_BLOCK * SCAN_ITEMS - 1) / (SCAN_BLOCK * SCAN_ITEMS));
         u32 *block_sums = at(l.scan_sums);
         scan_reduce_kernel<<<nblocks, SCAN_BLOCK, 0, stream>>>(in, items, block_sums);
@@ -1122,11 +1237,17 @@ cudaError_t run_batch(const Batch &b, const Layout &l, char *ws, cudaStream_t st
 
     StageProfiler &prof = profiler();
     prof.begin(stream);
-    ZK_TRY(cudaMemsetAsync(counts, 0, (nb + 1) * 4, stream));
-    ZK_TRY(cudaMemsetAsync(bs, 0, nb * 128, stream));
-    ZK_TRY(cudaMemsetAsync(pf, 0, l.chunks * 2 * 4, stream));
-    ZK_TRY(cudaMemsetAsync(nlong, 0, 4, stream));
-    ZK_TRY(cudaMemsetAsync(nchain, 0, 4, stream));
+    {
+        // everything the kernels below expect to be zero, in one launch
+        const ClearList z{{{reinterpret_cast<uint4 *>(counts), clear_words(nb + 1)},
+                           {reinterpret_cast<uint4 *>(bs), clear_words(nb * 32)},
+                           {reinterpret_cast<uint4 *>(pf), clear_words(l.chunks * 2)}},
+                          nlong,
+                          nchain};
+        const u64 most = z.r[1].n + z.r[2].n;
+        clear_kernel<<<grid_for(most, 256 * 4, 8), 256, 0, stream>>>(z);
+        ZK_TRY(cudaGetLastError());
+    }
     prof.mark("memset", stream);
     const u64 scalars = b.sc_first[b.ntasks];
     if (scalars) {
@@ -1183,8 +1304,7 @@ cudaError_t run_batch(const Batch &b, const Layout &l, char *ws, cudaStream_t st
                 if (L == TREE_LEVELS) return cudaErrorInvalidValue;  // beyond the laid-out levels
                 const u64 ctas = (sizes[L] + TREE_SPAN - 1) / TREE_SPAN;
                 tree_up_kernel<<<(u32)ctas, TREE_CTA, 0, stream>>>(dat[L], sizes[L], at(l.tree_pre[L]),
-                                                                   at(l.tree_ex[L]), at(l.tree_sx[L]),
-                                                                   at(l.tree_dat[L + 1]));
+                                                                   at(l.tree_es[L]), at(l.tree_dat[L + 1]));
                 ZK_TRY(cudaGetLastError());
                 dat[L + 1] = at(l.tree_dat[L + 1]);
                 sizes[L + 1] = ctas;
@@ -1194,8 +1314,7 @@ cudaError_t run_batch(const Batch &b, const Layout &l, char *ws, cudaStream_t st
             ZK_TRY(cudaGetLastError());
             for (u32 k = L; k-- > 0;) {
                 tree_down_kernel<<<(u32)sizes[k + 1], TREE_CTA, 0, stream>>>(dat[k], sizes[k], at(l.tree_pre[k]),
-                                                                             at(l.tree_ex[k]), at(l.tree_sx[k]),
-                                                                             dat[k + 1]);
+                                                                             at(l.tree_es[k]), dat[k + 1]);
                 ZK_TRY(cudaGetLastError());
             }
         }
@@ -1224,7 +1343,7 @@ cudaError_t run_batch(const Batch &b, const Layout &l, char *ws, cudaStream_t st
     }
     prof.mark("accumulate", stream);
     if (l.chunks) {
-        fixup_kernel<<<(u32)((l.chunks + 255) / 256), 256, 0, stream>>>(live, b.K, bs, pp, pb, pf, chains, nchain,
+        fixup_kernel<<<(u32)((l.chunks * 4 + 255) / 256), 256, 0, stream>>>(live, b.K, bs, pp, pb, pf, chains, nchain,
                                                                         longs, nlong);
         ZK_TRY(cudaGetLastError());
         long_chain_kernel<<<num_sms() * 2, 128, 0, stream>>>(live, b.K, bs, pp, pb, pf, longs, nlong);
@@ -1232,7 +1351,13 @@ cudaError_t run_batch(const Batch &b, const Layout &l, char *ws, cudaStream_t st
     }
     prof.mark("fixup", stream);
     if (l.segs) {
-        segment_kernel<<<(u32)((l.segs + 127) / 128), 128, 0, stream>>>(b, bs, seg, seg + l.segs * 32);
+        // two quads a segment shorten its chain (2^12 points: 53 -> 20 us); where the segments fill
+        // the GPU anyway, a thread each is faster (2^18 segments: 315 against 258 us; 32768: 84
+        // against 72)
+        if (l.segs <= SEG_QUAD_MAX)
+            segment_quad_kernel<<<(u32)((l.segs * 8 + 127) / 128), 128, 0, stream>>>(b, bs, seg, seg + l.segs * 32);
+        else
+            segment_kernel<<<(u32)((l.segs + 127) / 128), 128, 0, stream>>>(b, bs, seg, seg + l.segs * 32);
         ZK_TRY(cudaGetLastError());
     }
     prof.mark("segment", stream);
@@ -1301,14 +1426,14 @@ inline void resolve(u64 n, u32 window, u32 n_tables_hint, u32 *c, u32 *n_tables)
 }
 
 inline Batch single(const u32 *points, u32 n_tables, const u32 *scalars, u64 n, u32 c, u32 *result,
-                    int rounds = -1) {
+                    int rounds = -1, u32 min_chunk = 4) {
     Batch b{};
     b.ntasks = 1;
     b.task[0] = make_task(n, c, n_tables);
     b.task[0].points = points;
     b.task[0].scalars = scalars;
     b.task[0].result = result;
-    finish_batch(b, rounds);
+    finish_batch(b, rounds, min_chunk);
     return b;
 }
 
@@ -1738,8 +1863,9 @@ extern "C" cudaError_t zkp_msm_device_noalloc(const unsigned int *points_d, unsi
     msm::resolve(n, window, n_tables, &c, &nt);
     ZK_CHECK_ARG(c >= 2 && c <= 24 && nt >= 1);
     ZK_CHECK_ARG(n * nt < (1ull << 31));
-    // no pairing rounds: their lists would not fit the fixed scratch
-    const msm::Batch b = msm::single(points_d, nt, scalars_d, n, c, result_d, 0);
+    // no pairing rounds and no walk chunks below 8 entries: their lists and partial sums would not
+    // fit the fixed scratch
+    const msm::Batch b = msm::single(points_d, nt, scalars_d, n, c, result_d, 0, 8);
     ZK_CHECK_ARG(msm::batch_fits(b));
     const msm::Layout l = msm::make_layout(b);
     // larger problems do not fit the fixed scratch: refuse instead of overrunning it
