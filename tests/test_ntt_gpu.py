@@ -396,3 +396,23 @@ def test_coset_elementwise_prep_sizes(zk, orc, log_in, log_out):
     three = orc.to_mont(orc.int_to_limbs(3))
     want = orc.coset_ntt(a, log_out, log_out, orc.to_mont(orc.int_to_limbs(5)))
     assert np.array_equal(x.numpy_u64(), orc.vec_mul(want, np.tile(three, (n_out, 1))))
+
+
+@pytest.mark.parametrize("log_n", [10, 13, 14, 16, 17])
+def test_intt_small_tiles(zk, orc, log_n):
+    """The fused last pass over 16 x 16 tiles (and the first size above it), with the scale."""
+    a = orc.gen_fr(330 + log_n, 1 << log_n)
+    x = to_dev(zk, a)
+    zk.ntt.intt(x)
+    assert np.array_equal(x.numpy_u64(), orc.intt(a, log_n))
+
+
+@pytest.mark.parametrize("log_in,log_out", [(0, 10), (7, 10), (10, 10), (9, 12), (15, 16), (14, 17)])
+def test_coset_powers_edges(zk, orc, log_in, log_out):
+    """The coset preparation where its lanes' ladder starts: sources shorter than a warp's span, no
+    extension, and several warps and CTAs."""
+    coef = orc.gen_fr(340 + log_in, 1 << log_in)
+    g = orc.to_mont(orc.int_to_limbs(7))
+    out = zk.ScalarArray.zeros(1 << log_out)
+    zk.ntt.coset_ntt(out, to_dev(zk, coef))
+    assert np.array_equal(out.numpy_u64(), orc.coset_ntt(coef, log_in, log_out, g))

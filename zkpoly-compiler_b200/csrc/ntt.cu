@@ -259,10 +259,10 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) ntt_batch_pass_kernel(const Pa
 // per lane: lane l starts with local indices l and l + g, so the first stage is a butterfly
 // inside the lane.  Before each later stage (local bit k) the lane bit k and the register bit
 // trade places through one shuffle of one element per lane, bringing the stage's partners
-// into the same lane; after the last stage lane l holds local indices 2l and 2l + 1.  A lane
-// group works on P pencils (1 or 2); with two, they differ only in their top index bits where
-// there are any, so both use the same twiddle and a twiddle load feeds two products.  No
+// into the same lane; after the last stage lane l holds local indices 2l and 2l + 1.  No
 // shared memory and no block barrier; every element is one 32-byte sector in and out.
+// AHEAD: a stage's twiddle is loaded one stage earlier (16 more registers), for the sizes at which
+// few warps share an SM and a load's latency is as long as a product.
 // SH: the twiddle product is Shoup's (Fr::mul_shoup) from a table of (w^e plain,
 // floor(w^e 2^256 / m)) pairs, 64 bytes per root, built by shoup_table_kernel from the
 // Montgomery table; the results are the same values.
@@ -276,109 +276,105 @@ ZK_DI void lane_swap(Fr &a, Fr &b, u32 lane, u32 k) {
     if (hi) a = send; else b = send;
 }
 
-template <u32 D, u32 P, bool SH>
+// twiddle w^e: with SH also its Shoup quotient; e = 0 is left out (a product by one)
+template <bool SH>
+struct Twiddle {
+    u64 e;
+    Fr w, ws;
+    ZK_DI void load(const PassArgs &a, u64 exponent) {
+        e = exponent;
+        if (e == 0) return;
+        if (SH) {
+            w = Fr::load_nc(a.shoup + e * 16);
+            ws = Fr::load_nc(a.shoup + e * 16 + 8);
+        } else {
+            w = Fr::load_nc(a.tw + e * 8);
+        }
+    }
+    ZK_DI Fr times(const Fr &d) const { return e == 0 ? d : SH ? Fr::mul_shoup(d, w, ws) : Fr::mul(d, w); }
+};
+
+// the product with the twiddle loaded where it is used
+template <bool SH>
+ZK_DI Fr twiddle_now(const PassArgs &a, u64 e, Fr d) {
+    if (e != 0) {
+        if (SH) {
+            const Fr w = Fr::load_nc(a.shoup + e * 16), ws = Fr::load_nc(a.shoup + e * 16 + 8);
+            d = Fr::mul_shoup(d, w, ws);
+        } else {
+            d = Fr::mul(d, Fr::load_nc(a.tw + e * 8));
+        }
+    }
+    return d;
+}
+
+template <u32 D, bool SH, bool AHEAD>
 __global__ void __launch_bounds__(256) ntt_warp_pass_kernel(PassArgs a) {
     constexpr u32 g = 1u << (D - 1);  // lanes per pencil group
     const u32 lo = a.lo, L = a.L;
     const u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x;
-    const u64 grp = t >> (D - 1);
+    const u64 q = t >> (D - 1);
     const u32 l = (u32)t & (g - 1);
     const u32 lane = threadIdx.x & 31;
-    // P pencils per lane group: q = grp + j * 2^(L-D-1) (they differ in the top index bit)
-    const u64 half = 1ull << (L - D - 1);
-    const u64 cmask = (1ull << lo) - 1;
-    u64 base[P], c[P];
-#pragma unroll
-    for (u32 j = 0; j < P; j++) {
-        const u64 q = grp + (j ? half : 0);
-        c[j] = q & cmask;
-        base[j] = ((q >> lo) << (lo + D)) | c[j];
-    }
-    const bool shared_tw = P == 1 || c[0] == c[P - 1];
-    Fr x0[P], x1[P];
-#pragma unroll
-    for (u32 j = 0; j < P; j++) {
-        x0[j] = Fr::load(a.v.at(base[j] + ((u64)l << lo)));
-        x1[j] = Fr::load(a.v.at(base[j] + ((u64)(l + g) << lo)));
-    }
+    const u64 c = q & ((1ull << lo) - 1);
+    const u64 base = ((q >> lo) << (lo + D)) | c;
+    auto exponent = [&](int k) { return (((u64)(l & ((1u << k) - 1)) << lo) | c) << (L - 1 - lo - (u32)k); };
+    Twiddle<SH> tw, next;
+    if (AHEAD) tw.load(a, exponent((int)D - 1));
+    Fr x0 = Fr::load(a.v.at(base + ((u64)l << lo)));
+    Fr x1 = Fr::load(a.v.at(base + ((u64)(l + g) << lo)));
 #pragma unroll
     for (int k = (int)D - 1; k >= 0; k--) {
-        if (k < (int)D - 1) {
-#pragma unroll
-            for (u32 j = 0; j < P; j++) lane_swap(x0[j], x1[j], lane, (u32)k);
-        }
-        const u64 low = (u64)(l & ((1u << k) - 1)) << lo;
-        const u32 sh = L - 1 - lo - (u32)k;
-        Fr w, ws;
-#pragma unroll
-        for (u32 j = 0; j < P; j++) {
-            const u64 e = (low | c[j]) << sh;
-            Fr s = Fr::add(x0[j], x1[j]);
-            Fr d = Fr::sub(x0[j], x1[j]);
-            if (e != 0) {
-                if (SH) {
-                    if (j == 0 || !shared_tw) {
-                        w = Fr::load_nc(a.shoup + e * 16);
-                        ws = Fr::load_nc(a.shoup + e * 16 + 8);
-                    }
-                    d = Fr::mul_shoup(d, w, ws);
-                } else {
-                    if (j == 0 || !shared_tw) w = Fr::load_nc(a.tw + e * 8);
-                    d = Fr::mul(d, w);
-                }
-            }
-            x0[j] = s;
-            x1[j] = d;
-        }
+        if (AHEAD && k > 0) next.load(a, exponent(k - 1));
+        if (k < (int)D - 1) lane_swap(x0, x1, lane, (u32)k);
+        const Fr s = Fr::add(x0, x1);
+        Fr d = Fr::sub(x0, x1);
+        x1 = AHEAD ? tw.times(d) : twiddle_now<SH>(a, exponent(k), d);
+        x0 = s;
+        if (AHEAD) tw = next;
     }
-    const bool canon = (a.flags & F_CANON) != 0;
-    const bool postscale = (a.flags & F_POSTSCALE) != 0;
-    Fr scale;
-    if (postscale) scale = Fr::load_nc(a.scale);
-#pragma unroll
-    for (u32 j = 0; j < P; j++) {
-        Fr y0 = x0[j], y1 = x1[j];
-        if (postscale) {
-            y0 = Fr::mul(y0, scale);
-            y1 = Fr::mul(y1, scale);
-        }
-        if (canon) {
-            y0 = y0.canonical();
-            y1 = y1.canonical();
-        }
-        y0.store(a.v.at(base[j] + ((u64)(2 * l) << lo)));
-        y1.store(a.v.at(base[j] + ((u64)(2 * l + 1) << lo)));
+    if (a.flags & F_POSTSCALE) {
+        const Fr scale = Fr::load_nc(a.scale);
+        x0 = Fr::mul(x0, scale);
+        x1 = Fr::mul(x1, scale);
     }
+    if (a.flags & F_CANON) {
+        x0 = x0.canonical();
+        x1 = x1.canonical();
+    }
+    x0.store(a.v.at(base + ((u64)(2 * l) << lo)));
+    x1.store(a.v.at(base + ((u64)(2 * l + 1) << lo)));
 }
-
-#ifndef ZK_NTT_WARP_PENCILS
-#define ZK_NTT_WARP_PENCILS 1  // pencils per lane group in the register pass (1 or 2)
-#endif
 
 // CTA size of the register passes per transform size, set by the tuner through
 // zkp_ntt_set_block (0 = 128)
 std::atomic<u32> g_warp_block[29];
 
-template <u32 P, bool SH>
-cudaError_t launch_warp_pass(const PassArgs &a, cudaStream_t stream) {
-    // two elements of P pencils per thread; CTAs of 128 threads by default: at 52 registers
-    // (the Shoup variant) 9 of them fit an SM, 36 warps, against 4 CTAs of 256 (32 warps), 5 %
-    // faster.  The kernel keeps __launch_bounds__(256): with a bound of 128 the compiler takes
-    // 58 registers and the occupancy gain is gone.
-    const u64 threads = 1ull << (a.L - 1 - (P == 2 ? 1 : 0));
+// Up to this size the passes load their twiddles a stage ahead (2^10 16.6 -> 13 us, 2^14 26.7 ->
+// 18.5, 2^16 36 -> 28); above it the lost occupancy costs more (2^18 66 -> 70 us, 2^22 818 -> 853).
+constexpr u32 AHEAD_MAX_L = 17;
+
+template <bool SH, bool AHEAD>
+cudaError_t launch_warp_pass_as(const PassArgs &a, cudaStream_t stream) {
+    // two elements per thread; CTAs of 128 threads by default
+    const u64 threads = 1ull << (a.L - 1);
     const u32 tuned = a.L < 29 ? g_warp_block[a.L].load(std::memory_order_relaxed) : 0;
     const u32 want = tuned ? tuned : 128;
     const u32 block = (u32)(threads < want ? threads : want);
     const u32 grid = (u32)(threads / block);
     switch (a.D) {
-        case 1: ntt_warp_pass_kernel<1, P, SH><<<grid, block, 0, stream>>>(a); break;
-        case 2: ntt_warp_pass_kernel<2, P, SH><<<grid, block, 0, stream>>>(a); break;
-        case 3: ntt_warp_pass_kernel<3, P, SH><<<grid, block, 0, stream>>>(a); break;
-        case 4: ntt_warp_pass_kernel<4, P, SH><<<grid, block, 0, stream>>>(a); break;
-        case 5: ntt_warp_pass_kernel<5, P, SH><<<grid, block, 0, stream>>>(a); break;
-        default: ntt_warp_pass_kernel<6, P, SH><<<grid, block, 0, stream>>>(a); break;
+        case 1: ntt_warp_pass_kernel<1, SH, AHEAD><<<grid, block, 0, stream>>>(a); break;
+        case 2: ntt_warp_pass_kernel<2, SH, AHEAD><<<grid, block, 0, stream>>>(a); break;
+        case 3: ntt_warp_pass_kernel<3, SH, AHEAD><<<grid, block, 0, stream>>>(a); break;
+        case 4: ntt_warp_pass_kernel<4, SH, AHEAD><<<grid, block, 0, stream>>>(a); break;
+        case 5: ntt_warp_pass_kernel<5, SH, AHEAD><<<grid, block, 0, stream>>>(a); break;
+        default: ntt_warp_pass_kernel<6, SH, AHEAD><<<grid, block, 0, stream>>>(a); break;
     }
     return cudaGetLastError();
+}
+template <bool SH>
+cudaError_t launch_warp_pass(const PassArgs &a, cudaStream_t stream) {
+    return a.L <= AHEAD_MAX_L ? launch_warp_pass_as<SH, true>(a, stream) : launch_warp_pass_as<SH, false>(a, stream);
 }
 
 // Shoup table entry e = (w^e plain, floor(w^e 2^256 / m)) from the Montgomery table entry e
@@ -478,46 +474,54 @@ __global__ void __launch_bounds__(256) bitrev_tiled_kernel(View v, u32 L) {
 
 constexpr size_t BR_SMEM = 2 * 8 * BR_TILE * sizeof(u32);  // 64 KiB
 
-// The last register pass fused with the tiled bit reversal (L >= 2 BR_T, last digit D <= BR_T,
-// table mode).  The last pass's pencils (2^D consecutive elements, lo = 0) lie inside the rows
-// of 2^BR_T elements the tiled permutation moves, so CTA m (m <= rev m) loads the rows of tiles
-// m and rev m, runs the last pass's radix-2 stages on each row in registers (16 lanes a row,
-// two elements a lane, the register pass's lane swaps and twiddles), stores the canonical
-// results into shared memory and writes them back permuted as bitrev_tiled_kernel does.  The
-// vector is read and written once for both steps instead of twice.
-template <u32 D, bool SH>
-__global__ void __launch_bounds__(512, 2) ntt_last_bitrev_kernel(PassArgs a) {
-    extern __shared__ u32 br_sm[];  // 2 tiles x 8 planes x BR_TILE words
+// The last register pass fused with the tiled bit reversal (L >= 2 T, last digit D <= T, table
+// mode).  The last pass's pencils (2^D consecutive elements, lo = 0) lie inside the rows of 2^T
+// elements the tiled permutation moves, so CTA m (m <= rev m) loads the rows of tiles m and
+// rev m, runs the last pass's radix-2 stages on each row in registers (2^(T-1) lanes a row, two
+// elements a lane, the register pass's lane swaps and twiddles), stores the canonical results
+// into shared memory and writes them back permuted as bitrev_tiled_kernel does.  The vector is
+// read and written once for both steps instead of twice.  T = 5 moves 1 KB rows; T = 4 has four
+// times the CTAs, each with one row a lane group, which is what small transforms lack.
+template <u32 T>
+struct LastTile {
+    static constexpr u32 TILE = 1u << (2 * T);                     // elements
+    static constexpr u32 THREADS = T == 5 ? 512 : 2u << (2 * T - 1);
+    static constexpr size_t SMEM = 2 * 8 * TILE * sizeof(u32);
+};
+template <u32 D, bool SH, u32 T>
+__global__ void __launch_bounds__(LastTile<T>::THREADS, 2) ntt_last_bitrev_kernel(PassArgs a) {
+    constexpr u32 TILE = LastTile<T>::TILE, ROW = 1u << T;
+    extern __shared__ u32 br_sm[];  // 2 tiles x 8 planes x TILE words
     const u32 L = a.L;
-    const u32 M = L - 2 * BR_T;
+    const u32 M = L - 2 * T;
     const u32 m = blockIdx.x;
     const u32 mr = M ? (__brev(m) >> (32 - M)) : 0u;
     if (mr < m) return;  // the pair is handled by CTA mr
     const u32 ntile = mr == m ? 1 : 2;
     constexpr u32 g = 1u << (D - 1);             // lanes per pencil
     const u32 lane = threadIdx.x & 31;
-    const u32 u = threadIdx.x & 15;              // lane within the row
+    const u32 u = threadIdx.x & (ROW / 2 - 1);   // lane within the row
     const u32 j = u >> (D - 1), l = u & (g - 1);  // pencil within the row, lane within the pencil
     const bool postscale = (a.flags & F_POSTSCALE) != 0;
     Fr scale;
     if (postscale) scale = Fr::load_nc(a.scale);
-    for (u32 r = threadIdx.x >> 4; r < 32 * ntile; r += blockDim.x >> 4) {
-        const u32 t = r >> BR_T, ar = r & 31;    // tile, top bits of the row
-        const u64 base = ((u64)ar << (L - BR_T)) | ((u64)(t ? mr : m) << BR_T) | ((u64)j << D);
+    // whole warps leave the loop together: ROW rows are a multiple of the rows of a warp
+    for (u32 r = threadIdx.x >> (T - 1); r < ROW * ntile; r += blockDim.x >> (T - 1)) {
+        const u32 t = r >> T, ar = r & (ROW - 1);    // tile, top bits of the row
+        const u64 base = ((u64)ar << (L - T)) | ((u64)(t ? mr : m) << T) | ((u64)j << D);
+        auto exponent = [&](int k) { return (u64)(l & ((1u << k) - 1)) << (L - 1 - (u32)k); };
+        Twiddle<SH> tw, next;
+        if (T < 5) tw.load(a, exponent((int)D - 1));
         Fr x0 = Fr::load(a.v.at(base + l));
         Fr x1 = Fr::load(a.v.at(base + l + g));
 #pragma unroll
         for (int k = (int)D - 1; k >= 0; k--) {
+            if (T < 5 && k > 0) next.load(a, exponent(k - 1));  // few CTAs: hide the load (16 more registers)
             if (k < (int)D - 1) lane_swap(x0, x1, lane, (u32)k);
-            const u64 e = (u64)(l & ((1u << k) - 1)) << (L - 1 - (u32)k);
-            Fr s = Fr::add(x0, x1);
-            Fr d = Fr::sub(x0, x1);
-            if (e != 0) {
-                if (SH) d = Fr::mul_shoup(d, Fr::load_nc(a.shoup + e * 16), Fr::load_nc(a.shoup + e * 16 + 8));
-                else d = Fr::mul(d, Fr::load_nc(a.tw + e * 8));
-            }
+            const Fr s = Fr::add(x0, x1), d = Fr::sub(x0, x1);
+            x1 = T < 5 ? tw.times(d) : twiddle_now<SH>(a, exponent(k), d);
             x0 = s;
-            x1 = d;
+            if (T < 5) tw = next;
         }
         if (postscale) {
             x0 = Fr::mul(x0, scale);
@@ -526,57 +530,81 @@ __global__ void __launch_bounds__(512, 2) ntt_last_bitrev_kernel(PassArgs a) {
         x0 = x0.canonical();
         x1 = x1.canonical();
         // local outputs 2l and 2l + 1 of pencil j are row elements b0 and b0 + 1
-        u32 *tile = br_sm + t * 8 * BR_TILE;
+        u32 *tile = br_sm + t * 8 * TILE;
         const u32 b0 = (j << D) + 2 * l;
-        const u32 p0 = ar * 32 + (b0 ^ ar), p1 = ar * 32 + ((b0 + 1) ^ ar);
+        const u32 p0 = ar * ROW + (b0 ^ ar), p1 = ar * ROW + ((b0 + 1) ^ ar);
 #pragma unroll
         for (int w = 0; w < 8; w++) {
-            tile[w * BR_TILE + p0] = x0.v[w];
-            tile[w * BR_TILE + p1] = x1.v[w];
+            tile[w * TILE + p0] = x0.v[w];
+            tile[w * TILE + p1] = x1.v[w];
         }
     }
     __syncthreads();
-    const u32 warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-    for (u32 t = 0; t < ntile; t++) {
-        const u32 *src = br_sm + (ntile == 2 ? 1 - t : 0) * 8 * BR_TILE;
-        for (u32 ao = warp; ao < 32; ao += nwarp) {
-            const u32 ra = __brev(lane) >> 27, rb = __brev(ao) >> 27;
-            const u32 pos = ra * 32 + (rb ^ ra);
-            Fr x;
+    for (u32 i = threadIdx.x; i < ntile * TILE; i += blockDim.x) {
+        // element (ao, b) of the destination tile t = element (rev b, rev ao) of the other tile
+        const u32 t = i >> (2 * T), ao = (i >> T) & (ROW - 1), b = i & (ROW - 1);
+        const u32 *src = br_sm + (ntile == 2 ? 1 - t : 0) * 8 * TILE;
+        const u32 ra = __brev(b) >> (32 - T), rb = __brev(ao) >> (32 - T);
+        const u32 pos = ra * ROW + (rb ^ ra);
+        Fr x;
 #pragma unroll
-            for (int w = 0; w < 8; w++) x.v[w] = src[w * BR_TILE + pos];
-            const u64 i = ((u64)ao << (L - BR_T)) | ((u64)(t ? mr : m) << BR_T) | lane;
-            x.store(a.v.at(i));
-        }
+        for (int w = 0; w < 8; w++) x.v[w] = src[w * TILE + pos];
+        x.store(a.v.at(((u64)ao << (L - T)) | ((u64)(t ? mr : m) << T) | b));
     }
 }
 
-// Coset preparation for large table-mode transforms: v[i] = x[i] * shift^i, with x the source view (zero
-// beyond src_len: the zero-extension of a coset LDE) or v itself, so that the transform then
-// runs the tuned register passes; folding the shift into a shared-memory first pass (which must
-// build per-pencil shift tables) made a 2^22 -> 2^24 coset LDE 5.9 ms against 3.4 ms for the
+// Coset preparation for multi-pass table-mode transforms: v[i] = x[i] * shift^i, with x the
+// source view (zero beyond src_len: the zero-extension of a coset LDE) or v itself, so that the
+// transform then runs its plain passes; folding the shift into a shared-memory first pass, which
+// must build per-pencil shift tables, made a 2^22 -> 2^24 coset LDE 5.9 ms against 3.4 ms for the
 // plain transform.  Warp w owns elements [w * 32 C, (w + 1) * 32 C) and lane l the elements
-// base + l + 32 k: it raises the shift to base + l once (square-and-multiply) and then steps by
-// shift^32, so a carried element costs two products and every access is coalesced.
-constexpr u32 PREP_C = 64;
-// From this size the separate pass wins (2^20 -> 2^22: 0.98 against 1.40 ms; 2^22 -> 2^24: 3.80
-// against 5.89 ms); below it the shifted wide first pass is faster (2^14 -> 2^16: 0.16 against
-// 0.18 ms)
-constexpr u32 PREP_MIN_L = 20;
+// base + l + 32 k, so every access is coalesced; a lane steps by shift^32, and a carried element
+// costs two products.  The powers shift^(2^b) come from one warp of the CTA (lane b squares b
+// times: L products deep, against 2 L for a square-and-multiply in every lane), shift^base is
+// their product over the set bits of base by five shuffle steps, and the lane's own five bits
+// take five more.
+constexpr u32 PREP_MAX_C = 64, PREP_MIN_C = 4;
+// From this size the separate pass and the register passes are faster than the shifted wide first
+// pass (4 x extension to 2^11: 36 against 64 us, to 2^14 43 against 129, to 2^17 68 against 142)
+constexpr u32 PREP_MIN_L = 10;
+ZK_DI Fr fr_xor(const Fr &x, u32 mask) {
+    Fr r;
+#pragma unroll
+    for (int w = 0; w < 8; w++) r.v[w] = __shfl_xor_sync(0xffffffffu, x.v[w], mask);
+    return r;
+}
 __global__ void __launch_bounds__(256) coset_prep_kernel(View v, View src, u64 src_len, bool has_src,
-                                                         const u32 *shift, u64 n) {
+                                                         const u32 *shift, u64 n, u32 C, u32 bits) {
+    __shared__ __align__(16) u32 ladder[32 * 8];  // shift^(2^b)
     const u64 warp = ((u64)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const u32 lane = threadIdx.x & 31;
-    const u64 base = warp * 32 * PREP_C;
-    if (base >= n) return;
+    const u64 base = warp * 32 * C;
     const u64 live = has_src ? (src_len < n ? src_len : n) : n;  // elements that carry a value
     Fr s, step;
-    if (shift && base < live) {
-        const Fr g = Fr::load(shift);
-        s = Fr::pow_u64(g, base + lane);
-        step = Fr::pow_u64(g, 32);
+    if (shift && (u64)blockIdx.x * blockDim.x * C < live) {  // the whole CTA
+        if (threadIdx.x < 32) {
+            Fr x = Fr::load(shift);
+#pragma unroll 1
+            for (u32 b = 0; b < bits; b++) {
+                const Fr y = Fr::sqr(x);
+#pragma unroll
+                for (int w = 0; w < 8; w++) x.v[w] = lane > b ? y.v[w] : x.v[w];
+            }
+            x.store(ladder + lane * 8);
+        }
+        __syncthreads();
+        s = (base >> lane) & 1 ? Fr::load(ladder + lane * 8) : Fr::one();
+#pragma unroll 1
+        for (u32 d = 1; d < 32; d <<= 1) s = Fr::mul(s, fr_xor(s, d));
+#pragma unroll 1
+        for (u32 b = 0; b < 5; b++) {
+            const Fr y = Fr::mul(s, Fr::load(ladder + b * 8));
+#pragma unroll
+            for (int w = 0; w < 8; w++) s.v[w] = (lane >> b) & 1 ? y.v[w] : s.v[w];
+        }
+        step = Fr::load(ladder + 5 * 8);
     }
-    for (u32 k = 0; k < PREP_C; k++) {
+    for (u32 k = 0; k < C; k++) {
         const u64 i = base + lane + 32ull * k;
         if (i >= n) break;
         Fr x = Fr::zero();
@@ -647,6 +675,11 @@ inline void split_digits(Plan &p, u32 first, u32 L, u32 cap) {
     p.np = first + np;
 }
 
+// The tile of the fused last pass: 16 x 16 elements for transforms of these sizes (more CTAs, and
+// one row per lane group: 2^16 36 -> 31 us, with its last pass 25 -> 14), 32 x 32 above (2^18 66 us
+// with the large tile).
+constexpr u32 SMALL_TILE = 4, SMALL_TILE_MIN_L = 10, SMALL_TILE_MAX_L = 17;
+
 // Plan for 2^L elements.  The tuned digit cap applies to plain table-mode transforms.  A
 // transform whose first pass multiplies by a coset shift or reads a shorter source keeps that
 // pass at up to MAX_D bits: the first pass builds per-pencil shift tables, and the cost of
@@ -655,6 +688,15 @@ inline void split_digits(Plan &p, u32 first, u32 L, u32 cap) {
 inline Plan make_plan(u32 L, bool wide_first = false, bool ignore_cap = false) {
     Plan p{};
     const u32 cap = ignore_cap ? MAX_D : digit_cap(L);
+    if (!wide_first && !ignore_cap && L >= SMALL_TILE_MIN_L && L <= SMALL_TILE_MAX_L) {
+        // register passes of at most 2^6 points, the last one of 2^4 with the small tile
+        const u32 c = cap < WARP_MAX_D ? cap : WARP_MAX_D;
+        split_digits(p, 0, L - SMALL_TILE, c);
+        for (u32 i = 0; i < p.np; i++) p.lo[i] += SMALL_TILE;
+        p.D[p.np] = SMALL_TILE;
+        p.lo[p.np++] = 0;
+        return p;
+    }
     const u32 first_cap = wide_first ? (cap > MAX_D ? cap : MAX_D) : cap;
     if (L <= first_cap) {
         p.np = 1;
@@ -675,7 +717,6 @@ inline Plan make_plan(u32 L, bool wide_first = false, bool ignore_cap = false) {
 std::atomic<uint64_t> g_attr_done{0};
 std::atomic<uint64_t> g_batch_attr_done{0};
 std::atomic<uint64_t> g_br_attr_done{0};
-std::atomic<uint64_t> g_lbr_attr_done[BR_T + 1][2];
 
 inline size_t pass_smem(u32 D) {
     const size_t S = 1u << D, H = S > 1 ? S / 2 : 1;
@@ -692,8 +733,8 @@ inline bool warp_pass_ok(const PassArgs &a) {
 
 cudaError_t launch_pass(const PassArgs &a, cudaStream_t stream) {
     if (warp_pass_ok(a)) {
-        if (a.shoup) return launch_warp_pass<ZK_NTT_WARP_PENCILS, true>(a, stream);
-        return launch_warp_pass<ZK_NTT_WARP_PENCILS, false>(a, stream);
+        if (a.shoup) return launch_warp_pass<true>(a, stream);
+        return launch_warp_pass<false>(a, stream);
     }
     ZK_TRY(ensure_smem_attr(ntt_pass_kernel, (int)pass_smem(MAX_D), g_attr_done));
     const u64 pencils = 1ull << (a.L - a.D);
@@ -723,38 +764,46 @@ inline bool fuse_last(const Plan &plan, u32 L, bool recompute) {
     return plan.np > 1 && L >= 2 * BR_T && !recompute && plan.D[plan.np - 1] <= BR_T;
 }
 
-template <u32 D, bool SH>
+template <u32 D, bool SH, u32 T>
+cudaError_t prepare_last_bitrev() {
+    static std::atomic<uint64_t> done{0};
+    return ensure_smem_attr(ntt_last_bitrev_kernel<D, SH, T>, (int)LastTile<T>::SMEM, done);
+}
+template <u32 D, bool SH, u32 T>
 cudaError_t launch_last_bitrev_d(const PassArgs &a, cudaStream_t stream) {
-    ZK_TRY(ensure_smem_attr(ntt_last_bitrev_kernel<D, SH>, (int)BR_SMEM, g_lbr_attr_done[D][SH ? 1 : 0]));
-    ntt_last_bitrev_kernel<D, SH><<<1u << (a.L - 2 * BR_T), 512, BR_SMEM, stream>>>(a);
+    ZK_TRY((prepare_last_bitrev<D, SH, T>()));
+    ntt_last_bitrev_kernel<D, SH, T><<<1u << (a.L - 2 * T), LastTile<T>::THREADS, LastTile<T>::SMEM, stream>>>(a);
     return cudaGetLastError();
 }
 
 template <bool SH>
 cudaError_t launch_last_bitrev(const PassArgs &a, cudaStream_t stream) {
+    if (a.D == SMALL_TILE && a.L <= SMALL_TILE_MAX_L) return launch_last_bitrev_d<SMALL_TILE, SH, SMALL_TILE>(a, stream);
     switch (a.D) {
-        case 1: return launch_last_bitrev_d<1, SH>(a, stream);
-        case 2: return launch_last_bitrev_d<2, SH>(a, stream);
-        case 3: return launch_last_bitrev_d<3, SH>(a, stream);
-        case 4: return launch_last_bitrev_d<4, SH>(a, stream);
-        default: return launch_last_bitrev_d<5, SH>(a, stream);
+        case 1: return launch_last_bitrev_d<1, SH, BR_T>(a, stream);
+        case 2: return launch_last_bitrev_d<2, SH, BR_T>(a, stream);
+        case 3: return launch_last_bitrev_d<3, SH, BR_T>(a, stream);
+        case 4: return launch_last_bitrev_d<4, SH, BR_T>(a, stream);
+        default: return launch_last_bitrev_d<5, SH, BR_T>(a, stream);
     }
+}
+
+template <bool SH>
+cudaError_t prepare_last_bitrevs() {
+    ZK_TRY((prepare_last_bitrev<SMALL_TILE, SH, SMALL_TILE>()));
+    ZK_TRY((prepare_last_bitrev<1, SH, BR_T>()));
+    ZK_TRY((prepare_last_bitrev<2, SH, BR_T>()));
+    ZK_TRY((prepare_last_bitrev<3, SH, BR_T>()));
+    ZK_TRY((prepare_last_bitrev<4, SH, BR_T>()));
+    return prepare_last_bitrev<5, SH, BR_T>();
 }
 
 // the shared-memory limits of every kernel run() may launch, set ahead of a stream capture
 inline cudaError_t prepare_run_attrs() {
     ZK_TRY(ensure_smem_attr(ntt_pass_kernel, (int)pass_smem(MAX_D), g_attr_done));
     ZK_TRY(ensure_smem_attr(bitrev_tiled_kernel, (int)BR_SMEM, g_br_attr_done));
-    ZK_TRY(ensure_smem_attr(ntt_last_bitrev_kernel<1, false>, (int)BR_SMEM, g_lbr_attr_done[1][0]));
-    ZK_TRY(ensure_smem_attr(ntt_last_bitrev_kernel<2, false>, (int)BR_SMEM, g_lbr_attr_done[2][0]));
-    ZK_TRY(ensure_smem_attr(ntt_last_bitrev_kernel<3, false>, (int)BR_SMEM, g_lbr_attr_done[3][0]));
-    ZK_TRY(ensure_smem_attr(ntt_last_bitrev_kernel<4, false>, (int)BR_SMEM, g_lbr_attr_done[4][0]));
-    ZK_TRY(ensure_smem_attr(ntt_last_bitrev_kernel<5, false>, (int)BR_SMEM, g_lbr_attr_done[5][0]));
-    ZK_TRY(ensure_smem_attr(ntt_last_bitrev_kernel<1, true>, (int)BR_SMEM, g_lbr_attr_done[1][1]));
-    ZK_TRY(ensure_smem_attr(ntt_last_bitrev_kernel<2, true>, (int)BR_SMEM, g_lbr_attr_done[2][1]));
-    ZK_TRY(ensure_smem_attr(ntt_last_bitrev_kernel<3, true>, (int)BR_SMEM, g_lbr_attr_done[3][1]));
-    ZK_TRY(ensure_smem_attr(ntt_last_bitrev_kernel<4, true>, (int)BR_SMEM, g_lbr_attr_done[4][1]));
-    return ensure_smem_attr(ntt_last_bitrev_kernel<5, true>, (int)BR_SMEM, g_lbr_attr_done[5][1]);
+    ZK_TRY(prepare_last_bitrevs<false>());
+    return prepare_last_bitrevs<true>();
 }
 
 // Runs the full plan.  src (if non-null) is the pass-0 source for the coset LDE.
@@ -765,9 +814,13 @@ cudaError_t run(const View &v, const View *src, u64 src_len, u32 L, const u32 *t
         // a multi-pass table-mode plan: shift and zero-extend in one elementwise pass, then the
         // plain transform in place
         const u64 n = 1ull << L;
-        const u64 warps = (n + 32ull * PREP_C - 1) / (32ull * PREP_C);
+        // about eight warps an SM carry values, with at most PREP_MAX_C elements a lane
+        const u64 live = src && src_len < n ? src_len : n;
+        u32 C = PREP_MIN_C;
+        while (C < PREP_MAX_C && live > 32ull * C * 8 * num_sms()) C *= 2;
+        const u64 warps = (n + 32ull * C - 1) / (32ull * C);
         coset_prep_kernel<<<(u32)((warps * 32 + 255) / 256), 256, 0, stream>>>(v, src ? *src : View{}, src_len,
-                                                                               src != nullptr, shift, n);
+                                                                               src != nullptr, shift, n, C, L);
         ZK_TRY(cudaGetLastError());
         profiler().mark("ntt_prep", stream);
         shift = nullptr;
