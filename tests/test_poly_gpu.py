@@ -167,3 +167,38 @@ def test_permute_matches_oracle(zk, orc, log_n):
     ei, et = orc.permute(inp.numpy_u64(), table.numpy_u64(), usable)
     assert np.array_equal(ri.numpy_u64(), ei)
     assert np.array_equal(rt.numpy_u64(), et)
+
+
+@pytest.mark.parametrize("n", [2, 255, 511, 512, 1023, 1025, 75776, 75777, 606209])
+def test_sweeps_at_chunk_edges(zk, orc, n):
+    """Lengths around one CTA of two-element chunks, and where the chunk length changes."""
+    a = orc.gen_fr(15, n)
+    x = orc.gen_fr(16, 1)[0]
+    res = torch.zeros((1, 8), dtype=torch.int32, device="cuda")
+    zk.poly.poly_eval(dev(zk, a), scal(zk, x), res)
+    assert np.array_equal(res.cpu().numpy().view(np.uint64)[0], orc.eval_poly(a, x))
+    z = a.copy()
+    z[::7] = 0
+    t = dev(zk, z)
+    zk.poly.batched_invert(t)
+    assert np.array_equal(t.numpy_u64(), orc.batch_invert(z))
+    t = dev(zk, a)
+    zk.poly.scan_mul(t)
+    acc, expect = 1, []
+    for v in ints(orc, a):
+        acc = acc * v % M
+        expect.append(acc)
+    assert ints(orc, t.numpy_u64()) == expect
+
+
+@pytest.mark.parametrize("log_n", [8, 11, 13, 17, 20])
+def test_kate_division_chunk_edges(zk, orc, log_n):
+    """q (X - b) + p(b) = p: checked as q[i - 1] - b q[i] = p[i] for every i, with q[n - 1] = 0."""
+    n = 1 << log_n
+    p, b = orc.gen_fr(17, n), orc.gen_fr(18, 1)[0]
+    q = zk.ScalarArray.zeros(n)
+    zk.poly.kate_division(dev(zk, p), scal(zk, b), q)
+    got = q.numpy_u64()
+    assert not got[n - 1].any()
+    bq = orc.vec_mul(got, np.repeat(b[None], n, axis=0))
+    assert np.array_equal(orc.vec_sub(got[:-1], bq[1:]), p[1:])

@@ -5,14 +5,12 @@
 // Temp-buffer protocol as in the reference: a null temp buffer returns the size needed.
 //
 // The reference builds evaluation, inversion and scans from CUB device scans with a field
-// operator.  Here every reduction is a chunked tree of this library's own kernels: each thread
-// folds a contiguous chunk of CHUNK elements (Horner step, running product, ...), the chunk
-// results form a 1/CHUNK-size array that is folded the same way, and a second sweep pushes the
-// combined values back down.  Each element costs one to three Montgomery products and one or
-// two passes over HBM.
+// operator.  Here each of them is at most three launches of this library's own kernels: an up
+// pass (every thread folds a short contiguous chunk, the CTA's threads are joined by shuffle
+// scans), one CTA over the CTA results, and a down pass that walks the chunks again from their
+// carry.  Each element costs one to three Montgomery products and one or two passes over HBM.
 #include <cuda_runtime.h>
-#include <cstring>
-#include <vector>
+#include <utility>
 
 #include "../../include/poly.h"
 #include "common.cuh"
@@ -21,20 +19,39 @@
 namespace zk {
 namespace poly {
 
-constexpr u32 CHUNK = 64;   // elements folded by one evaluation thread on the first level
-// the same for the product scans, inversion and division, whose threads run one dependent
-// chain each (evaluation runs four): 32 gives them twice the chains of 64 (2^22: division
-// 0.365 -> 0.324 ms, inversion 0.487 -> 0.435 ms, product scan 0.332 -> 0.294 ms; 16 is no
-// faster at 2^22 and slower at 2^24)
-constexpr u32 SWEEP = 32;
-constexpr u32 UPPER = 8;    // on the upper levels: short chains, since those levels are tiny
-constexpr u32 BLOCK = 128;
-
-// The level sweeps (evaluation, product scans, inversion, division) fold chunks of `first`
-// elements on the input and chunks of UPPER on every level above it: the first level carries
-// the work, the upper levels are a few thousand values whose cost is the length of their
-// dependent chains.
-inline u32 chunk_at(size_t level, u32 first) { return level == 0 ? first : UPPER; }
+// Threads of the sweeps' CTAs, and the most CTA results the one-CTA step takes (TOP_C a thread).
+// What bounds a sweep is the length of its chain of dependent products, about 0.45 us each (a warp
+// alone on its scheduler): chunk + 8 scan steps per pass.  With 256 threads an SM (two warps a
+// scheduler) the chains nearly fill the multiply pipe, so the chunk is n over that many threads,
+// between 2 and MAX_C elements, and longer only where the CTA results would exceed TOP_MAX.
+// Fixed chunks of 32 to 64 elements and a tree of chunks of 8 above them (up to twelve launches)
+// took 153 / 95 / 76 / 65 us for inversion / product scan / division (2048) / evaluation at 4095
+// elements and 236 / 153 / 153 / 93 us at 2^20; this form 59 / 32 / 26 / 23 and 139 / 77 / 80 / 45
+// (2^24: 1057 / 703 / 679 / 337 us, before 1049 / 760 / 751 / 359).
+constexpr u32 CTA = 256, WARPS = CTA / 32;
+constexpr u32 TOP_C = 16, TOP_MAX = TOP_C * CTA, MAX_C = 32;
+// Up to ONE_CTA elements one CTA does everything in one launch: its chunks are longer (8 elements at
+// 2048), but a chain of some 40 products is shorter than three launches (division of 2048: 25
+// against 49 us; at 4095, with chunks of 16, the inversion took 87 against 62 us).
+constexpr u64 ONE_CTA = 2048;
+inline u32 chunk_for(u64 n) {
+    u32 c = 2;
+    if (n <= ONE_CTA) {
+        while (n > (u64)CTA * c) c *= 2;
+        return c;
+    }
+    while (c < MAX_C && n > (u64)num_sms() * CTA * c) c *= 2;
+    while (c < (1u << 30) && n > (u64)TOP_MAX * CTA * c) c *= 2;
+    return c;
+}
+// elements a thread of the one-CTA step
+inline u32 top_chunk(u64 m) {
+    u32 c = 1;
+    while (m > (u64)CTA * c) c *= 2;
+    return c;
+}
+inline u32 log2_of(u32 c) { return 31 - __builtin_clz(c); }
+inline u64 ctas_for(u64 n, u32 c) { return (n + (u64)CTA * c - 1) / ((u64)CTA * c); }
 
 inline u32 grid_for(u64 items, u32 block, u32 per_sm = 16) {
     const u64 b = (items + block - 1) / block;
@@ -85,117 +102,155 @@ __global__ void __launch_bounds__(256) fill_kernel(View dst, u64 n, u32 kind, bo
     }
 }
 
+// one warp
 __global__ void scalar_kernel(u32 *target, u64 exp, u32 kind) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    Fr x = Fr::load(target);
-    Fr r = kind == 0 ? inv_binary<FrParams>(x) : Fr::pow_u64(x, exp).canonical();
-    r.store(target);
+    const Fr x = Fr::load(target);
+    const Fr r = kind == 0 ? inv_binary_quad<FrParams>(x) : Fr::pow_u64(x, exp).canonical();
+    __syncwarp();
+    if (threadIdx.x == 0) r.store(target);
+}
+
+// ------------------------------------------------------------------ CTA-wide steps
+ZK_DI Fr lane_get(const Fr &x, u32 src) {
+    Fr r;
+#pragma unroll
+    for (int w = 0; w < 8; w++) r.v[w] = __shfl_sync(0xffffffffu, x.v[w], src);
+    return r;
+}
+ZK_DI Fr pick(bool c, const Fr &a, const Fr &b) {
+    Fr r;
+#pragma unroll
+    for (int w = 0; w < 8; w++) r.v[w] = c ? a.v[w] : b.v[w];
+    return r;
+}
+
+// lad[b] = base^(2^b) for b < count (<= 32), by warp 0: lane b squares b times
+ZK_DI void power_ladder(const Fr &base, u32 count, u32 *lad) {
+    if (threadIdx.x >= 32) return;
+    Fr x = base;
+#pragma unroll 1
+    for (u32 b = 0; b + 1 < count; b++) x = pick(threadIdx.x > b, Fr::sqr(x), x);
+    if (threadIdx.x < count) x.store(lad + threadIdx.x * 8);
+}
+
+// exclusive product of the threads before (e) and, with BOTH, after (f); sm: WARPS elements.  The
+// two directions' products of a step are independent.
+template <bool BOTH>
+ZK_DI void lane_products(Fr &x, Fr &y, u32 lane, u32 width) {
+#pragma unroll 1
+    for (u32 d = 1; d < width; d <<= 1) {
+        const Fr a = Fr::mul(x, lane_get(x, lane - d));
+        if (BOTH) y = pick(lane + d < width, Fr::mul(y, lane_get(y, lane + d)), y);
+        x = pick(lane >= d, a, x);
+    }
+}
+template <bool BOTH>
+ZK_DI void cta_products(const Fr &v, u32 *sm, Fr &e, Fr &f, Fr &total) {
+    const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    Fr x = v, y = v;
+    lane_products<BOTH>(x, y, lane, 32);
+    if (lane == 31) x.store(sm + warp * 8);
+    __syncthreads();
+    Fr wx = lane < WARPS ? Fr::load(sm + lane * 8) : Fr::one(), wy = wx;
+    lane_products<BOTH>(wx, wy, lane, WARPS);
+    total = lane_get(wx, WARPS - 1);
+    const Fr bx = lane_get(wx, warp - 1);
+    e = pick(lane > 0, lane_get(x, lane - 1), Fr::one());
+    if (warp > 0) e = Fr::mul(e, bx);
+    if (BOTH) {
+        const Fr by = lane_get(wy, warp + 1);
+        f = pick(lane < 31, lane_get(y, lane + 1), Fr::one());
+        if (warp + 1 < WARPS) f = Fr::mul(f, by);
+    }
+    __syncthreads();
 }
 
 // ------------------------------------------------------------------ evaluation
-// out[t] = sum_{i in chunk t} a_i X^(i - t*CHUNK), as EVAL_CHAINS interleaved Horner chains of
-// EVAL_LEN combined with X^EVAL_LEN; powers[2*level] = X, powers[2*level+1] = X^EVAL_LEN.  Four
-// chains (60 registers) measured fastest: eight (100 registers) 0.176 -> 0.190 ms at 2^22,
-// sixteen 0.255 ms.
-constexpr u32 EVAL_CHAINS = 4, EVAL_LEN = CHUNK / EVAL_CHAINS;
-__global__ void __launch_bounds__(BLOCK) eval_level_kernel(View in, u64 n, const u32 *powers, u32 *out) {
-    const u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x;
-    const u64 start = t * CHUNK;
-    if (start >= n) return;
-    const Fr X = Fr::load(powers), XL = Fr::load(powers + 8);
-    Fr h[EVAL_CHAINS];
-#pragma unroll
-    for (u32 k = 0; k < EVAL_CHAINS; k++) h[k] = Fr::zero();
-#pragma unroll 1
-    for (int j = (int)EVAL_LEN - 1; j >= 0; j--) {
-#pragma unroll
-        for (u32 k = 0; k < EVAL_CHAINS; k++) {
-            const u64 i = start + (u64)k * EVAL_LEN + j;
-            Fr a = i < n ? Fr::load(in.at(i)) : Fr::zero();
-            h[k] = Fr::add(Fr::mul(h[k], X), a);
-        }
-    }
-    Fr r = h[EVAL_CHAINS - 1];
-#pragma unroll
-    for (int k = (int)EVAL_CHAINS - 2; k >= 0; k--) r = Fr::add(Fr::mul(r, XL), h[k]);
-    r.canonical().store(out + t * 8);
-}
-
-// powers for every level: X_0 = x, X_1 = X_0^CHUNK, X_{k+1} = X_k^UPPER, and X_k^EVAL_LEN
-__global__ void eval_powers_kernel(const u32 *x, u32 levels, u32 *powers) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    Fr X = Fr::load(x);
-    for (u32 k = 0; k < levels; k++) {
-        Fr xl = X;
-        for (u32 s = 1; s < EVAL_LEN; s <<= 1) xl = Fr::sqr(xl);
-        X.canonical().store(powers + (2 * k) * 8);
-        xl.canonical().store(powers + (2 * k + 1) * 8);
-        if (k == 0) {
-            for (u32 s = EVAL_LEN; s < CHUNK; s <<= 1) xl = Fr::sqr(xl);
-            X = xl;  // X^CHUNK
-        } else {
-            for (u32 s = 1; s < UPPER; s <<= 1) X = Fr::sqr(X);  // X^UPPER
-        }
-    }
-}
-
-// an upper level: out[t] = sum_{i in chunk t} a_i X^(i - t*chunk), one Horner chain
-__global__ void __launch_bounds__(BLOCK) eval_small_kernel(View in, u64 n, const u32 *powers, u32 chunk, u32 *out) {
-    const u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x;
-    const u64 start = t * chunk;
-    if (start >= n) return;
-    const u64 end = start + chunk < n ? start + chunk : n;
-    const Fr X = Fr::load(powers);
+// out[cta] = sum over the CTA's CTA * c coefficients a_i X^(i - first); next_base = X^(CTA c), the
+// point of the next level.  A thread's chunk is a Horner chain, the chunks are joined by shuffles
+// with X^c, X^2c, ... from the ladder.
+__global__ void __launch_bounds__(CTA) eval_kernel(View in, u64 n, const u32 *base, u32 c, u32 logc, u32 *out,
+                                                   u32 *next_base) {
+    __shared__ __align__(16) u32 lad[32 * 8];
+    __shared__ __align__(16) u32 sm[WARPS * 8];
+    const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const Fr X = Fr::load(base);
+    power_ladder(X, logc + 9, lad);
+    const u64 start = ((u64)blockIdx.x * CTA + threadIdx.x) * c;
     Fr h = Fr::zero();
-    for (u64 i = end; i-- > start;) h = Fr::add(Fr::mul(h, X), Fr::load(in.at(i)));
-    h.canonical().store(out + t * 8);
+    if (start < n) {
+        const u64 end = start + c < n ? start + c : n;
+        h = Fr::load(in.at(end - 1));
+#pragma unroll 4
+        for (u64 i = end - 1; i-- > start;) h = Fr::add(Fr::mul(h, X), Fr::load(in.at(i)));
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (u32 s = 0; s < 5; s++) h = Fr::add(Fr::mul(lane_get(h, lane + (1u << s)), Fr::load(lad + (logc + s) * 8)), h);
+    if (lane == 0) h.store(sm + warp * 8);
+    __syncthreads();
+    if (warp) return;
+    h = lane < WARPS ? Fr::load(sm + lane * 8) : Fr::zero();
+#pragma unroll 1
+    for (u32 s = 0; s < 3; s++)
+        h = Fr::add(Fr::mul(lane_get(h, lane + (1u << s)), Fr::load(lad + (logc + 5 + s) * 8)), h);
+    if (lane == 0) {
+        h.canonical().store(out + (u64)blockIdx.x * 8);
+        if (blockIdx.x == 0 && next_base) Fr::load(lad + (logc + 8) * 8).store(next_base);
+    }
 }
 
-// ------------------------------------------------------------------ chunked product sweeps
-// up-sweep: prefix[i] = running product (inclusive) within the chunk, zeros skipped when
-// skip_zero; tot[t] = chunk product
-__global__ void __launch_bounds__(BLOCK) prod_up_kernel(View in, u64 n, u32 *prefix, u32 *tot, bool skip_zero,
-                                                      u32 chunk) {
-    const u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x;
-    const u64 start = t * chunk;
-    if (start >= n) return;
-    const u64 end = start + chunk < n ? start + chunk : n;
+// ------------------------------------------------------------------ product scan
+// A pass over few values a thread folds its chunk again in the down pass instead of keeping one
+// value a chunk (ex null): the chunk results of short chunks would not fit the scratch the tree of
+// chunks needed, and callers may hold scratch of that size.
+ZK_DI Fr chunk_product(const View &in, u64 n, u64 start, u32 c) {
+    if (start >= n) return Fr::one();
+    const u64 end = start + c < n ? start + c : n;
+    Fr acc = Fr::load(in.at(start));
+#pragma unroll 4
+    for (u64 i = start + 1; i < end; i++) acc = Fr::mul(acc, Fr::load(in.at(i)));
+    return acc;
+}
+// up: ex[t] = product of the CTA's chunks before chunk t, tot[cta] = the CTA's product
+__global__ void __launch_bounds__(CTA) scan_up_kernel(View in, u64 n, u32 c, u32 *ex, u32 *tot) {
+    __shared__ __align__(16) u32 sm[WARPS * 8];
+    const u64 t = (u64)blockIdx.x * CTA + threadIdx.x, start = t * c;
+    Fr e, f, total;
+    cta_products<false>(chunk_product(in, n, start, c), sm, e, f, total);
+    if (ex && start < n) e.store(ex + t * 8);
+    if (threadIdx.x == 0) total.store(tot + (u64)blockIdx.x * 8);
+}
+// exclusive product scan of at most TOP_MAX values in place (one CTA)
+__global__ void __launch_bounds__(CTA) scan_top_kernel(u32 *vals, u32 m, u32 c) {
+    __shared__ __align__(16) u32 sm[WARPS * 8];
+    const u32 start = threadIdx.x * c, end = start + c < m ? start + c : m;
     Fr acc = Fr::one();
-    for (u64 i = start; i < end; i++) {
-        Fr a = Fr::load(in.at(i));
-        if (!(skip_zero && a.is_zero())) acc = Fr::mul(acc, a);
-        if (prefix) acc.store(prefix + i * 8);
-    }
-    acc.canonical().store(tot + t * 8);
-}
-
-// batched inversion down-sweep: inv_tot[t] = (chunk product)^-1; walks the chunk backwards
-__global__ void __launch_bounds__(BLOCK) inv_down_kernel(View data, u64 n, const u32 *prefix, const u32 *inv_tot,
-                                                       u32 chunk) {
-    const u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x;
-    const u64 start = t * chunk;
-    if (start >= n) return;
-    const u64 end = start + chunk < n ? start + chunk : n;
-    Fr inv = Fr::load(inv_tot + t * 8);
-    for (u64 i = end; i-- > start;) {
-        u32 *p = data.at(i);
-        Fr a = Fr::load(p);
-        if (a.is_zero()) continue;
-        Fr before = i > start ? Fr::load(prefix + (i - 1) * 8) : Fr::one();
-        Fr r = Fr::mul(inv, before);
-        inv = Fr::mul(inv, a);
-        r.canonical().store(p);
+    for (u32 i = start; i < end; i++) acc = Fr::mul(acc, Fr::load(vals + (u64)i * 8));
+    Fr e, f, total;
+    cta_products<false>(acc, sm, e, f, total);
+    for (u32 i = start; i < end; i++) {
+        const Fr v = Fr::load(vals + (u64)i * 8);
+        e.store(vals + (u64)i * 8);
+        e = Fr::mul(e, v);
     }
 }
-
-// inclusive product scan down-sweep: `above` is the inclusive scan of the chunk products (or
-// null for the top level), so chunk t starts from above[t-1] (1 for t = 0)
-__global__ void __launch_bounds__(BLOCK) scan_down_kernel(View data, u64 n, const u32 *above, u32 chunk) {
-    const u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x;
-    const u64 start = t * chunk;
-    if (start >= n) return;
-    const u64 end = start + chunk < n ? start + chunk : n;
-    Fr acc = (above && t > 0) ? Fr::load(above + (t - 1) * 8) : Fr::one();
+// cta_ex null: a single CTA
+__global__ void __launch_bounds__(CTA) scan_down_kernel(View data, u64 n, u32 c, const u32 *ex, const u32 *cta_ex) {
+    __shared__ __align__(16) u32 sm[WARPS * 8];
+    const u64 t = (u64)blockIdx.x * CTA + threadIdx.x, start = t * c;
+    Fr acc;
+    if (ex) {
+        if (start >= n) return;
+        acc = Fr::load(ex + t * 8);
+    } else {
+        Fr f, total;
+        cta_products<false>(chunk_product(data, n, start, c), sm, acc, f, total);
+        if (start >= n) return;
+    }
+    if (cta_ex) acc = Fr::mul(acc, Fr::load(cta_ex + (u64)blockIdx.x * 8));
+    const u64 end = start + c < n ? start + c : n;
+#pragma unroll 4
     for (u64 i = start; i < end; i++) {
         u32 *p = data.at(i);
         acc = Fr::mul(acc, Fr::load(p));
@@ -203,104 +258,228 @@ __global__ void __launch_bounds__(BLOCK) scan_down_kernel(View data, u64 n, cons
     }
 }
 
-// top of the inversion tree: one thread inverts the product of at most SWEEP values
-__global__ void inv_top_kernel(u32 *vals, u64 m) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    Fr pre[SWEEP];
+// ------------------------------------------------------------------ batched inversion
+// Montgomery's trick: up, prefix[i] = running product inside the chunk (zeros skipped) for all but
+// its last element, whose place takes the product of the CTA's other chunks; tot[cta] = the CTA's
+// product; one CTA inverts the product
+// of all CTA products and hands every CTA its inverse; down, a chunk starts from
+// inv_tot[cta] prefix[last] = (chunk product)^-1 and walks backwards.
+__global__ void __launch_bounds__(CTA) inv_up_kernel(View in, u64 n, u32 c, u32 *prefix, u32 *tot) {
+    __shared__ __align__(16) u32 sm[WARPS * 8];
+    const u64 t = (u64)blockIdx.x * CTA + threadIdx.x, start = t * c;
     Fr acc = Fr::one();
-    for (u64 i = 0; i < m; i++) {
-        pre[i] = acc;
-        acc = Fr::mul(acc, Fr::load(vals + i * 8));
+    if (start < n) {
+        const u64 end = start + c < n ? start + c : n;
+#pragma unroll 4
+        for (u64 i = start; i < end; i++) {
+            const Fr a = Fr::load(in.at(i));
+            acc = pick(a.is_zero(), acc, Fr::mul(acc, a));
+            if (i + 1 < end) acc.store(prefix + i * 8);
+        }
     }
-    Fr inv = inv_binary<FrParams>(acc);
-    for (u64 i = m; i-- > 0;) {
-        Fr a = Fr::load(vals + i * 8);
-        Fr r = Fr::mul(inv, pre[i]);
-        inv = Fr::mul(inv, a);
-        r.canonical().store(vals + i * 8);
+    Fr e, f, total;
+    cta_products<true>(acc, sm, e, f, total);
+    if (start < n) Fr::mul(e, f).store(prefix + ((start + c < n ? start + c : n) - 1) * 8);
+    if (threadIdx.x == 0) total.store(tot + (u64)blockIdx.x * 8);
+}
+// inverses of at most TOP_MAX non-zero values in place (one CTA); prefix: m elements
+__global__ void __launch_bounds__(CTA) inv_top_kernel(u32 *vals, u32 m, u32 c, u32 *prefix) {
+    __shared__ __align__(16) u32 sm[WARPS * 8];
+    const u32 start = threadIdx.x * c, end = start + c < m ? start + c : m;
+    Fr acc = Fr::one();
+    for (u32 i = start; i < end; i++) {
+        acc.store(prefix + (u64)i * 8);
+        acc = Fr::mul(acc, Fr::load(vals + (u64)i * 8));
+    }
+    Fr e, f, total;
+    cta_products<true>(acc, sm, e, f, total);
+    if (threadIdx.x < 32) {
+        const Fr inv_all = inv_binary_quad<FrParams>(total);
+        if (threadIdx.x == 0) inv_all.store(sm);
+    }
+    __syncthreads();
+    Fr inv = Fr::mul(Fr::load(sm), Fr::mul(e, f));
+    for (u32 i = end; i-- > start;) {
+        const Fr v = Fr::load(vals + (u64)i * 8);
+        Fr::mul(inv, Fr::load(prefix + (u64)i * 8)).store(vals + (u64)i * 8);
+        inv = Fr::mul(inv, v);
     }
 }
-
-// top of the scan tree: exclusive product scan of at most SWEEP values in place
-__global__ void scan_top_kernel(u32 *vals, u64 m) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// all of it for one CTA's elements; prefix: n elements
+__global__ void __launch_bounds__(CTA) inv_one_kernel(View data, u32 n, u32 c, u32 *prefix) {
+    __shared__ __align__(16) u32 sm[WARPS * 8];
+    const u32 start = threadIdx.x * c, end = start + c < n ? start + c : n;
     Fr acc = Fr::one();
-    for (u64 i = 0; i < m; i++) {
-        Fr a = Fr::load(vals + i * 8);
-        acc.canonical().store(vals + i * 8);
-        acc = Fr::mul(acc, a);
+#pragma unroll 2
+    for (u32 i = start; i < end; i++) {
+        const Fr a = Fr::load(data.at(i));
+        acc.store(prefix + (u64)i * 8);
+        acc = pick(a.is_zero(), acc, Fr::mul(acc, a));
+    }
+    Fr e, f, total;
+    cta_products<true>(acc, sm, e, f, total);
+    const Fr ef = Fr::mul(e, f);
+    if (threadIdx.x < 32) {
+        const Fr inv_all = inv_binary_quad<FrParams>(total);
+        if (threadIdx.x == 0) inv_all.store(sm);
+    }
+    __syncthreads();
+    Fr inv = Fr::mul(Fr::load(sm), ef);
+#pragma unroll 2
+    for (u32 i = end; i-- > start;) {
+        u32 *p = data.at(i);
+        const Fr a = Fr::load(p);
+        if (a.is_zero()) continue;
+        const Fr r = Fr::mul(inv, Fr::load(prefix + (u64)i * 8));
+        inv = Fr::mul(inv, a);
+        r.canonical().store(p);
+    }
+}
+__global__ void __launch_bounds__(CTA) inv_down_kernel(View data, u64 n, u32 c, const u32 *prefix,
+                                                       const u32 *inv_tot) {
+    const u64 t = (u64)blockIdx.x * CTA + threadIdx.x, start = t * c;
+    if (start >= n) return;
+    const u64 end = start + c < n ? start + c : n;
+    Fr inv = Fr::mul(Fr::load(prefix + (end - 1) * 8), Fr::load(inv_tot + (u64)blockIdx.x * 8));
+#pragma unroll 2
+    for (u64 i = end; i-- > start;) {
+        u32 *p = data.at(i);
+        const Fr a = Fr::load(p);
+        if (a.is_zero()) continue;
+        const Fr before = i > start ? Fr::load(prefix + (i - 1) * 8) : Fr::one();
+        const Fr r = Fr::mul(inv, before);
+        inv = Fr::mul(inv, a);
+        r.canonical().store(p);
     }
 }
 
 // ------------------------------------------------------------------ kate division
 // q[i] = sum_{j > i} p_j b^(j-i-1), i.e. q[i] = p[i+1] + b q[i+1] with q[n-1] = 0
-// (kate_division.cuh:1-85, halo2 kate_division).  Chunk t holds the local recurrence value
-// with zero carry-in; a chunk's carry is q at its first index.  Up-sweep: local value at the
-// chunk start (Horner over the chunk from its top); the carries combine as another reversed
-// Horner with base b^CHUNK; down-sweep walks each chunk downwards from its carry-in.
-__global__ void __launch_bounds__(BLOCK) kate_up_kernel(View p, u64 n, const u32 *b, u32 *loc, u32 chunk) {
-    const u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x;
-    const u64 start = t * chunk;
-    if (start >= n) return;
-    const u64 end = start + chunk < n ? start + chunk : n;
-    const Fr B = Fr::load(b);
-    // value of q at `start` from the chunk's own terms: sum_{start < j < end+... }
-    Fr acc = Fr::zero();
-    for (u64 i = end; i-- > start;) {
-        // q[i] = p[i+1] + b q[i+1]; inside the chunk q[end-1] uses p[end] and carry q[end]
-        const u64 j = i + 1;
-        Fr pj = j < n ? Fr::load(p.at(j)) : Fr::zero();
-        acc = Fr::add(Fr::mul(acc, B), pj);
+// (kate_division.cuh:1-85, halo2 kate_division).  A chunk's carry is q at the first index after it.
+// up: the chunk-local value at the chunk's start (Horner from its top), then a suffix scan over
+// the CTA with b^c, b^2c, ... gives carry[t], the carry from the CTA's own later chunks, and
+// tot[cta], the value at the CTA's start; one CTA turns those into the carry into every CTA; down
+// adds b^(c (chunks to the CTA's end)) times that carry and walks each chunk downwards.
+// tab (written by CTA 0): b^(c j) for j < 32, then b^(32 c j) for j < WARPS, then b^(CTA c).
+constexpr u32 TAB = 32 + WARPS + 1;
+
+// lad: b^(2^k), k < logc + 9; pw[j] = b^(c j), j < 32 (warp 0)
+ZK_DI void chunk_powers(const u32 *lad, u32 logc, u32 *pw) {
+    if (threadIdx.x >= 32) return;
+    Fr x = Fr::one();
+#pragma unroll 1
+    for (u32 k = 0; k < 5; k++)
+        x = pick((threadIdx.x >> k) & 1, Fr::mul(x, Fr::load(lad + (logc + k) * 8)), x);
+    x.store(pw + threadIdx.x * 8);
+}
+// carry into the thread's chunk from the CTA's later chunks, for chunk-local values v; total = the
+// value at the CTA's start (in lane 0 of warp 0)
+ZK_DI Fr cta_suffix(Fr v, const u32 *lad, u32 logc, const u32 *pw, u32 *sm, Fr &total) {
+    const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll 1
+    for (u32 s = 0; s < 5; s++) {
+        const Fr x = Fr::add(Fr::mul(lane_get(v, lane + (1u << s)), Fr::load(lad + (logc + s) * 8)), v);
+        v = pick(lane + (1u << s) < 32, x, v);
     }
-    acc.canonical().store(loc + t * 8);
+    if (lane == 0) v.store(sm + warp * 8);
+    __syncthreads();
+    Fr w = lane < WARPS ? Fr::load(sm + lane * 8) : Fr::zero();
+#pragma unroll 1
+    for (u32 s = 0; s < 3; s++) {
+        const Fr x = Fr::add(Fr::mul(lane_get(w, lane + (1u << s)), Fr::load(lad + (logc + 5 + s) * 8)), w);
+        w = pick(lane + (1u << s) < WARPS, x, w);
+    }
+    total = w;
+    const Fr next = pick(warp + 1 < WARPS, lane_get(w, warp + 1), Fr::zero());
+    const Fr after = pick(lane < 31, lane_get(v, lane + 1), Fr::zero());
+    return Fr::add(Fr::mul(Fr::load(pw + (31 - lane) * 8), next), after);
 }
 
-// base of the next level: B^chunk
-__global__ void pow_chunk_kernel(const u32 *b, u32 chunk, u32 *out) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    Fr::pow_u64(Fr::load(b), chunk).canonical().store(out);
+// q at `start` from the chunk's own terms p[start + 1 .. end]
+ZK_DI Fr chunk_local(const View &p, u64 n, u64 start, u32 c, const Fr &B) {
+    if (start >= n) return Fr::zero();
+    const u64 end = start + c < n ? start + c : n;
+    Fr acc = end < n ? Fr::load(p.at(end)) : Fr::zero();
+#pragma unroll 4
+    for (u64 j = end - 1; j > start; j--) acc = Fr::add(Fr::mul(acc, B), Fr::load(p.at(j)));
+    return acc;
 }
-
-// a short level (n <= SWEEP): one thread runs the recurrence directly
-__global__ void kate_small_kernel(View p, View q, u64 n, const u32 *b) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+__global__ void __launch_bounds__(CTA) kate_up_kernel(View p, u64 n, const u32 *b, u32 c, u32 logc, u32 *carry,
+                                                      u32 *tot, u32 *tab) {
+    __shared__ __align__(16) u32 lad[32 * 8], pw[32 * 8], sm[WARPS * 8];
     const Fr B = Fr::load(b);
+    power_ladder(B, logc + 9, lad);
+    __syncwarp();
+    chunk_powers(lad, logc, pw);
+    const u64 t = (u64)blockIdx.x * CTA + threadIdx.x, start = t * c;
+    const Fr acc = chunk_local(p, n, start, c, B);
+    __syncthreads();
+    Fr total;
+    const Fr in = cta_suffix(acc, lad, logc, pw, sm, total);
+    if (carry && start < n) in.store(carry + t * 8);
+    if (threadIdx.x == 0) total.store(tot + (u64)blockIdx.x * 8);
+    if (blockIdx.x == 0 && threadIdx.x < 32) {
+        const u32 lane = threadIdx.x;
+        Fr::load(pw + lane * 8).store(tab + lane * 8);
+        Fr x = Fr::one();
+#pragma unroll 1
+        for (u32 k = 0; k < 3; k++) x = pick((lane >> k) & 1, Fr::mul(x, Fr::load(lad + (logc + 5 + k) * 8)), x);
+        if (lane < WARPS) x.store(tab + (32 + lane) * 8);
+        if (lane == 0) Fr::load(lad + (logc + 8) * 8).store(tab + (32 + WARPS) * 8);
+    }
+}
+// vals[i] <- the carry into CTA i: x_i = vals[i+1] + base x_(i+1), 0 for the last (one CTA)
+__global__ void __launch_bounds__(CTA) kate_top_kernel(u32 *vals, u32 m, const u32 *base, u32 c, u32 logc) {
+    __shared__ __align__(16) u32 lad[32 * 8], pw[32 * 8], sm[WARPS * 8];
+    const Fr B = Fr::load(base);
+    power_ladder(B, logc + 9, lad);
+    __syncwarp();
+    chunk_powers(lad, logc, pw);
+    const u32 start = threadIdx.x * c, end = start + c < m ? start + c : m;
     Fr acc = Fr::zero();
-    for (u64 i = n; i-- > 0;) {
+    for (u32 i = end; i-- > start;) acc = Fr::add(Fr::mul(acc, B), Fr::load(vals + (u64)i * 8));
+    __syncthreads();
+    Fr total;
+    Fr in = cta_suffix(acc, lad, logc, pw, sm, total);
+    for (u32 i = end; i-- > start;) {
+        const Fr v = Fr::load(vals + (u64)i * 8);
+        in.store(vals + (u64)i * 8);
+        in = Fr::add(Fr::mul(in, B), v);
+    }
+}
+// carry null: recomputed as in the up pass (see the product scan); tab null: a single CTA
+__global__ void __launch_bounds__(CTA) kate_down_kernel(View p, View q, u64 n, const u32 *b, u32 c, u32 logc,
+                                                        const u32 *carry, const u32 *cta_in, const u32 *tab) {
+    __shared__ __align__(16) u32 lad[32 * 8], pw[32 * 8], sm[WARPS * 8];
+    const u64 t = (u64)blockIdx.x * CTA + threadIdx.x, start = t * c;
+    const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const Fr B = Fr::load(b);
+    Fr acc;
+    if (carry) {
+        if (start >= n) return;
+        acc = Fr::load(carry + t * 8);
+    } else {
+        power_ladder(B, logc + 9, lad);
+        __syncwarp();
+        chunk_powers(lad, logc, pw);
+        const Fr local = chunk_local(p, n, start, c, B);
+        __syncthreads();
+        Fr total;
+        acc = cta_suffix(local, lad, logc, pw, sm, total);
+        if (start >= n) return;
+    }
+    if (tab) {
+        const Fr z = Fr::mul(Fr::load(cta_in + (u64)blockIdx.x * 8), Fr::load(tab + (32 + WARPS - 1 - warp) * 8));
+        acc = Fr::add(Fr::mul(z, Fr::load(tab + (31 - lane) * 8)), acc);
+    }
+    const u64 end = start + c < n ? start + c : n;
+#pragma unroll 4
+    for (u64 i = end; i-- > start;) {
         const u64 j = i + 1;
-        Fr pj = j < n ? Fr::load(p.at(j)) : Fr::zero();
+        const Fr pj = j < n ? Fr::load(p.at(j)) : Fr::zero();
         acc = Fr::add(Fr::mul(acc, B), pj);
         acc.canonical().store(q.at(i));
     }
-}
-
-__global__ void __launch_bounds__(BLOCK) kate_down_kernel(View p, View q, u64 n, const u32 *b, const u32 *carry,
-                                                        u32 chunk) {
-    const u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x;
-    const u64 start = t * chunk;
-    if (start >= n) return;
-    const u64 end = start + chunk < n ? start + chunk : n;
-    const Fr B = Fr::load(b);
-    // carry[t] = q at the first index of chunk t + 1: with loc the chunk-local values, that is
-    // the next level's quotient at t (which is 0 for the last chunk)
-    Fr acc = Fr::load(carry + t * 8);
-    for (u64 i = end; i-- > start;) {
-        const u64 j = i + 1;
-        Fr pj = j < n ? Fr::load(p.at(j)) : Fr::zero();
-        acc = Fr::add(Fr::mul(acc, B), pj);
-        acc.canonical().store(q.at(i));
-    }
-}
-
-// ------------------------------------------------------------------ temp planning
-inline std::vector<u64> level_sizes(u64 n, u32 first) {
-    std::vector<u64> s;
-    u64 m = n;
-    for (size_t k = 0; m > chunk_at(k, first); k++) {
-        m = (m + chunk_at(k, first) - 1) / chunk_at(k, first);
-        s.push_back(m);
-    }
-    return s;  // sizes of the chunk-result arrays; the last one fits in one chunk of its level
 }
 
 inline size_t al(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -361,14 +540,13 @@ extern "C" cudaError_t scalar_pow(unsigned int *target, unsigned long long exp, 
     return cudaGetLastError();
 }
 
-// ---- poly_eval: temp = powers (2 per level) + chunk-result arrays
+// ---- poly_eval: temp = CTA results and the next level's point, per level
 extern "C" cudaError_t poly_eval(void *temp_buf, unsigned long *temp_buf_size, ConstPolyPtr poly, unsigned int *res,
                                  const unsigned int *x, cudaStream_t stream) {
     const u64 n = poly.len;
-    std::vector<u64> lv = level_sizes(n, CHUNK);
-    const u32 levels = (u32)lv.size() + 1;
-    size_t need = al((size_t)levels * 2 * 32);
-    for (u64 m : lv) need += al(m * 32);
+    const u32 c0 = chunk_for(n);
+    const u64 m = ctas_for(n, c0);  // at most TOP_MAX: one CTA finishes
+    const size_t need = al(m * 32) + (m > 1 ? al(32) : 0);
     if (temp_buf == nullptr) {
         ZK_CHECK_ARG(temp_buf_size != nullptr);
         *temp_buf_size = need;
@@ -380,38 +558,22 @@ extern "C" cudaError_t poly_eval(void *temp_buf, unsigned long *temp_buf_size, C
     ZK_CHECK_ARG(make_view(poly, &v));
     if (n == 0) return cudaMemsetAsync(res, 0, 32, stream);
     char *base = reinterpret_cast<char *>(temp_buf);
-    u32 *powers = reinterpret_cast<u32 *>(base);
-    eval_powers_kernel<<<1, 32, 0, stream>>>(x, levels, powers);
-    size_t off = al((size_t)levels * 2 * 32);
-    View in = v;
-    u64 m = n;
-    for (u32 k = 0; k < levels; k++) {
-        u32 *out = (k + 1 < levels) ? reinterpret_cast<u32 *>(base + off) : res;
-        const u32 chunk = chunk_at(k, CHUNK);
-        const u64 threads = (m + chunk - 1) / chunk;
-        const u32 grid = (u32)((threads + BLOCK - 1) / BLOCK);
-        if (k == 0)
-            eval_level_kernel<<<grid, BLOCK, 0, stream>>>(in, m, powers, out);
-        else
-            eval_small_kernel<<<grid, BLOCK, 0, stream>>>(in, m, powers + 2 * k * 8, chunk, out);
-        ZK_TRY(cudaGetLastError());
-        if (k + 1 < levels) {
-            in = plain_view(out, threads);
-            off += al(threads * 32);
-            m = threads;
-        }
-    }
-    return cudaSuccess;
+    u32 *part = reinterpret_cast<u32 *>(base), *point = reinterpret_cast<u32 *>(base + al(m * 32));
+    eval_kernel<<<(u32)m, CTA, 0, stream>>>(v, n, x, c0, log2_of(c0), m == 1 ? res : part, m == 1 ? nullptr : point);
+    ZK_TRY(cudaGetLastError());
+    if (m == 1) return cudaSuccess;
+    const u32 c1 = top_chunk(m);
+    eval_kernel<<<1, CTA, 0, stream>>>(plain_view(part, m), m, point, c1, log2_of(c1), res, nullptr);
+    return cudaGetLastError();
 }
 
-// ---- batched_invert: temp = prefix arrays + chunk-product arrays per level
+// ---- batched_invert: temp = running products, per-CTA products
 extern "C" cudaError_t batched_invert(void *temp_buffer, unsigned long *buffer_size, PolyPtr poly,
                                       cudaStream_t stream) {
     const u64 n = poly.len;
-    std::vector<u64> lv = level_sizes(n, SWEEP);
-    size_t need = al(n * 32);
-    for (u64 m : lv) need += 2 * al(m * 32);
-    need += al(SWEEP * 32);
+    const u32 c = chunk_for(n);
+    const u64 m = ctas_for(n, c);
+    const size_t need = al(n * 32) + 2 * al(m * 32);
     if (temp_buffer == nullptr) {
         ZK_CHECK_ARG(buffer_size != nullptr);
         *buffer_size = need;
@@ -421,52 +583,29 @@ extern "C" cudaError_t batched_invert(void *temp_buffer, unsigned long *buffer_s
     ZK_CHECK_ARG(make_view(poly, &v));
     if (n == 0) return cudaSuccess;
     char *base = reinterpret_cast<char *>(temp_buffer);
-    // level k data: level 0 = poly; level k>0 = tot array of level k-1
-    std::vector<View> data;
-    std::vector<u32 *> prefix;
-    std::vector<u64> size;
-    data.push_back(v);
-    size.push_back(n);
-    size_t off = 0;
-    prefix.push_back(reinterpret_cast<u32 *>(base + off));
-    off += al(n * 32);
-    for (u64 m : lv) {
-        data.push_back(plain_view(base + off, m));
-        off += al(m * 32);
-        prefix.push_back(reinterpret_cast<u32 *>(base + off));
-        off += al(m * 32);
-        size.push_back(m);
+    u32 *prefix = reinterpret_cast<u32 *>(base);
+    u32 *tot = reinterpret_cast<u32 *>(base + al(n * 32));
+    u32 *top_prefix = reinterpret_cast<u32 *>(base + al(n * 32) + al(m * 32));
+    if (m == 1) {
+        inv_one_kernel<<<1, CTA, 0, stream>>>(v, (u32)n, c, prefix);
+        return cudaGetLastError();
     }
-    // the top array: product of the last level's chunks (one value)
-    u32 *top = reinterpret_cast<u32 *>(base + off);
-    const size_t L = data.size();
-    for (size_t k = 0; k < L; k++) {
-        const u64 m = size[k];
-        const u64 threads = (m + chunk_at(k, SWEEP) - 1) / chunk_at(k, SWEEP);
-        u32 *tot = (k + 1 < L) ? data[k + 1].base : top;
-        prod_up_kernel<<<(u32)((threads + BLOCK - 1) / BLOCK), BLOCK, 0, stream>>>(data[k], m, prefix[k], tot, k == 0,
-                                                                                  chunk_at(k, SWEEP));
-        ZK_TRY(cudaGetLastError());
-    }
-    inv_top_kernel<<<1, 32, 0, stream>>>(top, 1);
+    inv_up_kernel<<<(u32)m, CTA, 0, stream>>>(v, n, c, prefix, tot);
     ZK_TRY(cudaGetLastError());
-    for (size_t k = L; k-- > 0;) {
-        const u64 m = size[k];
-        const u64 threads = (m + chunk_at(k, SWEEP) - 1) / chunk_at(k, SWEEP);
-        const u32 *inv_tot = (k + 1 < L) ? data[k + 1].base : top;
-        inv_down_kernel<<<(u32)((threads + BLOCK - 1) / BLOCK), BLOCK, 0, stream>>>(data[k], m, prefix[k], inv_tot,
-                                                                                   chunk_at(k, SWEEP));
-        ZK_TRY(cudaGetLastError());
-    }
-    return cudaSuccess;
+    inv_top_kernel<<<1, CTA, 0, stream>>>(tot, (u32)m, top_chunk(m), top_prefix);
+    ZK_TRY(cudaGetLastError());
+    inv_down_kernel<<<(u32)m, CTA, 0, stream>>>(v, n, c, prefix, tot);
+    return cudaGetLastError();
 }
 
-// ---- scan_mul: inclusive product scan in place; temp = chunk-product arrays
+// ---- scan_mul: inclusive product scan in place; temp = per-CTA products, and per-chunk ones where
+// the chunks are of MAX_C elements or more
 extern "C" cudaError_t scan_mul(void *temp_buffer, unsigned long *buffer_size, PolyPtr target, cudaStream_t stream) {
     const u64 n = target.len;
-    std::vector<u64> lv = level_sizes(n, SWEEP);
-    size_t need = al(32);
-    for (u64 m : lv) need += al(m * 32);
+    const u32 c = chunk_for(n);
+    const u64 m = ctas_for(n, c);
+    const size_t keep = c >= MAX_C ? al(m * CTA * 32) : 0;
+    const size_t need = al((m ? m : 1) * 32) + keep;
     if (temp_buffer == nullptr) {
         ZK_CHECK_ARG(buffer_size != nullptr);
         *buffer_size = need;
@@ -476,42 +615,26 @@ extern "C" cudaError_t scan_mul(void *temp_buffer, unsigned long *buffer_size, P
     ZK_CHECK_ARG(make_view(target, &v));
     if (n == 0) return cudaSuccess;
     char *base = reinterpret_cast<char *>(temp_buffer);
-    std::vector<View> data{v};
-    std::vector<u64> size{n};
-    size_t off = 0;
-    for (u64 m : lv) {
-        data.push_back(plain_view(base + off, m));
-        off += al(m * 32);
-        size.push_back(m);
-    }
-    const size_t L = data.size();
-    for (size_t k = 0; k + 1 < L; k++) {
-        const u64 threads = (size[k] + chunk_at(k, SWEEP) - 1) / chunk_at(k, SWEEP);
-        prod_up_kernel<<<(u32)((threads + BLOCK - 1) / BLOCK), BLOCK, 0, stream>>>(data[k], size[k], nullptr,
-                                                                                  data[k + 1].base, false,
-                                                                                  chunk_at(k, SWEEP));
+    u32 *tot = reinterpret_cast<u32 *>(base), *ex = keep ? reinterpret_cast<u32 *>(base + al(m * 32)) : nullptr;
+    if (m > 1) {
+        scan_up_kernel<<<(u32)m, CTA, 0, stream>>>(v, n, c, ex, tot);
+        ZK_TRY(cudaGetLastError());
+        scan_top_kernel<<<1, CTA, 0, stream>>>(tot, (u32)m, top_chunk(m));
         ZK_TRY(cudaGetLastError());
     }
-    for (size_t k = L; k-- > 0;) {
-        const u64 threads = (size[k] + chunk_at(k, SWEEP) - 1) / chunk_at(k, SWEEP);
-        const u32 *above = (k + 1 < L) ? data[k + 1].base : nullptr;
-        scan_down_kernel<<<(u32)((threads + BLOCK - 1) / BLOCK), BLOCK, 0, stream>>>(data[k], size[k], above,
-                                                                                    chunk_at(k, SWEEP));
-        ZK_TRY(cudaGetLastError());
-    }
-    return cudaSuccess;
+    scan_down_kernel<<<(u32)m, CTA, 0, stream>>>(v, n, c, ex, m > 1 ? tot : nullptr);
+    return cudaGetLastError();
 }
 
-// ---- kate_division: q = (p - p(b)) / (X - b), length 2^log_p.
-// Chunk carries are themselves a kate division (of the chunk-local values by b^CHUNK), so the
-// levels recurse: level k+1 holds the chunk-local values of level k, and its quotient gives
-// the carries of level k.
+// ---- kate_division: q = (p - p(b)) / (X - b), length 2^log_p; temp = powers of b, CTA values, and
+// chunk carries where the chunks are of MAX_C elements or more
 extern "C" cudaError_t kate_division(void *temp_buf, unsigned long *temp_buf_size, unsigned int log_p, ConstPolyPtr p,
                                      const unsigned int *b, PolyPtr q, cudaStream_t stream) {
     const u64 n = 1ull << log_p;
-    std::vector<u64> lv = level_sizes(n, SWEEP);
-    size_t need = al((lv.size() + 1) * 32);
-    for (u64 m : lv) need += 2 * al(m * 32);
+    const u32 c = chunk_for(n);
+    const u64 m = ctas_for(n, c);
+    const size_t keep = c >= MAX_C ? al(m * CTA * 32) : 0;
+    const size_t need = m > 1 ? al(TAB * 32) + al(m * 32) + keep : 256;
     if (temp_buf == nullptr) {
         ZK_CHECK_ARG(temp_buf_size != nullptr);
         *temp_buf_size = need;
@@ -521,36 +644,17 @@ extern "C" cudaError_t kate_division(void *temp_buf, unsigned long *temp_buf_siz
     View vp, vq;
     ZK_CHECK_ARG(make_view(p, &vp) && make_view(q, &vq));
     char *base = reinterpret_cast<char *>(temp_buf);
-    const size_t L = lv.size() + 1;
-    std::vector<View> P{vp}, Q{vq};
-    std::vector<const u32 *> Bs{b};
-    std::vector<u64> size{n};
-    u32 *bases = reinterpret_cast<u32 *>(base);
-    size_t off = al(L * 32);
-    for (size_t k = 0; k < lv.size(); k++) {
-        P.push_back(plain_view(base + off, lv[k]));
-        off += al(lv[k] * 32);
-        Q.push_back(plain_view(base + off, lv[k]));
-        off += al(lv[k] * 32);
-        size.push_back(lv[k]);
-        pow_chunk_kernel<<<1, 32, 0, stream>>>(Bs.back(), chunk_at(k, SWEEP), bases + k * 8);
-        Bs.push_back(bases + k * 8);
-    }
-    // up-sweeps: P[k+1][t] = chunk-local value of level k at chunk t's start
-    for (size_t k = 0; k + 1 < L; k++) {
-        const u64 chunks = (size[k] + chunk_at(k, SWEEP) - 1) / chunk_at(k, SWEEP);
-        kate_up_kernel<<<(u32)((chunks + BLOCK - 1) / BLOCK), BLOCK, 0, stream>>>(P[k], size[k], Bs[k],
-                                                                                 P[k + 1].base, chunk_at(k, SWEEP));
+    u32 *tab = m > 1 ? reinterpret_cast<u32 *>(base) : nullptr;
+    u32 *tot = reinterpret_cast<u32 *>(base + al(TAB * 32));
+    u32 *carry = keep ? reinterpret_cast<u32 *>(base + al(TAB * 32) + al(m * 32)) : nullptr;
+    if (m > 1) {
+        kate_up_kernel<<<(u32)m, CTA, 0, stream>>>(vp, n, b, c, log2_of(c), carry, tot, tab);
+        ZK_TRY(cudaGetLastError());
+        const u32 c1 = top_chunk(m);
+        kate_top_kernel<<<1, CTA, 0, stream>>>(tot, (u32)m, tab + (32 + WARPS) * 8, c1, log2_of(c1));
         ZK_TRY(cudaGetLastError());
     }
-    kate_small_kernel<<<1, 32, 0, stream>>>(P[L - 1], Q[L - 1], size[L - 1], Bs[L - 1]);
-    ZK_TRY(cudaGetLastError());
-    for (size_t k = L - 1; k-- > 0;) {
-        const u64 chunks = (size[k] + chunk_at(k, SWEEP) - 1) / chunk_at(k, SWEEP);
-        kate_down_kernel<<<(u32)((chunks + BLOCK - 1) / BLOCK), BLOCK, 0, stream>>>(P[k], Q[k], size[k], Bs[k],
-                                                                                   Q[k + 1].base, chunk_at(k, SWEEP));
-        ZK_TRY(cudaGetLastError());
-    }
-    return cudaSuccess;
+    kate_down_kernel<<<(u32)m, CTA, 0, stream>>>(vp, vq, n, b, c, log2_of(c), carry, tot, tab);
+    return cudaGetLastError();
 }
 #include "permute.cuh"
