@@ -202,3 +202,30 @@ def test_kate_division_chunk_edges(zk, orc, log_n):
     assert not got[n - 1].any()
     bq = orc.vec_mul(got, np.repeat(b[None], n, axis=0))
     assert np.array_equal(orc.vec_sub(got[:-1], bq[1:]), p[1:])
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 2047, 2048, 2049, 9000])
+@pytest.mark.parametrize("kind", ["random", "small", "signed", "clash"])
+def test_permute_key_shapes(zk, orc, n, kind):
+    """Sort keys of every shape the word choice meets: random field elements, a small range, small
+    values and their negatives (one word cannot tell them apart), and values that agree in their
+    top bits in runs longer than the insertion step takes."""
+    rng = np.random.default_rng(n)
+    if kind == "random":
+        vals = [int.from_bytes(rng.bytes(32), "little") % M for _ in range(n)]
+    elif kind == "small":
+        vals = [int(v) for v in rng.integers(0, max(2, n // 3), n)]
+    elif kind == "signed":
+        vals = [int(v) if s else (M - 1 - int(v)) for v, s in zip(rng.integers(0, n + 1, n), rng.integers(0, 2, n))]
+    else:
+        tops = [int.from_bytes(rng.bytes(3), "little") << 220 for _ in range(3)]
+        vals = [tops[int(t)] | (int(m) << 100) | int(v)
+                for t, m, v in zip(rng.integers(0, 3, n), rng.integers(0, 4, n), rng.integers(0, 50, n))]
+    table = np.stack([orc.to_mont(orc.int_to_limbs(v % M)) for v in vals])
+    usable = max(1, n - 3)
+    inp = table[rng.integers(0, usable, n)]
+    ri, rt = zk.ScalarArray.alloc(usable), zk.ScalarArray.alloc(usable)
+    zk.poly.permute(dev(zk, inp), dev(zk, table), usable, ri, rt)
+    ei, et = orc.permute(inp, table, usable)
+    assert np.array_equal(ri.numpy_u64(), ei)
+    assert np.array_equal(rt.numpy_u64(), et)
