@@ -144,7 +144,7 @@ ZK_DI G1X g1_madd(const G1X &a, const G1A &b) {
     Fq q = fmul(a.x, pp);
     G1X o;
     o.x = Fq::sub(Fq::sub(Fq::sub(fsqr(r), ppp), q), q);
-    o.y = Fq::sub(fmul(r, Fq::sub(q, o.x)), fmul(a.y, ppp));
+    o.y = Fq::mul_sub(r, Fq::sub(q, o.x), a.y, ppp);
     o.zz = fmul(a.zz, pp);
     o.zzz = fmul(a.zzz, ppp);
     return o;
@@ -166,7 +166,7 @@ ZK_DI G1X g1_add(const G1X &a, const G1X &b) {
     Fq q = fmul(u1, pp);
     G1X o;
     o.x = Fq::sub(Fq::sub(Fq::sub(fsqr(r), ppp), q), q);
-    o.y = Fq::sub(fmul(r, Fq::sub(q, o.x)), fmul(s1, ppp));
+    o.y = Fq::mul_sub(r, Fq::sub(q, o.x), s1, ppp);
     o.zz = fmul(fmul(a.zz, b.zz), pp);
     o.zzz = fmul(fmul(a.zzz, b.zzz), ppp);
     return o;

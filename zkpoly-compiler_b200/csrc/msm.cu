@@ -72,7 +72,7 @@ struct Task {
 // exclusive prefixes (entry ntasks is the total).
 struct Batch {
     u32 ntasks;
-    u32 K;  // entries per accumulation chunk
+    u32 walkers, walk_min;  // threads of the walk and their least number of entries (walk_chunk)
     Task task[MAX_TASKS];
     u64 sc_first[MAX_TASKS + 1];   // scalars
     u64 key_first[MAX_TASKS + 1];  // buckets (Wp * B per task)
@@ -166,9 +166,20 @@ inline u64 next_list_bound(u64 e, u64 nb) {
     return x < e ? x : e;
 }
 
-// fills the prefixes and the chunk size (at least min_chunk entries: a chunk costs 280 bytes of
-// workspace); tasks[] must be set.  rounds < 0: the library setting (itself -1 = by size).
-inline void finish_batch(Batch &b, int rounds = -1, u32 min_chunk = 4) {
+// The walk's chunk length for a list of `live` entries: as many chunks as threads fit the GPU at once
+// (WALK_THREADS an SM, at 128 registers), so that the walk is one full wave and the lists are cut
+// as rarely as that allows (every cut leaves a chain to the fix-up), but at least walk_min entries.
+// The length is computed on the device from the list's real length: digits that are zero and pairs
+// already added shorten it below what the host can know.
+constexpr u32 WALK_THREADS = 512, WALK_MIN = 4;
+ZK_DI u32 walk_chunk(u32 live, u32 walkers, u32 walk_min) {
+    const u32 k = live / walkers + (live % walkers ? 1 : 0);
+    return k < walk_min ? walk_min : k;
+}
+
+// fills the prefixes and the launch shapes; tasks[] must be set.  rounds < 0: the library
+// setting (itself -1 = by size).
+inline void finish_batch(Batch &b, int rounds = -1, u32 walk_min = WALK_MIN) {
     b.sc_first[0] = b.key_first[0] = b.seg_first[0] = 0;
     b.win_first[0] = 0;
     b.ncls = b.nparts = 1;
@@ -196,15 +207,8 @@ inline void finish_batch(Batch &b, int rounds = -1, u32 min_chunk = 4) {
     }
     if (rounds < 0) rounds = affine_rounds_setting();
     b.rounds = rounds < 0 ? auto_rounds(entries) : (u32)(rounds > (int)MAX_ROUNDS ? MAX_ROUNDS : rounds);
-    u64 walk = entries;
-    for (u32 r = 0; r < b.rounds; r++) walk = next_list_bound(walk, b.key_first[b.ntasks]);
-    entries = walk;
-    // chunk so that roughly 4 waves of 384 threads per SM cover the walk's entries
-    const u64 threads = (u64)num_sms() * 384 * 4;
-    u64 k = (entries + threads - 1) / threads;
-    if (k < min_chunk) k = min_chunk;
-    if (k > 4096) k = 4096;
-    b.K = (u32)k;
+    b.walkers = (u32)num_sms() * WALK_THREADS;
+    b.walk_min = walk_min;
 }
 
 // ------------------------------------------------------------------ workspace layout
@@ -259,7 +263,14 @@ inline Layout make_layout(const Batch &b) {
         l.emax[r + 1] = next_list_bound(l.emax[r], l.nb);
         l.thr[r] = (l.emax[r] + KA - 1) / KA;
     }
-    l.chunks = (l.emax[l.rounds] + b.K - 1) / b.K;
+    l.chunks = (l.emax[l.rounds] + b.walk_min - 1) / b.walk_min;  // most that walk_chunk can ask for
+    if (l.chunks > b.walkers) l.chunks = b.walkers;
+    // Room for at least one chunk per eight entries, up to four waves of 384 threads an SM: what the
+    // partial sums have always taken.  zkp_msm_device_noalloc decides by the total which sizes fit
+    // its fixed array, and that limit is part of its interface.
+    const u64 waves = (u64)num_sms() * 384 * 4, per = (l.emax[l.rounds] + waves - 1) / waves;
+    const u64 usual = (l.emax[l.rounds] + (per < 8 ? 8 : per) - 1) / (per < 8 ? 8 : per);
+    const u64 room = l.chunks > usual ? l.chunks : usual;
     l.counts = take((l.nb + 1) * 4);
     l.cursor = take((l.nb + 1) * 4);
     l.scan_sums = take(((l.nb + 1) / 4096 + 2) * 4);
@@ -297,15 +308,23 @@ inline Layout make_layout(const Batch &b) {
         }
     }
     l.bucket_sums = take(l.nb * 128);
-    l.part_pts = take(l.chunks * 2 * 128);
-    l.part_bucket = take(l.chunks * 2 * 4);
-    l.part_flag = take(l.chunks * 2 * 4);
-    l.long_list = take((l.chunks + 1) * 4 + 4);  // long chain starts + a counter at the end
-    l.chain_list = take((l.chunks + 1) * 4);     // chain starts + a counter at the end
+    l.part_pts = take(room * 2 * 128);
+    l.part_bucket = take(room * 2 * 4);
+    l.part_flag = take(room * 2 * 4);
+    l.long_list = take((room + 1) * 4 + 4);  // long chain starts + a counter at the end
+    l.chain_list = take((room + 1) * 4);     // chain starts + a counter at the end
     l.seg = take(2 * l.segs * 128);  // U_g then T_g
-    // class parts: in the cursors' place (last used by the pairing rounds) where they fit
-    const size_t cls_bytes = l.wins * b.ncls * b.nparts * 128;
-    l.cls = cls_bytes <= (l.nb + 1) * 4 ? l.cursor : take(cls_bytes);
+    // class parts: room for one part per 2048 segment sums, as ever; more parts than that go where the
+    // cursors were (last used by the pairing rounds), if they fit there
+    u32 few = 1;
+    for (u32 t = 0; t < b.ntasks; t++) {
+        const u32 p = b.task[t].B / b.task[t].L / 2 / 2048;
+        few = p > few ? (p < MAX_PARTS ? p : MAX_PARTS) : few;
+    }
+    const size_t cls_usual = l.wins * b.ncls * few * 128, cls_bytes = l.wins * b.ncls * b.nparts * 128;
+    const bool in_cursor = cls_bytes > cls_usual && cls_bytes <= (l.nb + 1) * 4;
+    const size_t cls_at = take(in_cursor || cls_bytes < cls_usual ? cls_usual : cls_bytes);
+    l.cls = in_cursor ? l.cursor : cls_at;
     l.win = take(l.wins * 128);
     l.total = off;
     return l;
@@ -536,7 +555,7 @@ ZK_DI G1A fetch_point(const u32 *points, u32 code) {
     return p;
 }
 
-// The sorted array (live entries: *live) is cut into chunks of K; one thread per chunk walks
+// The sorted array (live entries: *live) is cut into chunks of walk_chunk; one thread per chunk walks
 // it with mixed additions.  A run of one bucket wholly inside the chunk is stored to its
 // bucket; a run cut by a chunk edge leaves a partial: part_flag 1 = head run (continued from
 // the previous chunk, ends here), 2 = head run that also continues into the next chunk,
@@ -556,9 +575,10 @@ __global__ void __launch_bounds__(256, ZK_ACC_MIN_BLOCKS) accumulate_kernel(cons
     constexpr u32 S = CODES ? 2 : 1;  // words between consecutive bucket ids
     const u64 entries = *live;
     const u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x;
-    const u64 start = t * b.K;
+    const u32 K = walk_chunk(*live, b.walkers, b.walk_min);
+    const u64 start = t * K;
     if (start >= entries) return;
-    const u64 end = start + b.K < entries ? start + b.K : entries;
+    const u64 end = start + K < entries ? start + K : entries;
     const bool from_prev = start > 0 && sorted_bucket[S * (start - 1)] == sorted_bucket[S * start];
     u64 run_start = start;
     u32 cur = sorted_bucket[S * start];
@@ -649,10 +669,11 @@ ZK_DI bool chain_member(const u32 *part_bucket, const u32 *part_flag, u64 u, u32
 }
 
 // One quad per chain start recorded by the walk (chain_list, chain_count entries).
-__global__ void __launch_bounds__(256) fixup_kernel(const u32 *live, u32 K, u32 *bucket_sums, const u32 *part_pts,
+__global__ void __launch_bounds__(256) fixup_kernel(const u32 *live, u32 walkers, u32 walk_min, u32 *bucket_sums, const u32 *part_pts,
                                                    const u32 *part_bucket, const u32 *part_flag,
                                                    const u32 *chain_list, const u32 *chain_count, u32 *long_list,
                                                    u32 *long_count) {
+    const u32 K = walk_chunk(*live, walkers, walk_min);
     const u64 chunks = ((u64)*live + K - 1) / K;
     const u32 count = *chain_count;
     const u64 i = ((u64)blockIdx.x * blockDim.x + threadIdx.x) >> 2;
@@ -697,11 +718,12 @@ ZK_DI Fq g1_sum_cta(u32 *sm, const Fq &mine) {
 }
 
 // one CTA per long chain (looping over the recorded list): strided partial sums, then a tree
-__global__ void __launch_bounds__(128) long_chain_kernel(const u32 *live, u32 K, u32 *bucket_sums,
+__global__ void __launch_bounds__(128) long_chain_kernel(const u32 *live, u32 walkers, u32 walk_min, u32 *bucket_sums,
                                                         const u32 *part_pts, const u32 *part_bucket,
                                                         const u32 *part_flag, const u32 *long_list,
                                                         const u32 *long_count) {
     __shared__ __align__(16) u32 sm[4 * 32];
+    const u32 K = walk_chunk(*live, walkers, walk_min);
     const u64 chunks = ((u64)*live + K - 1) / K;
     const u32 nlong = *long_count;
     const u32 quad = threadIdx.x >> 2, quads = blockDim.x >> 2, role = quad_role();
@@ -1343,10 +1365,10 @@ cudaError_t run_batch(const Batch &b, const Layout &l, char *ws, cudaStream_t st
     }
     prof.mark("accumulate", stream);
     if (l.chunks) {
-        fixup_kernel<<<(u32)((l.chunks * 4 + 255) / 256), 256, 0, stream>>>(live, b.K, bs, pp, pb, pf, chains, nchain,
+        fixup_kernel<<<(u32)((l.chunks * 4 + 255) / 256), 256, 0, stream>>>(live, b.walkers, b.walk_min, bs, pp, pb, pf, chains, nchain,
                                                                         longs, nlong);
         ZK_TRY(cudaGetLastError());
-        long_chain_kernel<<<num_sms() * 2, 128, 0, stream>>>(live, b.K, bs, pp, pb, pf, longs, nlong);
+        long_chain_kernel<<<num_sms() * 2, 128, 0, stream>>>(live, b.walkers, b.walk_min, bs, pp, pb, pf, longs, nlong);
         ZK_TRY(cudaGetLastError());
     }
     prof.mark("fixup", stream);
@@ -1426,14 +1448,14 @@ inline void resolve(u64 n, u32 window, u32 n_tables_hint, u32 *c, u32 *n_tables)
 }
 
 inline Batch single(const u32 *points, u32 n_tables, const u32 *scalars, u64 n, u32 c, u32 *result,
-                    int rounds = -1, u32 min_chunk = 4) {
+                    int rounds = -1, u32 walk_min = WALK_MIN) {
     Batch b{};
     b.ntasks = 1;
     b.task[0] = make_task(n, c, n_tables);
     b.task[0].points = points;
     b.task[0].scalars = scalars;
     b.task[0].result = result;
-    finish_batch(b, rounds, min_chunk);
+    finish_batch(b, rounds, walk_min);
     return b;
 }
 
