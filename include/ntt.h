@@ -81,7 +81,11 @@ cudaError_t zkp_coset_lde_shoup(PolyPtr out, ConstPolyPtr in, const unsigned int
 cudaError_t zkp_ntt_roots_device(unsigned int *out_d, unsigned long long count, const unsigned int *unit_d,
                                  cudaStream_t stream);
 
-/* Plan tuning (no counterpart in the reference): caps the digit width of the passes used for
+/* Buffers: elements are read and written 16 bytes at a time; a vector, root table and Shoup table
+ * that are all aligned to 32 bytes (as any allocation is) let transforms from 2^21 points use the
+ * tensor-core passes, others take the register passes, with the same results.
+ *
+ * Plan tuning (no counterpart in the reference): caps the digit width of the passes used for
  * transforms of 2^log_len elements (log_len 0: every size) at max_digit in [4, 12] (0 restores
  * the default 12).  Each pass transforms 2^D-element pencils in shared memory, D <= max_digit;
  * a smaller cap means more passes of smaller CTAs.  Plans made after the call use it. */

@@ -416,3 +416,42 @@ def test_coset_powers_edges(zk, orc, log_in, log_out):
     out = zk.ScalarArray.zeros(1 << log_out)
     zk.ntt.coset_ntt(out, to_dev(zk, coef))
     assert np.array_equal(out.numpy_u64(), orc.coset_ntt(coef, log_in, log_out, g))
+
+
+@pytest.mark.parametrize("log_n,fill", [(21, "top"), (21, "random"), (22, "top"), (23, "random"), (24, "random")])
+def test_ntt_radix16_passes(zk, orc, log_n, fill):
+    """The tensor-core passes with every split of the index bits around them, forward and inverse,
+    with the Shoup and the Montgomery table: element by element against best_fft, with the largest
+    bytes the column sums meet (all r - 1) and random values.  A buffer 16 bytes off a 32-byte
+    boundary takes the register passes and gives the same vector."""
+    import torch
+    n = 1 << log_n
+    a = orc.gen_fr(300 + log_n, n)
+    if fill == "top":
+        a[: 3 * n // 4] = orc.int_to_limbs(zk.field.FR_MODULUS - 1)
+        a[n // 2: n // 2 + 100] = 0
+    expect = orc.best_fft(a, orc.root_of_unity(log_n), log_n)
+    assert sum(zk.ntt.plan_digits(log_n)) == log_n
+    tw = zk.ntt.twiddle_table(log_n)
+    raw = torch.empty(n * 8 + 4, dtype=torch.int32, device="cuda")
+    off = zk.ScalarArray(raw[4:].view(n, 8))
+    for shoup in (zk.ntt.shoup_table(log_n), None):
+        x = to_dev(zk, a)
+        off.values.copy_(x.values)
+        for v in (x, off):
+            zk.ntt.ntt_ex(v, tw, shoup=shoup)
+            assert np.array_equal(v.numpy_u64(), expect), (shoup is None, v is off)
+        zk.ntt.ntt_ex(x, zk.ntt.twiddle_table(log_n, True), None, zk.ntt.n_inv(log_n),
+                      shoup=None if shoup is None else zk.ntt.shoup_table(log_n, True))
+        assert np.array_equal(x.numpy_u64(), a)
+
+
+def test_ntt_radix16_rotated_view(zk, orc):
+    log_n = 21
+    n = 1 << log_n
+    a = orc.gen_fr(320, n)
+    x = to_dev(zk, a)
+    x.rotate(12345)
+    expect = orc.best_fft(orc.poly_ptr_view(a, n, rotate=12345), orc.root_of_unity(log_n), log_n)
+    zk.ntt.ntt(x)
+    assert np.array_equal(x.numpy_u64(), expect)

@@ -553,6 +553,12 @@ __global__ void __launch_bounds__(LastTile<T>::THREADS, 2) ntt_last_bitrev_kerne
     }
 }
 
+}  // namespace ntt
+}  // namespace zk
+#include "ntt_umma.cuh"
+namespace zk {
+namespace ntt {
+
 // Coset preparation for multi-pass table-mode transforms: v[i] = x[i] * shift^i, with x the
 // source view (zero beyond src_len: the zero-extension of a coset LDE) or v itself, so that the
 // transform then runs its plain passes; folding the shift into a shared-memory first pass, which
@@ -673,6 +679,32 @@ inline void split_digits(Plan &p, u32 first, u32 L, u32 cap) {
         p.lo[first + i] = rem;
     }
     p.np = first + np;
+}
+
+// From this size table-mode transforms over 32-byte aligned buffers run radix-16 passes on the
+// integer tensor cores (ntt_umma.cuh), between register passes: 2^21 403 -> 376 us, 2^22 816 -> 752,
+// 2^24 3438 -> 2917; at 2^20 the constants' set-up and half-filled CTAs make them slower (209 -> 219).
+constexpr u32 UM_MIN_L = 21;
+inline bool aligned32(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 31) == 0; }
+inline bool umma_ok(u32 L, const View &v, const u32 *tw, const u32 *shoup) {
+    return L >= UM_MIN_L && tw != nullptr && aligned32(v.base) && aligned32(tw) && aligned32(shoup);
+}
+// [register pass over the top 1 or 2 bits where needed,] radix-16 passes, and a last register pass
+// of 2^4 or 2^5 points with the tiled bit reversal
+inline Plan umma_plan(u32 L) {
+    Plan p{};
+    const u32 um = (L - 4) / UM_D, rest = L - 4 - um * UM_D;
+    u32 rem = L;
+    auto pass = [&](u32 D) {
+        rem -= D;
+        p.D[p.np] = D;
+        p.lo[p.np++] = rem;
+    };
+    const u32 last = rest && digit_cap(L) >= 5 ? 5 : 4;
+    if (rest + 4 > last) pass(rest + 4 - last);
+    for (u32 i = 0; i < um; i++) pass(UM_D);
+    pass(last);
+    return p;
 }
 
 // The tile of the fused last pass: 16 x 16 elements for transforms of these sizes (more CTAs, and
@@ -798,10 +830,26 @@ cudaError_t prepare_last_bitrevs() {
     return prepare_last_bitrev<5, SH, BR_T>();
 }
 
+template <bool SH>
+cudaError_t prepare_umma() {
+    static std::atomic<uint64_t> done{0};
+    return ensure_smem_attr(ntt_umma_kernel<SH>, (int)UM_SMEM, done);
+}
+template <bool SH>
+cudaError_t launch_umma(const PassArgs &a, cudaStream_t stream) {
+    ZK_TRY(prepare_umma<SH>());
+    const u32 items = 1u << (a.L - UM_D - 7);
+    const u32 grid = items < (u32)num_sms() ? items : (u32)num_sms();
+    ntt_umma_kernel<SH><<<grid, UM_GROUPS * 128, UM_SMEM, stream>>>(a, items);
+    return cudaGetLastError();
+}
+
 // the shared-memory limits of every kernel run() may launch, set ahead of a stream capture
 inline cudaError_t prepare_run_attrs() {
     ZK_TRY(ensure_smem_attr(ntt_pass_kernel, (int)pass_smem(MAX_D), g_attr_done));
     ZK_TRY(ensure_smem_attr(bitrev_tiled_kernel, (int)BR_SMEM, g_br_attr_done));
+    ZK_TRY(prepare_umma<false>());
+    ZK_TRY(prepare_umma<true>());
     ZK_TRY(prepare_last_bitrevs<false>());
     return prepare_last_bitrevs<true>();
 }
@@ -827,7 +875,8 @@ cudaError_t run(const View &v, const View *src, u64 src_len, u32 L, const u32 *t
         src = nullptr;
         src_len = 0;
     }
-    const Plan plan = make_plan(L, shift != nullptr || src != nullptr, omegas != nullptr);
+    const bool um = shift == nullptr && src == nullptr && omegas == nullptr && umma_ok(L, v, tw, shoup);
+    const Plan plan = um ? umma_plan(L) : make_plan(L, shift != nullptr || src != nullptr, omegas != nullptr);
     const bool fused_tail = fuse_last(plan, L, omegas != nullptr);
     for (u32 p = 0; p < plan.np; p++) {
         PassArgs a{};
@@ -858,7 +907,8 @@ cudaError_t run(const View &v, const View *src, u64 src_len, u32 L, const u32 *t
             profiler().mark("ntt_pass", stream);
             return cudaSuccess;
         }
-        ZK_TRY(launch_pass(a, stream));
+        if (um && a.D == UM_D) ZK_TRY(shoup ? launch_umma<true>(a, stream) : launch_umma<false>(a, stream));
+        else ZK_TRY(launch_pass(a, stream));
         profiler().mark("ntt_pass", stream);
     }
     if (plan.np > 1) {
@@ -1188,13 +1238,13 @@ extern "C" cudaError_t zkp_ntt_set_block(unsigned int log_len, unsigned int thre
 
 extern "C" unsigned int zkp_ntt_plan_digits(unsigned int log_len, unsigned int *digits, unsigned int max) {
     if (log_len == 0 || log_len > 28) return 0;
-    const ntt::Plan p = ntt::make_plan(log_len);
+    const ntt::Plan p = log_len >= ntt::UM_MIN_L ? ntt::umma_plan(log_len) : ntt::make_plan(log_len);
     for (u32 i = 0; i < p.np && i < max && digits; i++) digits[i] = p.D[i];
     return p.np;
 }
 
 extern "C" unsigned int zkp_ntt_num_passes(unsigned int log_len) {
-    ntt::Plan p = ntt::make_plan(log_len);
+    ntt::Plan p = log_len >= ntt::UM_MIN_L ? ntt::umma_plan(log_len) : ntt::make_plan(log_len);
     if (ntt::fuse_last(p, log_len, false)) return p.np;  // the last pass also permutes
     return p.np + (p.np > 1 ? 1 : 0);
 }
