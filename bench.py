@@ -991,10 +991,10 @@ def emit(args, zk, rank, world, n_msm, n_ntt, ntt_ms, msm_ms, step_ms, pass_ms, 
     # log2(n) - 1 stages that have non-trivial twiddles (independent of the pass split)
     ntt_mults = (n_ntt // 2) * (NTT_LOG - 1)
     launches_per_ntt = zk.ntt.num_passes(NTT_LOG)
-    # sort (count, 3 scan, scatter), walk (accumulate, fixup, long chains), reduction (segment,
-    # classes, window), combine, zero results = 13; a pairing round: halve, 3 scan, up, tree
+    # clear, sort (count, 3 scan, scatter), walk (accumulate, fixup, long chains), reduction (segment,
+    # classes, scale, window), combine, zero results = 15; a pairing round: halve, 3 scan, up, tree
     # (one level + top + one level at these sizes), down = 9
-    launches_per_msm = 13 + 9 * rounds
+    launches_per_msm = 15 + 9 * rounds
     line = {
         "metric": METRIC, "value": world * n_msm / (msm_ms / 1e3), "unit": "points/s", "n_gpus": world,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": step_ms, "higher_is_better": True,
@@ -1010,14 +1010,15 @@ def emit(args, zk, rank, world, n_msm, n_ntt, ntt_ms, msm_ms, step_ms, pass_ms, 
         "ntt": {"metric": f"NTT elems/s (2^{NTT_LOG})", "value": world * n_ntt / (ntt_ms / 1e3), "unit": "elems/s",
                 "ms": ntt_ms, "pass_ms": pass_avg, "bitrev_ms": statistics.median(bitrev_ms) if bitrev_ms else None,
                 "hbm_frac_whole_ntt": (64 * n_ntt / (ntt_ms / 1e3) / 1e9) / hbm_peak,
-                "path": "zkp_ntt_ex_shoup: register passes with Shoup twiddle products (root table + Shoup "
-                        "table of 64 B per root, both built once outside the timed region)",
+                "path": "zkp_ntt_ex_shoup: radix-16 passes on the integer tensor cores and register passes, Shoup "
+                        "twiddle products (root table + Shoup table of 64 B per root, both built once "
+                        "outside the timed region)",
                 "ssip_ms": ssip_ms, "ssip_value": world * n_ntt / (ssip_ms / 1e3) if ssip_ms else None,
                 "ssip_path": "ssip_ntt (reference ABI): the same passes with Montgomery twiddle products"},
         # the NTT's HBM roofline: 64 B per element (one read + one write
         # of the vector) for the whole transform, over the transform's CUDA-event time
-        "roofline": {"kernel": f"NTT 2^{NTT_LOG} forward transform: {len(digits)} register passes "
-                               f"(ntt_warp_pass_kernel, the last fused with the bit reversal in "
+        "roofline": {"kernel": f"NTT 2^{NTT_LOG} forward transform: {len(digits)} passes (ntt_umma_kernel "
+                               f"radix-16 passes, the last a register pass fused with the bit reversal in "
                                f"ntt_last_bitrev_kernel), digits {digits}, Shoup twiddle products",
                      "bound": "imad", "achieved": ntt_alg_gbs, "peak": hbm_peak, "unit": "GB/s",
                      "frac": ntt_alg_gbs / hbm_peak, "peak_source": peak_kind,
@@ -1028,9 +1029,8 @@ def emit(args, zk, rank, world, n_msm, n_ntt, ntt_ms, msm_ms, step_ms, pass_ms, 
                      "frac_per_pass_note": "64 B per element for ONE pass over the median pass time: every pass "
                                            "reads and writes the vector, so this credits each pass with the "
                                            "transform's algorithmic bytes",
-                     "note": "bound by the integer multiply pipe, not HBM: the twiddle products at the measured "
-                             "Shoup-product peak take longer than the vector's HBM traffic; the binding fraction "
-                             "is int_roofline.ntt_passes.frac"},
+                     "note": "bound by the integer multiply pipe and its latency, not HBM; int_roofline.ntt_passes.frac "
+                             "credits the radix-2 transform's twiddle products (the radix-16 passes execute fewer)"},
         "int_roofline": {
             # denominator: Montgomery products per second of the library's own product routine
             # (zkp_mont_probe, measured in this run); the raw IMAD rate is listed beside it
