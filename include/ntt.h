@@ -64,11 +64,11 @@ cudaError_t zkp_coset_lde(PolyPtr out, ConstPolyPtr in, const unsigned int *twid
 cudaError_t zkp_ntt_shoup_table(const unsigned int *twiddle_d, unsigned int log_len, unsigned int *table_d,
                                 cudaStream_t stream);
 
-/* zkp_ntt_ex and zkp_coset_lde whose register passes (the passes of at most 2^6-point pencils
- * that make up the plan of every transform above 2^6 points) multiply by the twiddles of
- * shoup_d, a zkp_ntt_shoup_table of the same twiddle table: 207 multiply instructions per
- * twiddle product instead of the Montgomery product's 256, identical results.  twiddle is
- * still read by the other passes; shoup_d = NULL gives zkp_ntt_ex / zkp_coset_lde. */
+/* zkp_ntt_ex and zkp_coset_lde with a zkp_ntt_shoup_table of the same twiddle table: the register
+ * passes of transforms from 2^18 points multiply by its entries, 207 multiply instructions per
+ * twiddle product instead of the Montgomery product's 256, identical results.  Smaller transforms
+ * and the tensor-core passes read the Montgomery table, whose entries are half as long; twiddle is
+ * always needed.  shoup_d = NULL gives zkp_ntt_ex / zkp_coset_lde. */
 cudaError_t zkp_ntt_ex_shoup(PolyPtr x, const unsigned int *twiddle, const unsigned int *shoup_d,
                              unsigned int log_len, const unsigned int *shift_d, const unsigned int *scale_d,
                              cudaStream_t stream);

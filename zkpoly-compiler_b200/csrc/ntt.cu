@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(256) ntt_warp_pass_kernel(PassArgs a) {
 // zkp_ntt_set_block (0 = 128)
 std::atomic<u32> g_warp_block[29];
 
-// Up to this size the passes load their twiddles a stage ahead (2^10 16.6 -> 13 us, 2^14 26.7 ->
+// Up to this size the passes load their twiddles a stage ahead (2^10 16.6 -> 12.4 us, 2^14 26.7 ->
 // 18.5, 2^16 36 -> 28); above it the lost occupancy costs more (2^18 66 -> 70 us, 2^22 818 -> 853).
 constexpr u32 AHEAD_MAX_L = 17;
 
@@ -374,7 +374,10 @@ cudaError_t launch_warp_pass_as(const PassArgs &a, cudaStream_t stream) {
 }
 template <bool SH>
 cudaError_t launch_warp_pass(const PassArgs &a, cudaStream_t stream) {
-    return a.L <= AHEAD_MAX_L ? launch_warp_pass_as<SH, true>(a, stream) : launch_warp_pass_as<SH, false>(a, stream);
+    if constexpr (!SH) {  // run() drops the Shoup table at these sizes
+        if (a.L <= AHEAD_MAX_L) return launch_warp_pass_as<false, true>(a, stream);
+    }
+    return launch_warp_pass_as<SH, false>(a, stream);
 }
 
 // Shoup table entry e = (w^e plain, floor(w^e 2^256 / m)) from the Montgomery table entry e
@@ -682,12 +685,12 @@ inline void split_digits(Plan &p, u32 first, u32 L, u32 cap) {
 }
 
 // From this size table-mode transforms over 32-byte aligned buffers run radix-16 passes on the
-// integer tensor cores (ntt_umma.cuh), between register passes: 2^21 403 -> 376 us, 2^22 816 -> 752,
-// 2^24 3438 -> 2917; at 2^20 the constants' set-up and half-filled CTAs make them slower (209 -> 219).
+// integer tensor cores (ntt_umma.cuh), between register passes: 2^21 403 -> 368 us, 2^22 816 -> 738,
+// 2^24 3438 -> 2833; at 2^20 the constants' set-up and half-filled CTAs make them slower (209 -> 219).
 constexpr u32 UM_MIN_L = 21;
 inline bool aligned32(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 31) == 0; }
-inline bool umma_ok(u32 L, const View &v, const u32 *tw, const u32 *shoup) {
-    return L >= UM_MIN_L && tw != nullptr && aligned32(v.base) && aligned32(tw) && aligned32(shoup);
+inline bool umma_ok(u32 L, const View &v, const u32 *tw) {
+    return L >= UM_MIN_L && tw != nullptr && aligned32(v.base) && aligned32(tw);
 }
 // [register pass over the top 1 or 2 bits where needed,] radix-16 passes, and a last register pass
 // of 2^4 or 2^5 points with the tiled bit reversal
@@ -810,7 +813,10 @@ cudaError_t launch_last_bitrev_d(const PassArgs &a, cudaStream_t stream) {
 
 template <bool SH>
 cudaError_t launch_last_bitrev(const PassArgs &a, cudaStream_t stream) {
-    if (a.D == SMALL_TILE && a.L <= SMALL_TILE_MAX_L) return launch_last_bitrev_d<SMALL_TILE, SH, SMALL_TILE>(a, stream);
+    if constexpr (!SH) {  // run() drops the Shoup table at these sizes
+        if (a.D == SMALL_TILE && a.L <= SMALL_TILE_MAX_L)
+            return launch_last_bitrev_d<SMALL_TILE, false, SMALL_TILE>(a, stream);
+    }
     switch (a.D) {
         case 1: return launch_last_bitrev_d<1, SH, BR_T>(a, stream);
         case 2: return launch_last_bitrev_d<2, SH, BR_T>(a, stream);
@@ -822,7 +828,7 @@ cudaError_t launch_last_bitrev(const PassArgs &a, cudaStream_t stream) {
 
 template <bool SH>
 cudaError_t prepare_last_bitrevs() {
-    ZK_TRY((prepare_last_bitrev<SMALL_TILE, SH, SMALL_TILE>()));
+    if constexpr (!SH) ZK_TRY((prepare_last_bitrev<SMALL_TILE, false, SMALL_TILE>()));
     ZK_TRY((prepare_last_bitrev<1, SH, BR_T>()));
     ZK_TRY((prepare_last_bitrev<2, SH, BR_T>()));
     ZK_TRY((prepare_last_bitrev<3, SH, BR_T>()));
@@ -830,17 +836,15 @@ cudaError_t prepare_last_bitrevs() {
     return prepare_last_bitrev<5, SH, BR_T>();
 }
 
-template <bool SH>
 cudaError_t prepare_umma() {
     static std::atomic<uint64_t> done{0};
-    return ensure_smem_attr(ntt_umma_kernel<SH>, (int)UM_SMEM, done);
+    return ensure_smem_attr(ntt_umma_kernel, (int)UM_SMEM, done);
 }
-template <bool SH>
 cudaError_t launch_umma(const PassArgs &a, cudaStream_t stream) {
-    ZK_TRY(prepare_umma<SH>());
+    ZK_TRY(prepare_umma());
     const u32 items = 1u << (a.L - UM_D - 7);
     const u32 grid = items < (u32)num_sms() ? items : (u32)num_sms();
-    ntt_umma_kernel<SH><<<grid, UM_GROUPS * 128, UM_SMEM, stream>>>(a, items);
+    ntt_umma_kernel<<<grid, UM_GROUPS * 128, UM_SMEM, stream>>>(a, items);
     return cudaGetLastError();
 }
 
@@ -848,8 +852,7 @@ cudaError_t launch_umma(const PassArgs &a, cudaStream_t stream) {
 inline cudaError_t prepare_run_attrs() {
     ZK_TRY(ensure_smem_attr(ntt_pass_kernel, (int)pass_smem(MAX_D), g_attr_done));
     ZK_TRY(ensure_smem_attr(bitrev_tiled_kernel, (int)BR_SMEM, g_br_attr_done));
-    ZK_TRY(prepare_umma<false>());
-    ZK_TRY(prepare_umma<true>());
+    ZK_TRY(prepare_umma());
     ZK_TRY(prepare_last_bitrevs<false>());
     return prepare_last_bitrevs<true>();
 }
@@ -857,6 +860,9 @@ inline cudaError_t prepare_run_attrs() {
 // Runs the full plan.  src (if non-null) is the pass-0 source for the coset LDE.
 cudaError_t run(const View &v, const View *src, u64 src_len, u32 L, const u32 *tw, const u32 *omegas,
                 const u32 *shift, const u32 *scale, cudaStream_t stream, const u32 *shoup = nullptr) {
+    // small transforms wait for their twiddle loads, and a Montgomery root is half a Shoup pair's
+    // bytes (2^16 30.2 -> 27.9 us)
+    if (L <= AHEAD_MAX_L) shoup = nullptr;
     profiler().begin(stream);
     if (omegas == nullptr && (shift != nullptr || src != nullptr) && L >= PREP_MIN_L) {
         // a multi-pass table-mode plan: shift and zero-extend in one elementwise pass, then the
@@ -875,7 +881,7 @@ cudaError_t run(const View &v, const View *src, u64 src_len, u32 L, const u32 *t
         src = nullptr;
         src_len = 0;
     }
-    const bool um = shift == nullptr && src == nullptr && omegas == nullptr && umma_ok(L, v, tw, shoup);
+    const bool um = shift == nullptr && src == nullptr && omegas == nullptr && umma_ok(L, v, tw);
     const Plan plan = um ? umma_plan(L) : make_plan(L, shift != nullptr || src != nullptr, omegas != nullptr);
     const bool fused_tail = fuse_last(plan, L, omegas != nullptr);
     for (u32 p = 0; p < plan.np; p++) {
@@ -907,7 +913,7 @@ cudaError_t run(const View &v, const View *src, u64 src_len, u32 L, const u32 *t
             profiler().mark("ntt_pass", stream);
             return cudaSuccess;
         }
-        if (um && a.D == UM_D) ZK_TRY(shoup ? launch_umma<true>(a, stream) : launch_umma<false>(a, stream));
+        if (um && a.D == UM_D && a.lo > 0) ZK_TRY(launch_umma(a, stream));
         else ZK_TRY(launch_pass(a, stream));
         profiler().mark("ntt_pass", stream);
     }

@@ -19,7 +19,7 @@
 // products the other two read theirs and multiply by twiddles.
 //
 // Measured at 2^24: 0.44 ms a pass (the first, whose roots come from DRAM, 0.58) for four bits, where
-// the register pass takes 0.70 for five; the whole transform 3.39 -> 2.92 ms.  At 2^22 the multiply
+// the register pass takes 0.70 for five; the whole transform 3.39 -> 2.83 ms.  At 2^22 the multiply
 // pipe is 62 % busy, the tensor pipe 10 %, DRAM 26 %: what bounds it is the latency of each warp's
 // chain with three warps a scheduler.  Four groups need 128 registers a thread and spill (3.43 ms);
 // keeping the even half's sums in memory instead of registers avoids that but costs more (3.31 ms
@@ -194,8 +194,9 @@ ZK_DI void um_pencil(u64 item, u32 row, u32 lo, u32 log_h, u64 &c, u64 &h) {
     c = ((item & ((1ull << (lo - cb)) - 1)) << cb) | ((row >> (2 + hb)) << 2) | (row & 3);
 }
 
-// SH: twiddles from the Shoup table
-template <bool SH>
+// The twiddle product is the Montgomery one also for callers with a Shoup table: these passes wait
+// for loads more than for the multiply pipe, and its root is 32 bytes, not 64 (2^24 2.92 -> 2.83 ms,
+// 2^22 0.752 -> 0.738).
 __global__ void __launch_bounds__(UM_GROUPS * 128, 1) ntt_umma_kernel(const PassArgs a, u32 items) {
     extern __shared__ __align__(1024) unsigned char um_sm[];
     const u32 tid = threadIdx.x, g = tid >> 7, row = tid & 127;
@@ -271,32 +272,19 @@ __global__ void __launch_bounds__(UM_GROUPS * 128, 1) ntt_umma_kernel(const Pass
     u64 base = 0, c = 0;
     const u64 half = 1ull << (L - 1);
     const u32 esh = L - lo - UM_D;
-    struct Root {
-        Fr w, ws;
-    };
-    auto root = [&](u32 k) {
-        Root r;
-        const u64 ei = ((c * k) << esh) & (half - 1);
-        if (SH) {
-            r.w = um_ld_nc(a.shoup + ei * 16);
-            r.ws = um_ld_nc(a.shoup + ei * 16 + 8);
-        } else {
-            r.w = um_ld_nc(a.tw + ei * 8);
-        }
-        return r;
-    };
+    auto root = [&](u32 k) { return um_ld_nc(a.tw + (((c * k) << esh) & (half - 1)) * 8); };
     // outputs k = k0, k0 + dk, ... (four of them) from the group's TMEM columns; an output's twiddle
     // is loaded one output ahead
-    auto drain = [&](u32 k0, u32 dk, Root r) {
+    auto drain = [&](u32 k0, u32 dk, Fr r) {
 #pragma unroll 1
         for (u32 o = 0; o < 4; o++) {
             const u32 k = k0 + o * dk;
             u32 cs[32];
             um_load32(tmem_row + o * 32, cs);
-            const Root next = root(k + dk);  // past the last one: in range, unused
+            const Fr next = root(k + dk);  // past the last one: in range, unused
             Fr x = um_combine(cs);
             if (k != 0) {
-                x = SH ? Fr::mul_shoup(x, r.w, r.ws) : Fr::mul(x, r.w);
+                x = Fr::mul(x, r);
                 if (((c * k) << esh) >= half) {  // w^(n/2) = -1
                     Fr m2;
 #pragma unroll
@@ -323,7 +311,7 @@ __global__ void __launch_bounds__(UM_GROUPS * 128, 1) ntt_umma_kernel(const Pass
         }
         um_fence_async();
         issue(0, 0, 4096, 8);  // outputs 1, 3, 5, 7
-        Root r = root(1);
+        Fr r = root(1);
         finish();
         drain(1, 2, r);
         issue(0, 128 * 16, 4096, 8);  // outputs 9, 11, 13, 15
