@@ -29,9 +29,9 @@ sys.path.insert(0, ROOT)
 
 METRIC = "MSM points/s (2^22) & NTT elems/s (2^24); served p50/p99 vs plain per-call"
 MSM_LOG, NTT_LOG = 22, 24
-# ncu DRAM bytes (read + write) of one whole 2^24 transform (all five passes) per element, from the
-# capture summarised in profiles/ntt_passes_ntt2p24.md
-NTT_TRAFFIC_PER_ELEM = 398.0
+# ncu DRAM bytes (read + write) of one whole 2^24 transform (all six passes) per element, from the
+# capture summarised in profiles/ntt_umma_passes_ntt2p24.md
+NTT_TRAFFIC_PER_ELEM = 471.0
 
 
 def workload_config(world: int) -> dict:
@@ -1010,16 +1010,15 @@ def emit(args, zk, rank, world, n_msm, n_ntt, ntt_ms, msm_ms, step_ms, pass_ms, 
         "ntt": {"metric": f"NTT elems/s (2^{NTT_LOG})", "value": world * n_ntt / (ntt_ms / 1e3), "unit": "elems/s",
                 "ms": ntt_ms, "pass_ms": pass_avg, "bitrev_ms": statistics.median(bitrev_ms) if bitrev_ms else None,
                 "hbm_frac_whole_ntt": (64 * n_ntt / (ntt_ms / 1e3) / 1e9) / hbm_peak,
-                "path": "zkp_ntt_ex_shoup: radix-16 passes on the integer tensor cores and register passes, Shoup "
-                        "twiddle products (root table + Shoup table of 64 B per root, both built once "
-                        "outside the timed region)",
+                "path": "zkp_ntt_ex_shoup: radix-16 passes on the integer tensor cores (Montgomery roots) and a last "
+                        "register pass (Shoup roots); both root tables built once outside the timed region",
                 "ssip_ms": ssip_ms, "ssip_value": world * n_ntt / (ssip_ms / 1e3) if ssip_ms else None,
                 "ssip_path": "ssip_ntt (reference ABI): the same passes with Montgomery twiddle products"},
         # the NTT's HBM roofline: 64 B per element (one read + one write
         # of the vector) for the whole transform, over the transform's CUDA-event time
         "roofline": {"kernel": f"NTT 2^{NTT_LOG} forward transform: {len(digits)} passes (ntt_umma_kernel "
                                f"radix-16 passes, the last a register pass fused with the bit reversal in "
-                               f"ntt_last_bitrev_kernel), digits {digits}, Shoup twiddle products",
+                               f"ntt_last_bitrev_kernel), digits {digits}",
                      "bound": "imad", "achieved": ntt_alg_gbs, "peak": hbm_peak, "unit": "GB/s",
                      "frac": ntt_alg_gbs / hbm_peak, "peak_source": peak_kind,
                      "bytes_per_launch": ntt_alg_bytes, "launch": "one whole transform (all passes)",

@@ -18,8 +18,8 @@
 // per TMEM lane), 32 KB of A and 128 TMEM columns (four outputs), so while one group waits for its
 // products the other two read theirs and multiply by twiddles.
 //
-// Measured at 2^24: 0.44 ms a pass (the first, whose roots come from DRAM, 0.58) for four bits, where
-// the register pass takes 0.70 for five; the whole transform 3.39 -> 2.83 ms.  At 2^22 the multiply
+// Measured at 2^24: 0.44 ms a pass (the first, whose roots come from DRAM, 0.51) for four bits, where
+// the register pass takes 0.70 for five; the whole transform 3.39 -> 2.84 ms.  At 2^22 the multiply
 // pipe is 62 % busy, the tensor pipe 10 %, DRAM 26 %: what bounds it is the latency of each warp's
 // chain with three warps a scheduler.  Four groups need 128 registers a thread and spill (3.43 ms);
 // keeping the even half's sums in memory instead of registers avoids that but costs more (3.31 ms
