@@ -308,3 +308,33 @@ def test_msm_reduction_small_windows(zk, orc, window):
         dev_s = torch.from_numpy(s[:m].view(np.int32).reshape(m, 8).copy()).cuda()
         b.msm(dev_s, res, b.workspace())
         assert np.array_equal(res.cpu().numpy().view(np.uint64), orc.best_multiexp(s[:m], p[:m])), m
+
+
+@pytest.mark.parametrize("n,window,n_tables,rounds,held", [
+    (100, 8, 32, -1, 165888), (700, 5, 1, -1, 1732096), (4096, 15, 17, -1, 6274304), (5000, 0, 1, -1, 7755008),
+    (4096, 8, 1, 2, 11923200)])
+def test_msm_in_the_smaller_workspace(zk, orc, n, window, n_tables, rounds, held):
+    """A workspace with room for one partial sum per eight list entries (`held` bytes, less than the
+    size query asks for) serves too, single and as a batch, with the same result and nothing written
+    past its end; far smaller ones are refused."""
+    p, s = orc.gen_points(410, n), orc.gen_fr(411, n)
+    expect = orc.best_multiexp(s, p)
+    dev_s = torch.from_numpy(s.view(np.int32).reshape(n, 8).copy()).cuda()
+    zk.msm.set_affine_rounds(rounds)
+    try:
+        bases = zk.msm.ResidentBases(p, window=window, n_tables=n_tables)
+        assert held < bases.ws_bytes
+        guard = torch.full((held + 4096,), 0x5A, dtype=torch.uint8, device="cuda")
+        res = torch.zeros(16, dtype=torch.int32, device="cuda")
+        bases.msm(dev_s, res, guard[:held])
+        assert np.array_equal(res.cpu().numpy().view(np.uint64), expect)
+        batch = zk.msm.MsmBatch([{"points": bases.tables, "n_tables": n_tables, "scalars": dev_s, "n": n,
+                                  "window": bases.window, "result": res.zero_()}])
+        batch.workspace, batch.ws_bytes = guard, held
+        batch.run()
+        assert np.array_equal(res.cpu().numpy().view(np.uint64), expect)
+        assert bool((guard[held:] == 0x5A).all())
+        with pytest.raises(Exception):
+            bases.msm(dev_s, res, guard[: held // 2])
+    finally:
+        zk.msm.set_affine_rounds(-1)

@@ -93,7 +93,7 @@ ZK_DI u32 find_task(const T *first, u32 ntasks, T x) {
 }
 
 // CTAs per bit class in the bucket reduction (a power of two); scale_kernel and window_kernel
-// fold up to 32 parts and 32 classes, one per lane
+// fold up to 32 parts and 32 classes, eight quads of a warp at a time
 constexpr u32 MAX_PARTS = 32, CLASS_ITEMS = 256, CLASS_CTAS = 4;
 
 inline Task make_task(u64 n, u32 c, u32 n_tables) {
@@ -171,14 +171,27 @@ inline u64 next_list_bound(u64 e, u64 nb) {
 // as rarely as that allows (every cut leaves a chain to the fix-up), but at least walk_min entries.
 // The length is computed on the device from the list's real length: digits that are zero and pairs
 // already added shorten it below what the host can know.
-constexpr u32 WALK_THREADS = 512, WALK_MIN = 4;
+// walk_min: 4 entries where the workspace has room for that many partial sums (2^12 points 222 us,
+// 233 with 8), 8 in a workspace of the smaller size that callers may hold (WALK_TIGHT).
+constexpr u32 WALK_THREADS = 512, WALK_MIN = 4, WALK_TIGHT = 8;
 ZK_DI u32 walk_chunk(u32 live, u32 walkers, u32 walk_min) {
     const u32 k = live / walkers + (live % walkers ? 1 : 0);
     return k < walk_min ? walk_min : k;
 }
 
+// parts per class that the layout's own class region always has room for: one per 2048 segment sums
+inline u32 usual_parts(const Batch &b) {
+    u32 few = 1;
+    for (u32 t = 0; t < b.ntasks; t++) {
+        const u32 p = b.task[t].B / b.task[t].L / 2 / 2048;
+        few = p > few ? (p < MAX_PARTS ? p : MAX_PARTS) : few;
+    }
+    return few;
+}
+
 // fills the prefixes and the launch shapes; tasks[] must be set.  rounds < 0: the library
-// setting (itself -1 = by size).
+// setting (itself -1 = by size).  walk_min WALK_TIGHT: nothing may need more workspace than one
+// partial sum per eight entries and the usual class parts.
 inline void finish_batch(Batch &b, int rounds = -1, u32 walk_min = WALK_MIN) {
     b.sc_first[0] = b.key_first[0] = b.seg_first[0] = 0;
     b.win_first[0] = 0;
@@ -204,6 +217,12 @@ inline void finish_batch(Batch &b, int rounds = -1, u32 walk_min = WALK_MIN) {
         k.parts = 1;
         while (k.parts < MAX_PARTS && half / (2 * k.parts) >= CLASS_ITEMS && 2 * k.parts <= most) k.parts *= 2;
         b.nparts = b.nparts > k.parts ? b.nparts : k.parts;
+    }
+    const u32 few = usual_parts(b);
+    if (walk_min == WALK_TIGHT && b.nparts > few &&
+        (u64)b.win_first[b.ntasks] * b.ncls * b.nparts * 128 > (b.key_first[b.ntasks] + 1) * 4) {  // see make_layout
+        for (u32 t = 0; t < b.ntasks; t++) b.task[t].parts = b.task[t].parts < few ? b.task[t].parts : few;
+        b.nparts = few;
     }
     if (rounds < 0) rounds = affine_rounds_setting();
     b.rounds = rounds < 0 ? auto_rounds(entries) : (u32)(rounds > (int)MAX_ROUNDS ? MAX_ROUNDS : rounds);
@@ -265,9 +284,10 @@ inline Layout make_layout(const Batch &b) {
     }
     l.chunks = (l.emax[l.rounds] + b.walk_min - 1) / b.walk_min;  // most that walk_chunk can ask for
     if (l.chunks > b.walkers) l.chunks = b.walkers;
-    // Room for at least one chunk per eight entries, up to four waves of 384 threads an SM: what the
-    // partial sums have always taken.  zkp_msm_device_noalloc decides by the total which sizes fit
-    // its fixed array, and that limit is part of its interface.
+    // Room for at least one chunk per eight entries, up to four waves of 384 threads an SM: with
+    // WALK_TIGHT the total is then never above what it was before shorter chunks, so a workspace of
+    // that size still serves, and zkp_msm_device_noalloc, which decides by the total which sizes fit
+    // its fixed array, takes the same ones.
     const u64 waves = (u64)num_sms() * 384 * 4, per = (l.emax[l.rounds] + waves - 1) / waves;
     const u64 usual = (l.emax[l.rounds] + (per < 8 ? 8 : per) - 1) / (per < 8 ? 8 : per);
     const u64 room = l.chunks > usual ? l.chunks : usual;
@@ -296,32 +316,39 @@ inline Layout make_layout(const Batch &b) {
             for (u32 r = 1; r < l.rounds; r++) l.prefix[r] = at1;
         }
         l.tvals = take(l.thr[0] * 32);
-        u64 m = l.thr[0];
-        for (u32 k = 0; k <= TREE_LEVELS; k++) l.tree_pre[k] = l.tree_es[k] = l.tree_dat[k] = 0;
-        for (u32 k = 0; k <= TREE_LEVELS; k++) {
-            l.tree_pre[k] = take(m * 32);  // the top level uses only this one
-            if (m <= TREE_SPAN) break;
-            const u64 ctas = (m + TREE_SPAN - 1) / TREE_SPAN;
-            l.tree_es[k] = take(ctas * TREE_CTA * 32);
-            m = ctas;
-            l.tree_dat[k + 1] = take(m * 32);
-        }
+        l.tree_pre[0] = take(l.thr[0] * 32);
     }
     l.bucket_sums = take(l.nb * 128);
     l.part_pts = take(room * 2 * 128);
+    if (l.rounds) {
+        // The tree's other arrays (4.1 bytes a thread total, 64 list elements each) lie where the walk
+        // writes its partial sums once the rounds are done: 256 bytes per eight entries of the last
+        // list, which is at least a sixteenth of the first.
+        size_t at = l.part_pts;
+        auto borrow = [&](size_t bytes) {
+            const size_t o = at;
+            at += align_up(bytes);
+            return o;
+        };
+        u64 m = l.thr[0];
+        for (u32 k = 0; k <= TREE_LEVELS; k++) {
+            if (k) l.tree_pre[k] = borrow(m * 32);  // the top level uses only this one
+            if (m <= TREE_SPAN) break;
+            const u64 ctas = (m + TREE_SPAN - 1) / TREE_SPAN;
+            l.tree_es[k] = borrow(ctas * TREE_CTA * 32);
+            m = ctas;
+            l.tree_dat[k + 1] = borrow(m * 32);
+        }
+        if (at > off) off = at;  // not reached: see above
+    }
     l.part_bucket = take(room * 2 * 4);
     l.part_flag = take(room * 2 * 4);
     l.long_list = take((room + 1) * 4 + 4);  // long chain starts + a counter at the end
     l.chain_list = take((room + 1) * 4);     // chain starts + a counter at the end
     l.seg = take(2 * l.segs * 128);  // U_g then T_g
-    // class parts: room for one part per 2048 segment sums, as ever; more parts than that go where the
-    // cursors were (last used by the pairing rounds), if they fit there
-    u32 few = 1;
-    for (u32 t = 0; t < b.ntasks; t++) {
-        const u32 p = b.task[t].B / b.task[t].L / 2 / 2048;
-        few = p > few ? (p < MAX_PARTS ? p : MAX_PARTS) : few;
-    }
-    const size_t cls_usual = l.wins * b.ncls * few * 128, cls_bytes = l.wins * b.ncls * b.nparts * 128;
+    // class parts: the usual ones have room of their own; more than those go where the cursors were
+    // (last used by the pairing rounds), if they fit there
+    const size_t cls_usual = l.wins * b.ncls * usual_parts(b) * 128, cls_bytes = l.wins * b.ncls * b.nparts * 128;
     const bool in_cursor = cls_bytes > cls_usual && cls_bytes <= (l.nb + 1) * 4;
     const size_t cls_at = take(in_cursor || cls_bytes < cls_usual ? cls_usual : cls_bytes);
     l.cls = in_cursor ? l.cursor : cls_at;
@@ -1459,6 +1486,18 @@ inline Batch single(const u32 *points, u32 n_tables, const u32 *scalars, u64 n, 
     return b;
 }
 
+// The plan for a workspace of `bytes`: plan(walk_min) sets up the batch, with short walk chunks where
+// the workspace has room for them and the chunks of WALK_TIGHT where it has not.
+template <class F>
+inline cudaError_t plan_within(u64 bytes, const F &plan, Batch *b, Layout *l) {
+    for (const u32 walk_min : {WALK_MIN, WALK_TIGHT}) {
+        ZK_TRY(plan(walk_min, b));
+        *l = make_layout(*b);
+        if (l->total <= bytes) return cudaSuccess;
+    }
+    return cudaErrorInvalidValue;
+}
+
 }  // namespace msm
 }  // namespace zk
 
@@ -1564,15 +1603,19 @@ extern "C" cudaError_t zkp_msm_device(void *workspace_d, unsigned long long work
     msm::resolve(n, window, n_tables, &c, &nt);
     ZK_CHECK_ARG(c >= 2 && c <= 24 && nt >= 1);
     ZK_CHECK_ARG(n * nt < (1ull << 31));
-    const msm::Batch b = msm::single(points_d, nt, scalars_d, n, c, result_d);
-    ZK_CHECK_ARG(msm::batch_fits(b));
-    const msm::Layout l = msm::make_layout(b);
-    ZK_CHECK_ARG(workspace_bytes >= l.total);
+    msm::Batch b;
+    msm::Layout l;
+    ZK_TRY(msm::plan_within(workspace_bytes, [&](u32 walk_min, msm::Batch *out) {
+        *out = msm::single(points_d, nt, scalars_d, n, c, result_d, -1, walk_min);
+        ZK_CHECK_ARG(msm::batch_fits(*out));
+        return cudaSuccess;
+    }, &b, &l));
     return msm::run_batch(b, l, reinterpret_cast<char *>(workspace_d), stream);
 }
 
 // batches of more than MAX_TASKS are not split here; the caller chunks them
-static cudaError_t build_batch(const ZkpMsmTask *tasks, unsigned int ntasks, msm::Batch *out) {
+static cudaError_t build_batch(const ZkpMsmTask *tasks, unsigned int ntasks, msm::Batch *out,
+                               u32 walk_min = msm::WALK_MIN) {
     ZK_CHECK_ARG(ntasks >= 1 && ntasks <= msm::MAX_TASKS && tasks != nullptr);
     msm::Batch b{};
     b.ntasks = ntasks;
@@ -1589,7 +1632,7 @@ static cudaError_t build_batch(const ZkpMsmTask *tasks, unsigned int ntasks, msm
         b.task[t].scalars = k.scalars_d;
         b.task[t].result = k.result_d;
     }
-    msm::finish_batch(b);
+    msm::finish_batch(b, -1, walk_min);
     ZK_CHECK_ARG(msm::batch_fits(b));
     *out = b;
     return cudaSuccess;
@@ -1604,9 +1647,11 @@ extern "C" unsigned long long zkp_msm_batch_workspace_size(const ZkpMsmTask *tas
 extern "C" cudaError_t zkp_msm_batch(const ZkpMsmTask *tasks, unsigned int ntasks, void *workspace_d,
                                      unsigned long long workspace_bytes, cudaStream_t stream) {
     msm::Batch b;
-    ZK_TRY(build_batch(tasks, ntasks, &b));
-    const msm::Layout l = msm::make_layout(b);
-    ZK_CHECK_ARG(workspace_d != nullptr && workspace_bytes >= l.total);
+    msm::Layout l;
+    ZK_CHECK_ARG(workspace_d != nullptr);
+    ZK_TRY(msm::plan_within(workspace_bytes, [&](u32 walk_min, msm::Batch *out) {
+        return build_batch(tasks, ntasks, out, walk_min);
+    }, &b, &l));
     return msm::run_batch(b, l, reinterpret_cast<char *>(workspace_d), stream);
 }
 
@@ -1648,7 +1693,8 @@ static CardLayout card_layout(u64 cnt, u32 c, u32 nt, char *base) {
     u32 *res = base ? reinterpret_cast<u32 *>(base + cl.result) : nullptr;
     for (int i = 0; i < 2; i++) {
         u32 *sc = base ? reinterpret_cast<u32 *>(base + cl.scalars[i]) : nullptr;
-        cl.batch[i] = msm::single(pts, nt, sc, cnt, c, res);
+        // the smaller layout: this entry's run does not see its buffers' sizes
+        cl.batch[i] = msm::single(pts, nt, sc, cnt, c, res, -1, msm::WALK_TIGHT);
     }
     cl.l = msm::make_layout(cl.batch[0]);
     cl.total = off + cl.l.total;
@@ -1885,9 +1931,9 @@ extern "C" cudaError_t zkp_msm_device_noalloc(const unsigned int *points_d, unsi
     msm::resolve(n, window, n_tables, &c, &nt);
     ZK_CHECK_ARG(c >= 2 && c <= 24 && nt >= 1);
     ZK_CHECK_ARG(n * nt < (1ull << 31));
-    // no pairing rounds and no walk chunks below 8 entries: their lists and partial sums would not
-    // fit the fixed scratch
-    const msm::Batch b = msm::single(points_d, nt, scalars_d, n, c, result_d, 0, 8);
+    // no pairing rounds and no short walk chunks: their lists and partial sums would not fit the
+    // fixed scratch
+    const msm::Batch b = msm::single(points_d, nt, scalars_d, n, c, result_d, 0, msm::WALK_TIGHT);
     ZK_CHECK_ARG(msm::batch_fits(b));
     const msm::Layout l = msm::make_layout(b);
     // larger problems do not fit the fixed scratch: refuse instead of overrunning it
