@@ -229,3 +229,35 @@ def test_permute_key_shapes(zk, orc, n, kind):
     ei, et = orc.permute(inp, table, usable)
     assert np.array_equal(ri.numpy_u64(), ei)
     assert np.array_equal(rt.numpy_u64(), et)
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 5, 6, 7, 8, 9, 16, 17, 63, 64, 65, 66, 127, 129, 513])
+def test_sweeps_of_few_chunks(zk, orc, n):
+    """One CTA whose scans stop at the chunks there are: one chunk, part of a warp, one more than a
+    warp's, several warps; zeros at both ends for the inversion."""
+    a = orc.gen_fr(19, n)
+    x = orc.gen_fr(20, 1)[0]
+    res = torch.zeros((1, 8), dtype=torch.int32, device="cuda")
+    zk.poly.poly_eval(dev(zk, a), scal(zk, x), res)
+    assert np.array_equal(res.cpu().numpy().view(np.uint64)[0], orc.eval_poly(a, x))
+    for zeros in ([], [0], [n - 1], list(range(n))):
+        z = a.copy()
+        z[zeros] = 0
+        t = dev(zk, z)
+        zk.poly.batched_invert(t)
+        assert np.array_equal(t.numpy_u64(), orc.batch_invert(z)), zeros
+    t = dev(zk, a)
+    zk.poly.scan_mul(t)
+    acc, expect = 1, []
+    for v in ints(orc, a):
+        acc = acc * v % M
+        expect.append(acc)
+    assert ints(orc, t.numpy_u64()) == expect
+    if n & (n - 1) == 0:
+        q = zk.ScalarArray.zeros(n)
+        zk.poly.kate_division(dev(zk, a), scal(zk, x), q)
+        b, p, acc, expect = ints(orc, x[None])[0], ints(orc, a), 0, []
+        for i in reversed(range(n)):
+            acc = (acc * b + (p[i + 1] if i + 1 < n else 0)) % M
+            expect.append(acc)
+        assert ints(orc, q.numpy_u64()) == expect[::-1]

@@ -51,6 +51,13 @@ inline u32 top_chunk(u64 m) {
     return c;
 }
 inline u32 log2_of(u32 c) { return 31 - __builtin_clz(c); }
+// the sweeps that walk their elements twice: up to four elements are one chunk, walked by one thread
+inline u32 walk_chunk_for(u64 n) { return n <= 4 ? 4 : chunk_for(n); }
+// One warp where its lanes hold all the chunks (SMALL kernels).  Its scans then stop at the chunks there
+// are, which for a handful of elements is most of the chain (1 / 8 elements through a whole CTA's
+// steps, by one thread, and here: product scan 7.3 / 8.4, 2.3 / 8.1 and 2.1 / 4.2 us, division 13.5 / 14.6,
+// 2.0 / 7.0 and 2.2 / 5.2, inversion 45 / 48, 35 / 49 and 21 / 26).
+inline bool one_warp(u64 n, u32 c) { return n <= 32ull * c; }
 inline u64 ctas_for(u64 n, u32 c) { return (n + (u64)CTA * c - 1) / ((u64)CTA * c); }
 
 inline u32 grid_for(u64 items, u32 block, u32 per_sm = 16) {
@@ -165,6 +172,17 @@ ZK_DI void cta_products(const Fr &v, u32 *sm, Fr &e, Fr &f, Fr &total) {
     __syncthreads();
 }
 
+// the same for a CTA of one warp whose first `chunks` lanes hold values (ones after them)
+template <bool BOTH>
+ZK_DI void warp_products(const Fr &v, u32 chunks, Fr &e, Fr &f, Fr &total) {
+    const u32 lane = threadIdx.x & 31;
+    Fr x = v, y = v;
+    lane_products<BOTH>(x, y, lane, chunks);
+    total = lane_get(x, chunks - 1);
+    e = pick(lane > 0, lane_get(x, lane - 1), Fr::one());
+    if (BOTH) f = pick(lane < 31, lane_get(y, lane + 1), Fr::one());
+}
+
 // ------------------------------------------------------------------ evaluation
 // out[cta] = sum over the CTA's CTA * c coefficients a_i X^(i - first); next_base = X^(CTA c), the
 // point of the next level.  A thread's chunk is a Horner chain, the chunks are joined by shuffles
@@ -235,7 +253,8 @@ __global__ void __launch_bounds__(CTA) scan_top_kernel(u32 *vals, u32 m, u32 c) 
         e = Fr::mul(e, v);
     }
 }
-// cta_ex null: a single CTA
+// cta_ex null: a single CTA; SMALL: it is one warp
+template <bool SMALL>
 __global__ void __launch_bounds__(CTA) scan_down_kernel(View data, u64 n, u32 c, const u32 *ex, const u32 *cta_ex) {
     __shared__ __align__(16) u32 sm[WARPS * 8];
     const u64 t = (u64)blockIdx.x * CTA + threadIdx.x, start = t * c;
@@ -245,7 +264,9 @@ __global__ void __launch_bounds__(CTA) scan_down_kernel(View data, u64 n, u32 c,
         acc = Fr::load(ex + t * 8);
     } else {
         Fr f, total;
-        cta_products<false>(chunk_product(data, n, start, c), sm, acc, f, total);
+        if (!SMALL) cta_products<false>(chunk_product(data, n, start, c), sm, acc, f, total);
+        else if (n <= c) acc = Fr::one();
+        else warp_products<false>(chunk_product(data, n, start, c), (u32)((n + c - 1) / c), acc, f, total);
         if (start >= n) return;
     }
     if (cta_ex) acc = Fr::mul(acc, Fr::load(cta_ex + (u64)blockIdx.x * 8));
@@ -305,7 +326,8 @@ __global__ void __launch_bounds__(CTA) inv_top_kernel(u32 *vals, u32 m, u32 c, u
         inv = Fr::mul(inv, v);
     }
 }
-// all of it for one CTA's elements; prefix: n elements
+// all of it for one CTA's elements (SMALL: a CTA of one warp); prefix: n elements
+template <bool SMALL>
 __global__ void __launch_bounds__(CTA) inv_one_kernel(View data, u32 n, u32 c, u32 *prefix) {
     __shared__ __align__(16) u32 sm[WARPS * 8];
     const u32 start = threadIdx.x * c, end = start + c < n ? start + c : n;
@@ -317,14 +339,16 @@ __global__ void __launch_bounds__(CTA) inv_one_kernel(View data, u32 n, u32 c, u
         acc = pick(a.is_zero(), acc, Fr::mul(acc, a));
     }
     Fr e, f, total;
-    cta_products<true>(acc, sm, e, f, total);
-    const Fr ef = Fr::mul(e, f);
+    const bool alone = SMALL && n <= c;  // one chunk: nothing before or after it
+    if (!SMALL) cta_products<true>(acc, sm, e, f, total);
+    else warp_products<true>(acc, (n + c - 1) / c, e, f, total);
+    const Fr ef = alone ? Fr::one() : Fr::mul(e, f);
     if (threadIdx.x < 32) {
         const Fr inv_all = inv_binary_quad<FrParams>(total);
         if (threadIdx.x == 0) inv_all.store(sm);
     }
     __syncthreads();
-    Fr inv = Fr::mul(Fr::load(sm), ef);
+    Fr inv = alone ? Fr::load(sm) : Fr::mul(Fr::load(sm), ef);
 #pragma unroll 2
     for (u32 i = end; i-- > start;) {
         u32 *p = data.at(i);
@@ -395,6 +419,17 @@ ZK_DI Fr cta_suffix(Fr v, const u32 *lad, u32 logc, const u32 *pw, u32 *sm, Fr &
     return Fr::add(Fr::mul(Fr::load(pw + (31 - lane) * 8), next), after);
 }
 
+// the same for a CTA of one warp whose first `chunks` lanes hold values (zeros after them)
+ZK_DI Fr warp_suffix(Fr v, const u32 *lad, u32 logc, u32 chunks) {
+    const u32 lane = threadIdx.x & 31;
+#pragma unroll 1
+    for (u32 s = 0; (1u << s) < chunks; s++) {
+        const Fr x = Fr::add(Fr::mul(lane_get(v, lane + (1u << s)), Fr::load(lad + (logc + s) * 8)), v);
+        v = pick(lane + (1u << s) < 32, x, v);
+    }
+    return pick(lane < 31, lane_get(v, lane + 1), Fr::zero());
+}
+
 // q at `start` from the chunk's own terms p[start + 1 .. end]
 ZK_DI Fr chunk_local(const View &p, u64 n, u64 start, u32 c, const Fr &B) {
     if (start >= n) return Fr::zero();
@@ -447,7 +482,9 @@ __global__ void __launch_bounds__(CTA) kate_top_kernel(u32 *vals, u32 m, const u
         in = Fr::add(Fr::mul(in, B), v);
     }
 }
-// carry null: recomputed as in the up pass (see the product scan); tab null: a single CTA
+// carry null: recomputed as in the up pass (see the product scan); tab null: a single CTA; SMALL: it is
+// one warp
+template <bool SMALL>
 __global__ void __launch_bounds__(CTA) kate_down_kernel(View p, View q, u64 n, const u32 *b, u32 c, u32 logc,
                                                         const u32 *carry, const u32 *cta_in, const u32 *tab) {
     __shared__ __align__(16) u32 lad[32 * 8], pw[32 * 8], sm[WARPS * 8];
@@ -458,6 +495,15 @@ __global__ void __launch_bounds__(CTA) kate_down_kernel(View p, View q, u64 n, c
     if (carry) {
         if (start >= n) return;
         acc = Fr::load(carry + t * 8);
+    } else if (SMALL) {
+        acc = Fr::zero();
+        if (n > c) {
+            const u32 chunks = (u32)((n + c - 1) / c);
+            power_ladder(B, logc + 32 - __clz(chunks - 1), lad);  // up to b^(c 2^(steps - 1))
+            __syncwarp();
+            acc = warp_suffix(chunk_local(p, n, start, c, B), lad, logc, chunks);
+        }
+        if (start >= n) return;
     } else {
         power_ladder(B, logc + 9, lad);
         __syncwarp();
@@ -571,7 +617,7 @@ extern "C" cudaError_t poly_eval(void *temp_buf, unsigned long *temp_buf_size, C
 extern "C" cudaError_t batched_invert(void *temp_buffer, unsigned long *buffer_size, PolyPtr poly,
                                       cudaStream_t stream) {
     const u64 n = poly.len;
-    const u32 c = chunk_for(n);
+    const u32 c = walk_chunk_for(n);
     const u64 m = ctas_for(n, c);
     const size_t need = al(n * 32) + 2 * al(m * 32);
     if (temp_buffer == nullptr) {
@@ -587,7 +633,8 @@ extern "C" cudaError_t batched_invert(void *temp_buffer, unsigned long *buffer_s
     u32 *tot = reinterpret_cast<u32 *>(base + al(n * 32));
     u32 *top_prefix = reinterpret_cast<u32 *>(base + al(n * 32) + al(m * 32));
     if (m == 1) {
-        inv_one_kernel<<<1, CTA, 0, stream>>>(v, (u32)n, c, prefix);
+        if (one_warp(n, c)) inv_one_kernel<true><<<1, 32, 0, stream>>>(v, (u32)n, c, prefix);
+        else inv_one_kernel<false><<<1, CTA, 0, stream>>>(v, (u32)n, c, prefix);
         return cudaGetLastError();
     }
     inv_up_kernel<<<(u32)m, CTA, 0, stream>>>(v, n, c, prefix, tot);
@@ -602,7 +649,7 @@ extern "C" cudaError_t batched_invert(void *temp_buffer, unsigned long *buffer_s
 // the chunks are of MAX_C elements or more
 extern "C" cudaError_t scan_mul(void *temp_buffer, unsigned long *buffer_size, PolyPtr target, cudaStream_t stream) {
     const u64 n = target.len;
-    const u32 c = chunk_for(n);
+    const u32 c = walk_chunk_for(n);
     const u64 m = ctas_for(n, c);
     const size_t keep = c >= MAX_C ? al(m * CTA * 32) : 0;
     const size_t need = al((m ? m : 1) * 32) + keep;
@@ -622,7 +669,8 @@ extern "C" cudaError_t scan_mul(void *temp_buffer, unsigned long *buffer_size, P
         scan_top_kernel<<<1, CTA, 0, stream>>>(tot, (u32)m, top_chunk(m));
         ZK_TRY(cudaGetLastError());
     }
-    scan_down_kernel<<<(u32)m, CTA, 0, stream>>>(v, n, c, ex, m > 1 ? tot : nullptr);
+    if (one_warp(n, c)) scan_down_kernel<true><<<1, 32, 0, stream>>>(v, n, c, nullptr, nullptr);
+    else scan_down_kernel<false><<<(u32)m, CTA, 0, stream>>>(v, n, c, ex, m > 1 ? tot : nullptr);
     return cudaGetLastError();
 }
 
@@ -631,7 +679,7 @@ extern "C" cudaError_t scan_mul(void *temp_buffer, unsigned long *buffer_size, P
 extern "C" cudaError_t kate_division(void *temp_buf, unsigned long *temp_buf_size, unsigned int log_p, ConstPolyPtr p,
                                      const unsigned int *b, PolyPtr q, cudaStream_t stream) {
     const u64 n = 1ull << log_p;
-    const u32 c = chunk_for(n);
+    const u32 c = walk_chunk_for(n);
     const u64 m = ctas_for(n, c);
     const size_t keep = c >= MAX_C ? al(m * CTA * 32) : 0;
     const size_t need = m > 1 ? al(TAB * 32) + al(m * 32) + keep : 256;
@@ -654,7 +702,9 @@ extern "C" cudaError_t kate_division(void *temp_buf, unsigned long *temp_buf_siz
         kate_top_kernel<<<1, CTA, 0, stream>>>(tot, (u32)m, tab + (32 + WARPS) * 8, c1, log2_of(c1));
         ZK_TRY(cudaGetLastError());
     }
-    kate_down_kernel<<<(u32)m, CTA, 0, stream>>>(vp, vq, n, b, c, log2_of(c), carry, tot, tab);
+    if (one_warp(n, c))
+        kate_down_kernel<true><<<1, 32, 0, stream>>>(vp, vq, n, b, c, log2_of(c), nullptr, nullptr, nullptr);
+    else kate_down_kernel<false><<<(u32)m, CTA, 0, stream>>>(vp, vq, n, b, c, log2_of(c), carry, tot, tab);
     return cudaGetLastError();
 }
 #include "permute.cuh"
