@@ -261,3 +261,20 @@ def test_sweeps_of_few_chunks(zk, orc, n):
             acc = (acc * b + (p[i + 1] if i + 1 < n else 0)) % M
             expect.append(acc)
         assert ints(orc, q.numpy_u64()) == expect[::-1]
+
+
+def test_empty_polynomial_through_the_size_query(zk):
+    """Length 0 with buffers of exactly the queried sizes: the query asks for some bytes (a buffer of
+    none is a null pointer, which would be a query again), and the evaluation writes zero."""
+    import ctypes
+    lib = zk.poly._lib()
+    stream = torch.cuda.current_stream().cuda_stream
+    empty = zk.native.PolyPtr(None, 0, 0, 0, 0)
+    x = torch.ones(8, dtype=torch.int32, device="cuda")
+    res = torch.full((8,), 7, dtype=torch.int32, device="cuda")
+    for fn, args in ((lib.poly_eval, (res.data_ptr(), x.data_ptr())), (lib.batched_invert, ()), (lib.scan_mul, ())):
+        size = ctypes.c_ulong(0)
+        assert fn(None, ctypes.byref(size), empty, *args, stream) == 0
+        temp = torch.empty(size.value, dtype=torch.uint8, device="cuda")
+        assert size.value > 0 and fn(temp.data_ptr(), ctypes.byref(size), empty, *args, stream) == 0
+    assert not res.any()

@@ -58,7 +58,9 @@ inline u32 walk_chunk_for(u64 n) { return n <= 4 ? 4 : chunk_for(n); }
 // steps, by one thread, and here: product scan 7.3 / 8.4, 2.3 / 8.1 and 2.1 / 4.2 us, division 13.5 / 14.6,
 // 2.0 / 7.0 and 2.2 / 5.2, inversion 45 / 48, 35 / 49 and 21 / 26).
 inline bool one_warp(u64 n, u32 c) { return n <= 32ull * c; }
-inline u64 ctas_for(u64 n, u32 c) { return (n + (u64)CTA * c - 1) / ((u64)CTA * c); }
+// an empty polynomial counts as one CTA, so that no size query answers 0 (a caller's buffer of 0 bytes
+// is a null pointer, which asks for the size again)
+inline u64 ctas_for(u64 n, u32 c) { return n ? (n + (u64)CTA * c - 1) / ((u64)CTA * c) : 1; }
 
 inline u32 grid_for(u64 items, u32 block, u32 per_sm = 16) {
     const u64 b = (items + block - 1) / block;
@@ -652,7 +654,7 @@ extern "C" cudaError_t scan_mul(void *temp_buffer, unsigned long *buffer_size, P
     const u32 c = walk_chunk_for(n);
     const u64 m = ctas_for(n, c);
     const size_t keep = c >= MAX_C ? al(m * CTA * 32) : 0;
-    const size_t need = al((m ? m : 1) * 32) + keep;
+    const size_t need = al(m * 32) + keep;
     if (temp_buffer == nullptr) {
         ZK_CHECK_ARG(buffer_size != nullptr);
         *buffer_size = need;
