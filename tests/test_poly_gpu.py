@@ -278,3 +278,68 @@ def test_empty_polynomial_through_the_size_query(zk):
         temp = torch.empty(size.value, dtype=torch.uint8, device="cuda")
         assert size.value > 0 and fn(temp.data_ptr(), ctypes.byref(size), empty, *args, stream) == 0
     assert not res.any()
+
+
+def permute_expected(vals, table):
+    """canonical integers: the input sorted; the table's arrangement (see oracle.permute)"""
+    a, left = sorted(vals), {}
+    for v in table:
+        left[v] = left.get(v, 0) + 1
+    out = list(a)
+    repeated = []
+    for i, v in enumerate(a):
+        if i == 0 or v != a[i - 1]:
+            left[v] -= 1
+        else:
+            repeated.append(i)
+    for i, v in zip(repeated, sorted(v for v, c in left.items() for _ in range(c))):
+        out[i] = v
+    return a, out
+
+
+def mont_words(vals):
+    return np.frombuffer(b"".join((v * R % M).to_bytes(32, "little") for v in vals), dtype=np.uint64).reshape(-1, 4)
+
+
+def permute_table(kind, n, rng):
+    if kind == "random":
+        return [int.from_bytes(rng.bytes(32), "little") % M for _ in range(n)]
+    if kind == "signed":  # a range around zero
+        return [(int(v) - n // 2) % M for v in rng.permutation(n)]
+    if kind == "wide":  # 62-bit magnitudes of either sign
+        return [int(v) * int(s) % M for v, s in zip(rng.integers(0, 1 << 62, n), rng.choice([-1, 1], n))]
+    if kind == "clash":  # three top words, a few middle ones, values below
+        tops = [int.from_bytes(rng.bytes(3), "little") << 220 for _ in range(3)]
+        return [tops[int(t)] | (int(m) << 100) | int(v)
+                for t, m, v in zip(rng.integers(0, 3, n), rng.integers(0, 4, n), rng.integers(0, 1 << 20, n))]
+    vals = permute_table("random", n, rng)
+    if kind == "some":  # small values among random ones
+        vals[: n // 8] = range(n // 8)
+    if kind == "nested":  # long runs under one top word, under two, under three, ...
+        for w in range(7):
+            part = range(w * n // 16, (w + 1) * n // 16)
+            for i in part:
+                vals[i] = (0x1234567 << 228 | vals[i] >> (26 + 32 * w)) % M
+    if kind == "repeated":  # few values, many rows of each
+        vals = [vals[int(i)] for i in rng.integers(0, max(1, n // 40), n)]
+    return [vals[int(i)] for i in rng.permutation(n)]
+
+
+@pytest.mark.parametrize("kind", ["random", "signed", "wide", "clash", "some", "nested", "repeated"])
+@pytest.mark.parametrize("n", [40, 1024, 2048, 2049, 65536, 65537, 152000])
+def test_permute_sort_rounds(zk, n, kind):
+    """Every way the sort settles ties (none, insertion, one or more further words, all words), on one CTA
+    an array, several, and all of them, with the 24-bit and the 32-bit word."""
+    rng = np.random.default_rng(n)
+    table = permute_table(kind, n, rng)
+    vals = [table[int(i)] for i in rng.integers(0, n, n)]
+    ri, rt = zk.ScalarArray.alloc(n), zk.ScalarArray.alloc(n)
+    zk.poly.permute(dev(zk, mont_words(vals)), dev(zk, mont_words(table)), n, ri, rt)
+    ei, et = permute_expected(vals, table)
+    assert np.array_equal(ri.numpy_u64(), mont_words(ei))
+    assert np.array_equal(rt.numpy_u64(), mont_words(et))
+
+
+@pytest.mark.parametrize("kind", ["random", "signed", "some"])
+def test_permute_2_20_rows(zk, kind):
+    test_permute_sort_rounds(zk, 1 << 20, kind)

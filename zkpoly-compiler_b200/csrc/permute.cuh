@@ -13,13 +13,19 @@
 // table entries); and the outputs.  Its steps are separated by grid barriers, where launches of
 // their own (about 90 with library radix sorts) cost 0.58 ms at 4095 rows.
 //
-// The sort is a least-significant-digit radix sort of (word, row) pairs, 8 bits a pass.  Which word:
-// the 32 bits (24 up to SHORT_WORD rows) below the highest bit in which any two keys differ.  For random field
-// elements these leave a handful of ties, for small values (range tables) they hold the whole
-// value.  Ties between different keys are put right afterwards: a run of equal words of at most
-// TIE_RUN rows by insertion on the full keys; if a longer run mixes keys, the sort runs again
-// over all eight words, least significant first (digits that no two keys differ in are skipped in
-// every case).  So any values sort exactly, and the usual ones in three or four passes instead of 32.
+// The sort is a least-significant-digit radix sort of (word, row) pairs, 8 bits a pass.  Which word: bit
+// 253, called the sign, and the 31 bits (23 up to SHORT_WORD rows) below the highest bit in which any
+// two keys, those with the sign first XORed with r, differ.  For random field elements these leave a
+// handful of ties; for range tables they hold the whole value, also of negative values, which
+// are r - v and have r's high words.  Ties between different keys are put right afterwards: a run of
+// equal words of at most TIE_RUN rows by insertion on the full keys.  Where a longer run mixes keys (a
+// few dozen small values among random ones), the runs are numbered and the rows sorted again by the
+// 32 bits below the highest bit in which keys of a long run differ, then by run number, each only over
+// the digits that vary.  All words are sorted by, least significant first, where they have few varying
+// digits (FEW_DIGITS) or long runs are left after two such rounds.
+// 2^20 rows of random elements take 0.48 ms, a range table of either sign 0.45 (1.14 where all words had
+// to settle it, 0.92 with library sorts), 2^19 or 100 small values among random ones 0.85 / 0.76 (1.51 /
+// 1.55, 0.98 / 1.16).
 #pragma once
 #include <cooperative_groups.h>
 
@@ -30,6 +36,7 @@ struct __align__(16) Key {
     u32 w[8];  // canonical value, little-endian words
 };
 
+ZK_DI u32 key_sign(const Key &k) { return k.w[7] >> 29; }
 ZK_DI bool key_eq(const Key &a, const Key &b) {
     u32 d = 0;
 #pragma unroll
@@ -37,14 +44,18 @@ ZK_DI bool key_eq(const Key &a, const Key &b) {
     return d == 0;
 }
 ZK_DI bool key_lt(const Key &a, const Key &b) {
-#pragma unroll
-    for (int i = 7; i >= 0; i--)
-        if (a.w[i] != b.w[i]) return a.w[i] < b.w[i];
-    return false;
+    if (a.w[7] != b.w[7]) return a.w[7] < b.w[7];
+    u32 d[8];
+    return Fr::sub_raw(d, a.w, b.w) != 0;
 }
 
 constexpr u32 CTA = 1024, WARPS = CTA / 32;
 constexpr u32 TIE_RUN = 16, SHORT_WORD = 1u << 16;
+// A round costs its passes and the time of three to six more for the runs; all words at once need no other.
+constexpr u32 FEW_DIGITS = 12, ROUNDS = 3;
+// flags, zero at the start: bits in which keys (XORed with r by sign) differ, and whether signs do;
+// then per round the bits in which keys of a long run differ, by array, and whether a long run mixes keys
+constexpr u32 FLAGS_ALL = 9, FLAGS_ROUND = 17, FLAGS = FLAGS_ALL + ROUNDS * FLAGS_ROUND;
 
 struct Args {
     View in[2];  // the input and the table
@@ -54,10 +65,12 @@ struct Args {
     Key *keys[2], *sorted[2];
     u32 *word[2][2], *idx[2][2];  // sort pairs, ping-pong
     u32 *hist;                    // [array][CTA][256], with more than one CTA an array
-    u32 *diff;                    // 8 words: bits in which keys differ; word 8: mixed long run seen
+    u32 *flags;                   // FLAGS words
     u32 *first, *free_;           // run starts of the sorted input; table entries not taken
     u32 *counts;                  // [2][CTA]: run starts / free entries per CTA
     u32 *left;                    // rows of the sorted table that stay, in order
+    u32 *start[2];                // of the sort: rows that begin a run (`first` and `left`, written later)
+    u32 *run[2];                  // of the sort: run numbers by original row
 };
 
 // the 32 bits of k below (and with) bit hb
@@ -70,6 +83,12 @@ ZK_DI u32 key_word(const Key &k, u32 hb) {
         hi = i == (s >> 5) + 1 ? k.w[i] : hi;
     }
     return __funnelshift_r(lo, hi, s & 31);
+}
+// the sign and the 31 bits below (and with) bit hb, of a key in memory
+ZK_DI u32 sign_word(const Key &k, u32 hb, u32 sign) {
+    const u32 s = hb >= 30 ? hb - 30 : 0, q = s >> 5;
+    const u32 bits = __funnelshift_r(k.w[q], q < 7 ? k.w[q + 1] : 0u, s & 31);
+    return (sign << 31) | (bits & 0x7fffffffu);
 }
 
 ZK_DI u32 warp_incl(u32 x, u32 lane) {
@@ -92,6 +111,21 @@ ZK_DI u32 cta_excl(u32 v, u32 *sm, u32 &total) {
     total = sm[WARPS - 1];
     __syncthreads();
     return r;
+}
+
+// fn(i) for the thread's rows whose word is that of the row before, the loads of four rows in flight
+template <class F>
+ZK_DI void for_ties(u32 n, u32 gt, u32 gs, const u32 *word, const F &fn) {
+    for (u32 i0 = gt; i0 < n; i0 += 4 * gs) {
+        u32 ties = 0;
+#pragma unroll
+        for (u32 u = 0; u < 4; u++) {
+            const u32 i = i0 + u * gs;
+            const u32 w = i < n ? word[i] : 0, v = i < n && i > 0 ? word[i - 1] : ~w;
+            ties |= (w == v ? 1u : 0u) << u;
+        }
+        for (; ties; ties &= ties - 1) fn(i0 + (__ffs(ties) - 1) * gs);
+    }
 }
 
 // One stable radix pass over bits [shift, shift + 8) of an array's pairs.  Every warp owns a
@@ -168,111 +202,204 @@ __global__ void __launch_bounds__(CTA, 1) permute_kernel(const Args a) {
     const u32 s = blockIdx.x >= a.half ? 1 : 0, cta = blockIdx.x - s * a.half;
     const u32 n = a.n;
     const u32 gt = cta * CTA + tid, gs = a.half * CTA;  // thread and stride within the array
-    // ---- canonical keys and the bits they differ in
+    // ---- keys and the bits they differ in
     {
-        const Key k0 = [&] {
-            const Fr x = Fr::load(a.in[s].at(0)).to_number();
-            Key k;
+        auto signed_word = [](const Fr &x, int w) { return x.v[w] ^ (FrParams::m(w) & (0u - (x.v[7] >> 29))); };
+        Fr first = Fr::load(a.in[s].at(0)).to_number();
+        const u32 sign0 = first.v[7] >> 29;
+        u32 k0[8], diff[9];
 #pragma unroll
-            for (int w = 0; w < 8; w++) k.w[w] = x.v[w];
-            return k;
-        }();
-        u32 diff[8];
+        for (int w = 0; w < 8; w++) k0[w] = signed_word(first, w);
 #pragma unroll
-        for (int w = 0; w < 8; w++) diff[w] = 0;
+        for (int w = 0; w < 9; w++) diff[w] = 0;
         for (u32 i = gt; i < n; i += gs) {
             const Fr x = Fr::load(a.in[s].at(i)).to_number();
             Key k;
 #pragma unroll
             for (int w = 0; w < 8; w++) {
                 k.w[w] = x.v[w];
-                diff[w] |= x.v[w] ^ k0.w[w];
+                diff[w] |= signed_word(x, w) ^ k0[w];
             }
+            diff[8] |= (x.v[7] >> 29) ^ sign0;
             a.keys[s][i] = k;
         }
 #pragma unroll
-        for (int w = 0; w < 8; w++) {
+        for (int w = 0; w < 9; w++) {
             const u32 d = __reduce_or_sync(0xffffffffu, diff[w]);
-            if (lane == 0 && d) atomicOr(a.diff + w, d);
+            if (lane == 0 && d) atomicOr(a.flags + w, d);
         }
     }
     grid.sync();
-    u32 diff[8], hb = 0;
+    auto read_diff = [&](const u32 *f, Key &d) {  // returns the highest bit
+        u32 hb = 0;
 #pragma unroll
-    for (u32 w = 0; w < 8; w++) {
-        diff[w] = __ldcg(a.diff + w);
-        if (diff[w]) hb = 32 * w + 31 - __clz(diff[w]);
-    }
-    // ---- sort by one word, or by all of them
-    const u32 drop = n <= SHORT_WORD && hb >= 31 ? 8 : 0;  // up to 2^16 rows 24 bits leave few ties
+        for (u32 w = 0; w < 8; w++) {
+            d.w[w] = __ldcg(f + w);
+            if (d.w[w]) hb = 32 * w + 31 - __clz(d.w[w]);
+        }
+        return hb;
+    };
+    auto barrier = [&] {  // for what an array's own CTAs exchange
+        if (a.half > 1) grid.sync();
+        else __syncthreads();
+    };
     u32 cur = 0;
-    bool full = false;
-    for (;;) {
-        for (u32 word = 0; word < (full ? 8u : 1u); word++) {
-            u32 vary = 0;
-            if (full) {
+    auto sort_digits = [&](u32 vary) {
+        barrier();
+        for (u32 shift = 0; shift < 32; shift += 8) {
+            if (!((vary >> shift) & 255u)) continue;
+            radix_pass(a, s, cta, shift, cur, whist, sm, grid);
+            cur ^= 1;
+        }
+    };
+    // ---- sort by the top word
+    u32 hb;  // the highest bit of the array's current word
+    {
+        Key all;
+        hb = read_diff(a.flags, all);
+        const u32 signs = __ldcg(a.flags + 8);
+        const u32 drop = n <= SHORT_WORD && hb >= 30 ? 8 : 0;  // up to 2^16 rows 24 bits leave few ties
+        for (u32 i = gt; i < n; i += gs) {
+            const Key &x = a.keys[s][i];
+            a.word[s][0][i] = sign_word(x, hb, key_sign(x)) >> drop;
+            a.idx[s][0][i] = i;
+        }
+        sort_digits(sign_word(all, hb, signs) >> drop);
+    }
+    // ---- put ties right
+    Key *const k = a.sorted[s];
+    for (u32 round = 0;; round++) {
+        u32 *word = a.word[s][cur], *idx = a.idx[s][cur];
+        for (u32 i = gt; i < n; i += gs) k[i] = a.keys[s][idx[i]];
+        // rows i start free; the barriers up to the take step below order this
+        if (round == 0)
+            for (u32 i = blockIdx.x * CTA + tid; i < n; i += gridDim.x * CTA) a.free_[i] = 1u;
+        grid.sync();
+        // ties: rows the sort so far has not told apart (after the first round: of one run, with equal words)
+        auto tied = [&](u32 i) {
+            return i > 0 && word[i] == word[i - 1] && (round == 0 || key_word(k[i], hb) == key_word(k[i - 1], hb));
+        };
+        u32 *flags = a.flags + FLAGS_ALL + round * FLAGS_ROUND;
+        bool mixed = false;  // one witness a thread is enough
+        for_ties(n, gt, gs, word, [&](u32 i) {
+            if (mixed || !tied(i) || key_eq(k[i], k[i - 1])) return;
+            u32 lo = i - 1, hi = i + 1;
+            while (hi - lo <= TIE_RUN && tied(lo)) lo--;
+            while (hi - lo <= TIE_RUN && hi < n && tied(hi)) hi++;
+            mixed = hi - lo > TIE_RUN;
+        });
+        if (mixed) atomicOr(flags + 16, 1u);
+        grid.sync();
+        const bool again = __ldcg(flags + 16) != 0;
+        u32 *const start = a.start[s];
+        for_ties(n, gt, gs, word, [&](u32 second) {  // the second row of a short run sorts it
+            const u32 i = second - 1;
+            if (!tied(second) || tied(i)) return;
+            u32 end = i + 2;
+            while (end < n && end - i <= TIE_RUN && tied(end)) end++;
+            if (end - i > TIE_RUN) return;
+            for (u32 j = i + 1; j < end; j++) {
+                const Key x = k[j];
+                const u32 r = idx[j];
+                u32 p = j;
+                for (; p > i && key_lt(x, k[p - 1]); p--) {
+                    k[p] = k[p - 1];
+                    idx[p] = idx[p - 1];
+                }
+                if (p != j) {
+                    k[p] = x;
+                    idx[p] = r;
+                }
+            }
+        });
+        if (again)
+            for (u32 i = gt; i < n; i += gs) start[i] = tied(i) ? 0u : 1u;
+        grid.sync();
+        if (__builtin_expect(!again, 1)) break;
+        Key all;
+        read_diff(a.flags, all);
+        const u32 signs = __ldcg(a.flags + 8);
+        u32 digits = signs;
 #pragma unroll
-                for (u32 w = 0; w < 8; w++) vary = w == word ? diff[w] : vary;
+        for (int w = 0; w < 8; w++)
+#pragma unroll
+            for (int b = 0; b < 32; b += 8) digits += (all.w[w] >> b) & 255u ? 1 : 0;
+        if (digits <= FEW_DIGITS || round + 1 == ROUNDS) {
+            for (u32 w = 0; w < 9; w++) {  // the sign last
+                u32 vary = w == 8 ? signs : 0;
+#pragma unroll
+                for (u32 v = 0; v < 8; v++) vary = v == w ? all.w[v] : vary;
                 if (!vary) continue;
                 for (u32 i = gt; i < n; i += gs) {
-                    const u32 r = word == 0 ? i : a.idx[s][cur][i];
-                    a.idx[s][cur][i] = r;
-                    a.word[s][cur][i] = a.keys[s][r].w[word];
+                    const Key &x = a.keys[s][a.idx[s][cur][i]];
+                    a.word[s][cur][i] = w == 8 ? key_sign(x) : x.w[w];
                 }
-            } else {
-                Key d;
-#pragma unroll
-                for (int w = 0; w < 8; w++) d.w[w] = diff[w];
-                vary = key_word(d, hb) >> drop;
-                for (u32 i = gt; i < n; i += gs) {
-                    a.idx[s][cur][i] = i;
-                    a.word[s][cur][i] = key_word(a.keys[s][i], hb) >> drop;
-                }
+                sort_digits(vary);
             }
-            if (a.half > 1) grid.sync();
-            else __syncthreads();
-            for (u32 shift = 0; shift < 32; shift += 8) {
-                if (!((vary >> shift) & 255u)) continue;
-                radix_pass(a, s, cta, shift, cur, whist, sm, grid);
-                cur ^= 1;
-            }
-        }
-        for (u32 i = gt; i < n; i += gs) a.sorted[s][i] = a.keys[s][a.idx[s][cur][i]];
-        // rows i start free; the barriers up to the take step below order this
-        for (u32 i = blockIdx.x * CTA + tid; i < n; i += gridDim.x * CTA) a.free_[i] = 1u;
-        grid.sync();
-        if (full) break;
-        // rows whose key differs from the one before it under an equal word
-        const u32 *word = a.word[s][cur];
-        bool mixed_long = false;
-        for (u32 i = gt; i < n; i += gs) {
-            if (i == 0 || word[i] != word[i - 1] || key_eq(a.sorted[s][i], a.sorted[s][i - 1])) continue;
-            u32 lo = i, hi = i + 1;
-            while (lo > 0 && word[lo - 1] == word[i] && hi - lo <= TIE_RUN) lo--;
-            while (hi < n && word[hi] == word[i] && hi - lo <= TIE_RUN) hi++;
-            mixed_long = mixed_long || hi - lo > TIE_RUN;
-        }
-        if (mixed_long) atomicOr(a.diff + 8, 1u);
-        grid.sync();
-        if (!__ldcg(a.diff + 8)) {
-            for (u32 i = gt; i < n; i += gs) {  // the head of a short run sorts it
-                if ((i > 0 && word[i] == word[i - 1]) || i + 1 >= n || word[i + 1] != word[i]) continue;
-                u32 end = i + 2;
-                while (end < n && word[end] == word[i] && end - i <= TIE_RUN) end++;
-                if (end - i > TIE_RUN) continue;  // a long run of one key
-                Key *k = a.sorted[s];
-                for (u32 j = i + 1; j < end; j++) {
-                    const Key x = k[j];
-                    u32 p = j;
-                    for (; p > i && key_lt(x, k[p - 1]); p--) k[p] = k[p - 1];
-                    if (p != j) k[p] = x;
-                }
-            }
+            for (u32 i = gt; i < n; i += gs) k[i] = a.keys[s][a.idx[s][cur][i]];
             grid.sync();
             break;
         }
-        full = true;
-        cur = 0;
+        // number the runs; the rows of a short one, in order now, are runs of their own
+        for (u32 i = gt; i < n; i += gs) {
+            if (!start[i] || i + 1 >= n || start[i + 1]) continue;
+            u32 end = i + 2;
+            while (end < n && end - i <= TIE_RUN && !start[end]) end++;
+            if (end - i > TIE_RUN) continue;
+            for (u32 j = i + 1; j < end; j++) start[j] = 1u;
+        }
+        barrier();
+        const u32 share = (n + a.half - 1) / a.half;  // rows of the array's CTAs, in order
+        const u64 f64 = (u64)cta * share;
+        const u32 first = f64 < n ? (u32)f64 : n, last = n - first < share ? n : first + share;
+        u32 starts = 0, bits[8];
+#pragma unroll
+        for (int w = 0; w < 8; w++) bits[w] = 0;
+        for (u32 i = first + tid; i < last; i += CTA) {
+            if (start[i]) {
+                starts++;
+                continue;
+            }
+#pragma unroll
+            for (int w = 0; w < 8; w++) bits[w] |= k[i].w[w] ^ k[i - 1].w[w];
+        }
+#pragma unroll
+        for (int w = 0; w < 8; w++) {
+            const u32 d = __reduce_or_sync(0xffffffffu, bits[w]);
+            if (lane == 0 && d) atomicOr(flags + 8 * s + w, d);
+        }
+        u32 total;
+        cta_excl(starts, sm, total);
+        if (tid == 0) a.counts[blockIdx.x] = total;
+        grid.sync();
+        u32 before = 0, runs0 = 0, runs1 = 0;
+        for (u32 b = tid; b < 2 * a.half; b += CTA) {
+            const u32 c = __ldcg(a.counts + b);
+            runs0 += b < a.half ? c : 0;
+            runs1 += b < a.half ? 0 : c;
+            before += b >= s * a.half && b < blockIdx.x ? c : 0;
+        }
+        cta_excl(before, sm, before);
+        cta_excl(runs0, sm, runs0);
+        cta_excl(runs1, sm, runs1);
+        for (u32 i0 = first; i0 < last; i0 += CTA) {
+            const u32 i = i0 + tid, f = i < last ? start[i] : 0;
+            const u32 p = cta_excl(f, sm, total);
+            if (i < last) a.run[s][idx[i]] = before + p + f - 1;
+            before += total;
+        }
+        // by the next word, then by run
+        Key mix;
+        const u32 top0 = read_diff(flags, mix);
+        u32 vary = key_word(mix, top0);
+        const u32 top1 = read_diff(flags + 8, mix);
+        vary |= key_word(mix, top1);
+        hb = s ? top1 : top0;
+        for (u32 i = gt; i < n; i += gs) word[i] = key_word(a.keys[s][idx[i]], hb);
+        sort_digits(vary);
+        for (u32 i = gt; i < n; i += gs) a.word[s][cur][i] = a.run[s][a.idx[s][cur][i]];
+        const u32 most = max(runs0, runs1) - 1;
+        sort_digits(most ? 0xffffffffu >> __clz(most) : 0u);
     }
     // ---- run starts of the input take a table entry each (any of equal entries)
     const Key *A = a.sorted[0], *T = a.sorted[1];
@@ -359,7 +486,7 @@ inline u32 ctas_per_array(u64 n) {
 }
 
 struct Layout {
-    size_t keys[2], sorted[2], word[2][2], idx[2][2], hist, diff, first, free_, counts, left, total;
+    size_t keys[2], sorted[2], word[2][2], idx[2][2], run[2], hist, flags, first, free_, counts, left, total;
 };
 
 inline Layout layout(u64 n) {
@@ -383,8 +510,9 @@ inline Layout layout(u64 n) {
     l.left = take(n * 4);
     const u64 ctas = 2 * ctas_per_array(n);
     l.hist = ctas > 2 ? take(ctas * 256 * 4) : 0;
-    l.diff = take((9 + ctas * 2) * 4);
-    l.counts = l.diff + 9 * 4;
+    l.flags = take((FLAGS + ctas * 2) * 4);
+    l.counts = l.flags + FLAGS * 4;
+    for (int s = 0; s < 2; s++) l.run[s] = take(n * 4);
     l.total = off;
     return l;
 }
@@ -419,14 +547,17 @@ extern "C" cudaError_t permute(void *temp_buffer, unsigned long *buffer_size, un
             a.word[s][i] = words(l.word[s][i]);
             a.idx[s][i] = words(l.idx[s][i]);
         }
+        a.run[s] = words(l.run[s]);
     }
     a.hist = words(l.hist);
-    a.diff = words(l.diff);
+    a.flags = words(l.flags);
     a.first = words(l.first);
     a.free_ = words(l.free_);
     a.counts = words(l.counts);
     a.left = words(l.left);
-    ZK_TRY(cudaMemsetAsync(a.diff, 0, 9 * 4, stream));
+    a.start[0] = a.first;
+    a.start[1] = a.left;
+    ZK_TRY(cudaMemsetAsync(a.flags, 0, perm::FLAGS * 4, stream));
     void *args[] = {&a};
     return cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(perm::permute_kernel), dim3(2 * a.half),
                                        dim3(perm::CTA), args, 0, stream);
