@@ -55,6 +55,12 @@ cudaError_t scalar_pow(unsigned int *target, unsigned long long exp, cudaStream_
 cudaError_t permute(void *temp_buffer, unsigned long *buffer_size, unsigned long usable, ConstPolyPtr input,
                     ConstPolyPtr table, PolyPtr res_input, PolyPtr res_table, cudaStream_t stream);
 
+/* permute is one cooperative launch: it starts once all its CTAs (at most one an SM) fit on the SMs that
+ * the stream's context, or its green context, has, and waits behind longer kernels of other streams
+ * until they do.  *ctas = the CTAs of 1024 threads it launches for `usable` rows on `stream`
+ * (addition, no counterpart in the reference). */
+cudaError_t zkp_permute_ctas(unsigned long usable, cudaStream_t stream, unsigned int *ctas);
+
 #ifdef __cplusplus
 }
 #endif

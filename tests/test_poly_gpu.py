@@ -343,3 +343,72 @@ def test_permute_sort_rounds(zk, n, kind):
 @pytest.mark.parametrize("kind", ["random", "signed", "some"])
 def test_permute_2_20_rows(zk, kind):
     test_permute_sort_rounds(zk, 1 << 20, kind)
+
+
+def permute_case(zk, n, kind="some"):
+    rng = np.random.default_rng(n)
+    table = permute_table(kind, n, rng)
+    vals = [table[int(i)] for i in rng.integers(0, n, n)]
+    ei, et = permute_expected(vals, table)
+    return (dev(zk, mont_words(vals)), dev(zk, mont_words(table)), zk.ScalarArray.alloc(n), zk.ScalarArray.alloc(n),
+            mont_words(ei), mont_words(et))
+
+
+def test_permute_captured_and_beside_other_work(zk):
+    """The cooperative launch in a stream capture, replayed on other values, and while another stream
+    keeps the GPU busy with transforms."""
+    n = 30000
+    inp, table, ri, rt, ei, et = permute_case(zk, n)
+    other = permute_case(zk, n, "signed")
+    stream, busy = torch.cuda.Stream(), torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        zk.poly.permute(inp, table, n, ri, rt)
+    graph.replay()
+    assert np.array_equal(ri.numpy_u64(), ei) and np.array_equal(rt.numpy_u64(), et)
+    inp.values.copy_(other[0].values)
+    table.values.copy_(other[1].values)
+    graph.replay()
+    assert np.array_equal(ri.numpy_u64(), other[4]) and np.array_equal(rt.numpy_u64(), other[5])
+    x = zk.ScalarArray(zk.gen.fr(3, 1 << 20))
+    zk.ntt.ntt(x)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(busy):
+        for _ in range(20):
+            zk.ntt.ntt(x)
+    with torch.cuda.stream(stream):
+        zk.poly.permute(other[0], other[1], n, other[2], other[3])
+    torch.cuda.synchronize()
+    assert np.array_equal(other[2].numpy_u64(), other[4]) and np.array_equal(other[3].numpy_u64(), other[5])
+
+
+def test_permute_on_a_partition(zk):
+    """A stream of a green context with a few SMs: the grid is cut to what is resident there at once."""
+    driver = pytest.importorskip("cuda.bindings.driver")
+    import ctypes
+
+    def ok(r):
+        if int(r[0]) != 0:
+            pytest.skip(f"green contexts: {r[0]}")
+        return r[1] if len(r) == 2 else r[1:]
+    torch.zeros(1, device="cuda")
+    device = ok(driver.cuDeviceGet(0))
+    sms = ok(driver.cuDeviceGetDevResource(device, driver.CUdevResourceType.CU_DEV_RESOURCE_TYPE_SM))
+    groups = ok(driver.cuDevSmResourceSplitByCount(1, sms, 0, 8))[0]
+    desc = ok(driver.cuDevResourceGenerateDesc([groups[0]], 1))
+    green = ok(driver.cuGreenCtxCreate(desc, device, driver.CUgreenCtxCreate_flags.CU_GREEN_CTX_DEFAULT_STREAM))
+    stream = ok(driver.cuGreenCtxStreamCreate(green, driver.CUstream_flags.CU_STREAM_NON_BLOCKING, 0))
+    try:
+        n = 65536
+        ctas = ctypes.c_uint(0)
+        assert zk.poly._lib().zkp_permute_ctas(n, None, ctypes.byref(ctas)) == 0 and ctas.value == 64
+        assert zk.poly._lib().zkp_permute_ctas(n, int(stream), ctypes.byref(ctas)) == 0
+        assert 2 <= ctas.value <= groups[0].sm.smCount < 64  # no launch unless all its CTAs fit
+        inp, table, ri, rt, ei, et = permute_case(zk, n)
+        torch.cuda.synchronize()
+        zk.poly.permute(inp, table, n, ri, rt, stream=torch.cuda.ExternalStream(int(stream)))
+        ok(driver.cuStreamSynchronize(stream) + (None,))
+        assert np.array_equal(ri.numpy_u64(), ei) and np.array_equal(rt.numpy_u64(), et)
+    finally:
+        driver.cuStreamDestroy(stream)
+        driver.cuGreenCtxDestroy(green)

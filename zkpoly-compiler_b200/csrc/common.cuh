@@ -4,6 +4,7 @@
 #include <atomic>
 #include <cstdint>
 #include <cstdio>
+#include <mutex>
 
 #include "../../include/poly_ptr.h"
 #include "field.cuh"

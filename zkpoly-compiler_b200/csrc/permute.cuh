@@ -28,6 +28,7 @@
 // 1.55, 0.98 / 1.16).
 #pragma once
 #include <cooperative_groups.h>
+#include <cudaTypedefs.h>
 
 namespace zk {
 namespace perm {
@@ -485,6 +486,52 @@ inline u32 ctas_per_array(u64 n) {
     return (u32)(want < 1 ? 1 : (want < most ? want : most));
 }
 
+// SMs that kernels on the stream can use: those of its green context (a partition of the device) or of
+// its context (fewer than the device's under an execution-resource limit)
+inline cudaError_t stream_sms(cudaStream_t stream, u32 *sms) {
+    int dev = 0, all = 0;
+    ZK_TRY(cudaGetDevice(&dev));
+    ZK_TRY(cudaDeviceGetAttribute(&all, cudaDevAttrMultiProcessorCount, dev));
+    *sms = (u32)all;
+    static PFN_cuStreamGetCtx_v12050 get_ctx = nullptr;
+    static PFN_cuCtxGetDevResource_v12040 ctx_resource = nullptr;
+    static PFN_cuGreenCtxGetDevResource_v12040 green_resource = nullptr;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        auto find = [](const char *name, unsigned version) {
+            void *f = nullptr;
+            cudaDriverEntryPointQueryResult q;
+            const cudaError_t e = cudaGetDriverEntryPointByVersion(name, &f, version, cudaEnableDefault, &q);
+            return e == cudaSuccess && q == cudaDriverEntryPointSuccess ? f : nullptr;
+        };
+        ctx_resource = reinterpret_cast<PFN_cuCtxGetDevResource_v12040>(find("cuCtxGetDevResource", 12040));
+        green_resource = reinterpret_cast<PFN_cuGreenCtxGetDevResource_v12040>(find("cuGreenCtxGetDevResource", 12040));
+        if (ctx_resource && green_resource)
+            get_ctx = reinterpret_cast<PFN_cuStreamGetCtx_v12050>(find("cuStreamGetCtx", 12050));
+    });
+    CUcontext ctx = nullptr;
+    CUgreenCtx green = nullptr;
+    CUdevResource r{};
+    if (get_ctx && get_ctx(stream, &ctx, &green) == CUDA_SUCCESS &&
+        (green ? green_resource(green, &r, CU_DEV_RESOURCE_TYPE_SM)
+               : ctx_resource(ctx, &r, CU_DEV_RESOURCE_TYPE_SM)) == CUDA_SUCCESS &&
+        r.sm.smCount > 0 && r.sm.smCount < *sms)
+        *sms = r.sm.smCount;
+    return cudaSuccess;
+}
+
+// CTAs per array of a launch: the grid barriers need all CTAs on the stream's SMs at once
+inline cudaError_t launch_ctas_per_array(u64 n, cudaStream_t stream, u32 *half) {
+    u32 sms = 0;
+    int per_sm = 0;
+    ZK_TRY(stream_sms(stream, &sms));
+    ZK_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, permute_kernel, (int)CTA, 0));
+    const u32 fit = sms * (u32)per_sm / 2, want = ctas_per_array(n);
+    if (fit == 0) return cudaErrorCooperativeLaunchTooLarge;
+    *half = want < fit ? want : fit;
+    return cudaSuccess;
+}
+
 struct Layout {
     size_t keys[2], sorted[2], word[2][2], idx[2][2], run[2], hist, flags, first, free_, counts, left, total;
 };
@@ -539,7 +586,7 @@ extern "C" cudaError_t permute(void *temp_buffer, unsigned long *buffer_size, un
     char *base = reinterpret_cast<char *>(temp_buffer);
     auto words = [&](size_t off) { return reinterpret_cast<u32 *>(base + off); };
     a.n = (u32)usable;
-    a.half = perm::ctas_per_array(usable);
+    ZK_TRY(perm::launch_ctas_per_array(usable, stream, &a.half));
     for (int s = 0; s < 2; s++) {
         a.keys[s] = reinterpret_cast<perm::Key *>(base + l.keys[s]);
         a.sorted[s] = reinterpret_cast<perm::Key *>(base + l.sorted[s]);
@@ -561,4 +608,12 @@ extern "C" cudaError_t permute(void *temp_buffer, unsigned long *buffer_size, un
     void *args[] = {&a};
     return cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(perm::permute_kernel), dim3(2 * a.half),
                                        dim3(perm::CTA), args, 0, stream);
+}
+
+extern "C" cudaError_t zkp_permute_ctas(unsigned long usable, cudaStream_t stream, unsigned int *ctas) {
+    using namespace zk;
+    ZK_CHECK_ARG(ctas != nullptr && usable < (1ull << 31));
+    ZK_TRY(perm::launch_ctas_per_array(usable, stream, ctas));
+    *ctas *= 2;
+    return cudaSuccess;
 }

@@ -131,6 +131,7 @@ SIGNATURES = {
         "batched_invert": (cudaError_t, [c_void_p, ctypes.POINTER(ctypes.c_ulong), PolyPtr, c_void_p]),
         "permute": (cudaError_t, [c_void_p, ctypes.POINTER(ctypes.c_ulong), ctypes.c_ulong, PolyPtr, PolyPtr, PolyPtr,
                                   PolyPtr, c_void_p]),
+        "zkp_permute_ctas": (cudaError_t, [ctypes.c_ulong, c_void_p, ctypes.POINTER(ctypes.c_uint)]),
         "inv_scalar": (cudaError_t, [c_void_p, c_void_p]),
         "scalar_pow": (cudaError_t, [c_void_p, ctypes.c_ulonglong, c_void_p]),
     },
