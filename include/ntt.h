@@ -130,6 +130,16 @@ cudaError_t zkp_ntt_batch_set_solo_log(unsigned int log_len);
 cudaError_t zkp_ntt_batch_run(const ZkpNttBatchPlan *plan, cudaStream_t stream);
 void zkp_ntt_batch_plan_destroy(ZkpNttBatchPlan *plan);
 
+/* The tensor-core passes wait for their products inside the kernel, for about a second at most.  A pass
+ * whose wait runs out leaves its vector undefined; like other errors of a kernel that shows once the
+ * work has run: transforms of the context refuse with cudaErrorTimeout until zkp_ntt_status, called
+ * after a synchronisation, has returned it (and cleared it).  cudaSuccess: no wait ran out. */
+cudaError_t zkp_ntt_status(void);
+/* Test support: the first tensor-core pass of a transform of x whose waits give up after `polls` polls (0:
+ * at once); vector, table and length as the tensor-core passes need them. */
+cudaError_t zkp_ntt_wait_probe(PolyPtr x, const unsigned int *twiddle, unsigned int log_len, unsigned int polls,
+                               cudaStream_t stream);
+
 /* Benchmark support: throughput probe of the Shoup twiddle product (blocks x 256 threads x
  * iters x 2 products; out_d holds blocks * 256 * 8 words). */
 cudaError_t zkp_ntt_shoup_probe(unsigned int blocks, unsigned int iters, unsigned int *out_d, cudaStream_t stream);

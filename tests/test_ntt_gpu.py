@@ -455,3 +455,38 @@ def test_ntt_radix16_rotated_view(zk, orc):
     expect = orc.best_fft(orc.poly_ptr_view(a, n, rotate=12345), orc.root_of_unity(log_n), log_n)
     zk.ntt.ntt(x)
     assert np.array_equal(x.numpy_u64(), expect)
+
+
+def test_wait_that_runs_out_is_reported(zk, orc):
+    """A tensor-core pass whose waits give up at once returns, its error shows after the synchronisation
+    and in every later transform until it is taken, and the context then works as before; a pass that
+    waits as usual reports nothing."""
+    import torch
+    log_n = 21
+    lib = zk.native.load(zk.ntt.LIB)
+    a = orc.gen_fr(350, 1 << log_n)
+    x, tw = to_dev(zk, a), zk.ntt.twiddle_table(log_n)
+    stream = torch.cuda.current_stream().cuda_stream
+    zk.ntt.status()
+    assert lib.zkp_ntt_wait_probe(x.poly_ptr(), tw.values.data_ptr(), log_n, 1 << 16, stream) == 0
+    torch.cuda.synchronize()
+    zk.ntt.status()
+    assert lib.zkp_ntt_wait_probe(x.poly_ptr(), tw.values.data_ptr(), log_n, 0, stream) == 0
+    torch.cuda.synchronize()
+    small = to_dev(zk, a[: 1 << 8])
+    batch = zk.ntt.NttBatch([(to_dev(zk, a[: 1 << 8]), "ntt")])
+    for refused in (lambda: zk.ntt.ntt(x), lambda: zk.ntt.ntt(small), batch.run, zk.ntt.status):
+        with pytest.raises(zk.native.CudaError) as e:
+            refused()
+        assert e.value.code == 909  # cudaErrorTimeout
+    zk.ntt.status()
+    x = to_dev(zk, a)
+    zk.ntt.ntt(x)
+    assert np.array_equal(x.numpy_u64(), orc.best_fft(a, orc.root_of_unity(log_n), log_n))
+    zk.ntt.status()
+
+
+def test_wait_probe_refuses_other_passes(zk):
+    lib = zk.native.load(zk.ntt.LIB)
+    x, tw = zk.ScalarArray.zeros(1 << 10), zk.ntt.twiddle_table(10)
+    assert lib.zkp_ntt_wait_probe(x.poly_ptr(), tw.values.data_ptr(), 10, 0, None) == 1

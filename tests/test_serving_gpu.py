@@ -97,6 +97,24 @@ def test_failures_stay_with_their_request(zk, bases):
         ref.close()
 
 
+def test_a_wait_that_ran_out_fails_the_requests_in_flight(zk, bases):
+    """The server takes a timeout reported by the transforms' kernels: what it has in flight or launches
+    next fails, and the requests after that do not."""
+    lib = zk.native.load(zk.ntt.LIB)
+    x = zk.ScalarArray(zk.gen.fr(1, 1 << 21))
+    srv = server(zk, bases, 1)
+    try:
+        assert srv.wait(srv.submit(11, 21)).status == 0
+        assert lib.zkp_ntt_wait_probe(x.poly_ptr(), zk.ntt.twiddle_table(21).values.data_ptr(), 21, 0,
+                                      torch.cuda.current_stream().cuda_stream) == 0
+        torch.cuda.synchronize()
+        assert srv.wait(srv.submit(11, 22)).status == -3
+        assert srv.wait(srv.submit(11, 23)).status == 0
+        zk.ntt.status()
+    finally:
+        srv.close()
+
+
 def test_admission_by_hbm_footprint(zk, bases):
     probe = server(zk, bases, 1)
     fp13, fp14 = probe.footprint(13), probe.footprint(14)

@@ -91,6 +91,39 @@ inline int num_sms() {
     return v;
 }
 
+// The id of the calling thread's current context (cuCtxGetId ids are never reused within a process).
+// Without a current context the runtime's own rule applies: the current device's primary context,
+// which cudaSetDevice initialises and makes current.
+inline cudaError_t current_context_id(unsigned long long *id) {
+    using CtxGetCurrentFn = int (*)(void **ctx);
+    using CtxGetIdFn = int (*)(void *ctx, unsigned long long *id);
+    static CtxGetCurrentFn get_current = nullptr;
+    static CtxGetIdFn get_id = nullptr;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        cudaDriverEntryPointQueryResult q;
+        void *f = nullptr;
+        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &f, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            get_current = reinterpret_cast<CtxGetCurrentFn>(f);
+        f = nullptr;
+        if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            get_id = reinterpret_cast<CtxGetIdFn>(f);
+    });
+    if (!get_current || !get_id) return cudaErrorNotSupported;
+    void *ctx = nullptr;
+    if (get_current(&ctx) != 0) return cudaErrorDeviceUninitialized;
+    if (!ctx) {
+        int dev = 0;
+        ZK_TRY(cudaGetDevice(&dev));
+        ZK_TRY(cudaSetDevice(dev));
+        if (get_current(&ctx) != 0 || !ctx) return cudaErrorDeviceUninitialized;
+    }
+    if (get_id(ctx, id) != 0) return cudaErrorDeviceUninitialized;
+    return cudaSuccess;
+}
+
 }  // namespace zk
 
 namespace zk {

@@ -1855,9 +1855,6 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratch
 // makes its own driver-API context current, or a cudaDeviceReset, brings a new context with its
 // own copy of the array.  So the address is looked up with the calling context current and
 // cached under that context's unique id (cuCtxGetId ids are never reused within a process).
-using CtxGetCurrentFn = int (*)(void **ctx);
-using CtxGetIdFn = int (*)(void *ctx, unsigned long long *id);
-
 struct NoAllocEntry {
     unsigned long long ctx_id;
     void *ptr;
@@ -1865,36 +1862,6 @@ struct NoAllocEntry {
 static std::mutex g_noalloc_mu;
 static NoAllocEntry g_noalloc_cache[64];
 static unsigned g_noalloc_used = 0, g_noalloc_next = 0;
-
-static cudaError_t current_context_id(unsigned long long *id) {
-    static CtxGetCurrentFn get_current = nullptr;
-    static CtxGetIdFn get_id = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        cudaDriverEntryPointQueryResult q;
-        void *f = nullptr;
-        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &f, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            get_current = reinterpret_cast<CtxGetCurrentFn>(f);
-        f = nullptr;
-        if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            get_id = reinterpret_cast<CtxGetIdFn>(f);
-    });
-    if (!get_current || !get_id) return cudaErrorNotSupported;
-    void *ctx = nullptr;
-    if (get_current(&ctx) != 0) return cudaErrorDeviceUninitialized;
-    if (!ctx) {
-        // no context current yet on this thread: the runtime's own rule applies, the current
-        // device's primary context (cudaSetDevice initialises it and makes it current)
-        int dev = 0;
-        ZK_TRY(cudaGetDevice(&dev));
-        ZK_TRY(cudaSetDevice(dev));
-        if (get_current(&ctx) != 0 || !ctx) return cudaErrorDeviceUninitialized;
-    }
-    if (get_id(ctx, id) != 0) return cudaErrorDeviceUninitialized;
-    return cudaSuccess;
-}
 
 static cudaError_t noalloc_scratch(cudaStream_t stream, void **out) {
     unsigned long long id = 0;

@@ -836,15 +836,65 @@ cudaError_t prepare_last_bitrevs() {
     return prepare_last_bitrev<5, SH, BR_T>();
 }
 
+// The status words: one of mapped host memory per CUDA context (by its id, as ids are never reused; the
+// memory ends with its context), which a pass whose wait ran out sets.
+struct StatusWord {
+    unsigned long long ctx;
+    u32 *word;
+};
+std::mutex g_status_mu;
+StatusWord g_status[64];
+std::atomic<u32> g_status_used{0};
+u32 g_status_next = 0;
+
+// the current context's word, or null: none yet, and `create` not asked for
+cudaError_t status_word(bool create, u32 **out) {
+    *out = nullptr;
+    if (!create && g_status_used.load(std::memory_order_acquire) == 0) return cudaSuccess;
+    unsigned long long id = 0;
+    ZK_TRY(current_context_id(&id));
+    std::lock_guard<std::mutex> lock(g_status_mu);
+    const u32 used = g_status_used.load(std::memory_order_relaxed);
+    for (u32 i = 0; i < used; i++)
+        if (g_status[i].ctx == id) {
+            *out = g_status[i].word;
+            return cudaSuccess;
+        }
+    if (!create) return cudaSuccess;
+    // not a stream operation, so allowed while this thread captures one
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    ZK_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
+    void *p = nullptr;
+    const cudaError_t err = cudaHostAlloc(&p, sizeof(u32), cudaHostAllocMapped);
+    ZK_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
+    ZK_TRY(err);
+    u32 *word = static_cast<u32 *>(p);
+    *word = 0;
+    g_status[used < 64 ? used : g_status_next++ % 64] = {id, word};
+    if (used < 64) g_status_used.store(used + 1, std::memory_order_release);
+    *out = word;
+    return cudaSuccess;
+}
+// cudaErrorTimeout while the current context's word is set
+cudaError_t status_check() {
+    u32 *word = nullptr;
+    ZK_TRY(status_word(false, &word));
+    return word && __atomic_load_n(word, __ATOMIC_ACQUIRE) ? cudaErrorTimeout : cudaSuccess;
+}
+
 cudaError_t prepare_umma() {
     static std::atomic<uint64_t> done{0};
+    u32 *word = nullptr;
+    ZK_TRY(status_word(true, &word));
     return ensure_smem_attr(ntt_umma_kernel, (int)UM_SMEM, done);
 }
-cudaError_t launch_umma(const PassArgs &a, cudaStream_t stream) {
+cudaError_t launch_umma(const PassArgs &a, cudaStream_t stream, u32 polls = UM_POLLS) {
     ZK_TRY(prepare_umma());
+    u32 *word = nullptr;
+    ZK_TRY(status_word(true, &word));
     const u32 items = 1u << (a.L - UM_D - 7);
     const u32 grid = items < (u32)num_sms() ? items : (u32)num_sms();
-    ntt_umma_kernel<<<grid, UM_GROUPS * 128, UM_SMEM, stream>>>(a, items);
+    ntt_umma_kernel<<<grid, UM_GROUPS * 128, UM_SMEM, stream>>>(a, items, polls, word);
     return cudaGetLastError();
 }
 
@@ -860,6 +910,7 @@ inline cudaError_t prepare_run_attrs() {
 // Runs the full plan.  src (if non-null) is the pass-0 source for the coset LDE.
 cudaError_t run(const View &v, const View *src, u64 src_len, u32 L, const u32 *tw, const u32 *omegas,
                 const u32 *shift, const u32 *scale, cudaStream_t stream, const u32 *shoup = nullptr) {
+    ZK_TRY(status_check());
     // small transforms wait for their twiddle loads, and a Montgomery root is half a Shoup pair's
     // bytes (2^16 30.2 -> 27.9 us)
     if (L <= AHEAD_MAX_L) shoup = nullptr;
@@ -1188,6 +1239,7 @@ extern "C" cudaError_t zkp_ntt_batch_plan_create(const ZkpNttTask *tasks, unsign
 // launches only (no allocation, no host copies), so a stream capture can record it
 extern "C" cudaError_t zkp_ntt_batch_run(const ZkpNttBatchPlan *plan, cudaStream_t stream) {
     ZK_CHECK_ARG(plan != nullptr);
+    ZK_TRY(ntt::status_check());
     for (const auto &P : plan->phases) {
         if (P.count == 0 || P.grid == 0) continue;
         ntt::ntt_batch_pass_kernel<<<P.grid, P.threads, P.smem, stream>>>(P.args, P.first, P.count);
@@ -1219,6 +1271,26 @@ extern "C" void zkp_ntt_batch_plan_destroy(ZkpNttBatchPlan *plan) {
     cudaFree(plan->mem);
     cudaSetDevice(prev);
     delete plan;
+}
+
+extern "C" cudaError_t zkp_ntt_status(void) {
+    u32 *word = nullptr;
+    ZK_TRY(ntt::status_word(false, &word));
+    return word && __atomic_exchange_n(word, 0u, __ATOMIC_ACQ_REL) ? cudaErrorTimeout : cudaSuccess;
+}
+
+extern "C" cudaError_t zkp_ntt_wait_probe(PolyPtr x, const unsigned int *twiddle, unsigned int log_len,
+                                          unsigned int polls, cudaStream_t stream) {
+    View v;
+    ZK_CHECK_ARG(log_len <= 28 && x.len == (1ull << log_len) && make_view(x, &v));
+    ZK_CHECK_ARG(ntt::umma_ok(log_len, v, twiddle));
+    ntt::PassArgs a{};
+    a.v = v;
+    a.tw = twiddle;
+    a.L = log_len;
+    a.D = ntt::UM_D;
+    a.lo = log_len - ntt::UM_D;
+    return ntt::launch_umma(a, stream, polls);
 }
 
 extern "C" cudaError_t zkp_ntt_set_max_digit(unsigned int log_len, unsigned int max_digit) {

@@ -43,11 +43,10 @@ constexpr u32 UM_BAR = UM_A + UM_GROUPS * UM_A_BYTES;  // one mbarrier a group, 
 constexpr u32 UM_SMEM = UM_BAR + 64;
 // D = S32, A and B unsigned bytes, both K-major, N = 128, M = 128
 constexpr u32 UM_IDESC = (2u << 4) | ((UM_COLS >> 3) << 17) | ((UM_ROWS >> 4) << 24);
-// polls of an mbarrier before a group gives up (a pass runs well under a second)
-constexpr u32 UM_WAIT_LIMIT = 1u << 22;
-
-// set when a wait ran out (the results of that launch are then undefined)
-__device__ u32 g_um_timeouts;
+// A wait for the tensor core (some microseconds) gives up after this many polls of an mbarrier, each
+// of at most UM_POLL_NS: about a second.  Its group then stores nothing more, waits once more for what is in
+// flight, sets the context's status word (zkp_ntt_status) and leaves.
+constexpr u32 UM_POLLS = 1u << 16, UM_POLL_NS = 16384;
 
 ZK_DI u32 um_smem_addr(const void *p) { return (u32)__cvta_generic_to_shared(p); }
 // shared-memory matrix descriptor: no swizzle, K-major; core matrices of 8 rows x 16 bytes,
@@ -66,15 +65,15 @@ ZK_DI void um_mma(u32 tmem, u64 a, u64 b, bool accumulate) {
 ZK_DI void um_commit(u32 bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
-ZK_DI bool um_wait(u32 bar, u32 parity) {
-    for (u32 i = 0; i < UM_WAIT_LIMIT; i++) {
+ZK_DI bool um_wait(u32 bar, u32 parity, u32 polls) {
+    for (u32 i = 0; i < polls; i++) {
         u32 done;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
             "selp.b32 %0, 1, 0, p;\n\t}\n"
             : "=r"(done)
-            : "r"(bar), "r"(parity)
+            : "r"(bar), "r"(parity), "r"(UM_POLL_NS)
             : "memory");
         if (done) return true;
     }
@@ -83,7 +82,19 @@ ZK_DI bool um_wait(u32 bar, u32 parity) {
 ZK_DI void um_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 ZK_DI void um_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 ZK_DI void um_fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-ZK_DI void um_group_sync(u32 g) { asm volatile("bar.sync %0, 128;" ::"r"(g + 1) : "memory"); }
+// group barrier; whether any thread of the group passed true
+ZK_DI bool um_group_any(u32 g, bool f) {
+    u32 any;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %2, 0;\n\t"
+        "bar.red.or.pred q, %1, 128, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}\n"
+        : "=r"(any)
+        : "r"(g + 1), "r"(f ? 1u : 0u)
+        : "memory");
+    return any != 0;
+}
 
 // the warp's 32 TMEM lanes x 32 columns: this thread's row
 ZK_DI void um_load32(u32 tmem, u32 *c) {
@@ -197,7 +208,8 @@ ZK_DI void um_pencil(u64 item, u32 row, u32 lo, u32 log_h, u64 &c, u64 &h) {
 // The twiddle product is the Montgomery one also for callers with a Shoup table: these passes wait
 // for loads more than for the multiply pipe, and its root is 32 bytes, not 64 (2^24 2.92 -> 2.83 ms,
 // 2^22 0.752 -> 0.738).
-__global__ void __launch_bounds__(UM_GROUPS * 128, 1) ntt_umma_kernel(const PassArgs a, u32 items) {
+__global__ void __launch_bounds__(UM_GROUPS * 128, 1) ntt_umma_kernel(const PassArgs a, u32 items, u32 polls,
+                                                                       u32 *status) {
     extern __shared__ __align__(1024) unsigned char um_sm[];
     const u32 tid = threadIdx.x, g = tid >> 7, row = tid & 127;
     const u32 L = a.L, lo = a.lo;
@@ -246,12 +258,13 @@ __global__ void __launch_bounds__(UM_GROUPS * 128, 1) ntt_umma_kernel(const Pass
     unsigned char *A = um_sm + UM_A + g * UM_A_BYTES;
     const u32 a_addr = um_smem_addr(A), b_addr = um_smem_addr(um_sm);
     u32 parity = 0;
-    bool dead = false;
+    bool late = false;  // a wait of this warp ran out
 
-    // `steps` K steps of 32 bytes from A offset a_off and the constant block at b_off
+    // `steps` K steps of 32 bytes from A offset a_off and the constant block at b_off; false, and nothing
+    // issued, once a wait of the group has run out
     auto issue = [&](u32 a_off, u32 b_off, u32 b_lbo, u32 steps) {
         um_fence_before();
-        um_group_sync(g);
+        if (um_group_any(g, late)) return false;
         if (row == 0) {
             um_fence_after();
             for (u32 s = 0; s < steps; s++)
@@ -259,12 +272,14 @@ __global__ void __launch_bounds__(UM_GROUPS * 128, 1) ntt_umma_kernel(const Pass
                        um_desc(b_addr + b_off + s * 2 * b_lbo, b_lbo), s > 0);
             um_commit(bar);
         }
+        return true;
     };
     auto finish = [&]() {
-        if (!dead && !um_wait(bar, parity)) {
-            dead = true;
-            atomicAdd(&g_um_timeouts, 1u);
+        if (!um_wait(bar, parity, polls)) {
+            late = true;
+            um_wait(bar, parity, UM_POLLS);  // still in flight: reads A, writes TMEM
         }
+        late = __any_sync(0xffffffffu, late);
         parity ^= 1;
         um_fence_after();
     };
@@ -276,6 +291,7 @@ __global__ void __launch_bounds__(UM_GROUPS * 128, 1) ntt_umma_kernel(const Pass
     // outputs k = k0, k0 + dk, ... (four of them) from the group's TMEM columns; an output's twiddle
     // is loaded one output ahead
     auto drain = [&](u32 k0, u32 dk, Fr r) {
+        if (late) return;
 #pragma unroll 1
         for (u32 o = 0; o < 4; o++) {
             const u32 k = k0 + o * dk;
@@ -310,11 +326,11 @@ __global__ void __launch_bounds__(UM_GROUPS * 128, 1) ntt_umma_kernel(const Pass
             um_put(A, j, row, um_sub_raw(x0, x1));
         }
         um_fence_async();
-        issue(0, 0, 4096, 8);  // outputs 1, 3, 5, 7
+        if (!issue(0, 0, 4096, 8)) break;  // outputs 1, 3, 5, 7
         Fr r = root(1);
         finish();
         drain(1, 2, r);
-        issue(0, 128 * 16, 4096, 8);  // outputs 9, 11, 13, 15
+        if (!issue(0, 128 * 16, 4096, 8)) break;  // outputs 9, 11, 13, 15
         r = root(9);
         finish();
         // A is free again: the even half's second stage
@@ -325,13 +341,17 @@ __global__ void __launch_bounds__(UM_GROUPS * 128, 1) ntt_umma_kernel(const Pass
         }
         um_fence_async();
         drain(9, 2, r);
-        issue(4 * 2 * (UM_ROWS * 16), UM_B_SD, 2048, 4);  // outputs 2, 6, 10, 14
+        if (!issue(4 * 2 * (UM_ROWS * 16), UM_B_SD, 2048, 4)) break;  // outputs 2, 6, 10, 14
         r = root(2);
         finish();
         drain(2, 4, r);
-        issue(0, UM_B_SS, 2048, 4);  // outputs 0, 4, 8, 12
+        if (!issue(0, UM_B_SS, 2048, 4)) break;  // outputs 0, 4, 8, 12
         finish();
         drain(0, 4, r);
+    }
+    if (late && (tid & 31) == 0) {
+        *(volatile u32 *)status = 1;
+        __threadfence_system();
     }
     um_fence_before();
     __syncthreads();

@@ -122,6 +122,7 @@ struct Request {
     bool done = false;
     cudaStream_t stream = nullptr;  // the slot's stream of the request's priority class
     bool large = false;             // counted against the policy's large-request limit
+    bool spoiled = false;           // was in flight when a transform's wait ran out
     // a request of a compiled program (null for the built-in prover program)
     const ZkpProgram *prog = nullptr;
     std::vector<const void *> inputs;
@@ -501,6 +502,13 @@ void finish(ZkpServer *s, Request *r, int status) {
         s->stats.failed++;
 }
 
+// A transform's wait that ran out (zkp_ntt_status) may have been any request's in flight: all of them fail.
+void note_timeout(ZkpServer *s) {
+    if (zkp_ntt_status() != cudaErrorTimeout) return;
+    for (auto &slot : s->slots)
+        if (slot.req) slot.req->spoiled = true;
+}
+
 // a request of the class the policy limits; the class is fixed at admission (r->large)
 bool is_large(const ZkpServer *s, Request *r) {
     if (r->slot < 0) r->large = s->policy.max_large_inflight && s->policy.large_bytes &&
@@ -519,7 +527,8 @@ void worker_loop(ZkpServer *s) {
             cudaError_t q = cudaEventQuery(slot.done);
             if (q == cudaErrorNotReady) continue;
             Request *r = slot.req;
-            if (q == cudaSuccess) {
+            if (q == cudaSuccess) note_timeout(s);
+            if (q == cudaSuccess && !r->spoiled) {
                 if (r->prog) {
                     for (const ZkpProgOut &o : r->prog->outs)
                         memcpy(static_cast<char *>(r->results) + o.result_offset, slot.prog_host + o.host_offset,
@@ -590,6 +599,7 @@ void worker_loop(ZkpServer *s) {
                 if (e == cudaSuccess) slot.prog_host_bytes = r->prog->host_bytes;
             }
             if (e == cudaSuccess) e = r->prog ? launch_compiled(s, r, slot) : launch_program(s, r, slot);
+            if (e == cudaErrorTimeout) note_timeout(s);
             if (e != cudaSuccess) {
                 // the request fails alone: drain what was queued on its stream, release it
                 cudaStreamSynchronize(r->stream);

@@ -142,6 +142,12 @@ def num_passes(log_len: int) -> int:
     return int(_lib().zkp_ntt_num_passes(log_len))
 
 
+def status() -> None:
+    """Raises if a wait inside a transform's kernel ran out since the last call (the vector is then
+    undefined, and transforms refuse until this has been called); call after a synchronisation."""
+    check(_lib().zkp_ntt_status(), "zkp_ntt_status")
+
+
 # ------------------------------------------------------------------ cached constants
 @functools.lru_cache(maxsize=64)
 def twiddle_table(log_n: int, inverse: bool = False, device: str = "cuda") -> ScalarArray:
