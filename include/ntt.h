@@ -53,7 +53,8 @@ cudaError_t zkp_ntt_ex(PolyPtr x, const unsigned int *twiddle, unsigned int log_
                        const unsigned int *scale_d, cudaStream_t stream);
 
 /* Coset low-degree extension: out (len 2^log_out) = DFT_{2^log_out}(in[i] * shift^i, zero
- * padded), in has length 2^log_in <= 2^log_out; twiddle is the table for 2^log_out. */
+ * padded), in has length 2^log_in <= 2^log_out; twiddle is the table for 2^log_out.  in may be the first
+ * elements of out; up to 2^12 points it may also lie elsewhere in out's buffer. */
 cudaError_t zkp_coset_lde(PolyPtr out, ConstPolyPtr in, const unsigned int *twiddle, unsigned int log_in,
                           unsigned int log_out, const unsigned int *shift_d, cudaStream_t stream);
 

@@ -490,3 +490,29 @@ def test_wait_probe_refuses_other_passes(zk):
     lib = zk.native.load(zk.ntt.LIB)
     x, tw = zk.ScalarArray.zeros(1 << 10), zk.ntt.twiddle_table(10)
     assert lib.zkp_ntt_wait_probe(x.poly_ptr(), tw.values.data_ptr(), 10, 0, None) == 1
+
+
+@pytest.mark.parametrize("log_out", [9, 10, 12])
+@pytest.mark.parametrize("where", ["upper half", "rotated", "shifted by one", "wrapped", "in place"])
+def test_coset_from_its_own_buffer(zk, orc, log_out, where):
+    """An extension (up to 2^12 points) whose coefficients lie in the output's buffer, at other places than
+    the outputs of the same index: all of them are read before the first one is written."""
+    n = 1 << log_out
+    a = orc.gen_fr(360, n)
+    out = to_dev(zk, a)
+    if where == "upper half":
+        coef = out.slice(n // 2, n)
+    elif where == "rotated":
+        coef = zk.ScalarArray(out.values)
+        coef.rotate(n // 3)
+    elif where == "shifted by one":
+        coef = out.slice(1, n // 2 + 1)
+    elif where == "wrapped":
+        coef = out.set_slice_raw(n - 5, n // 4)
+    else:
+        coef = out.slice(0, n // 2)
+    log_in = coef.len.bit_length() - 1
+    expect = orc.coset_ntt(np.ascontiguousarray(coef.numpy_u64()), log_in, log_out,
+                           orc.to_mont(orc.int_to_limbs(7)))
+    zk.ntt.coset_ntt(out, coef)
+    assert np.array_equal(out.numpy_u64(), expect)

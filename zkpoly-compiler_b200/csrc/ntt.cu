@@ -715,15 +715,14 @@ inline Plan umma_plan(u32 L) {
 // with the large tile).
 constexpr u32 SMALL_TILE = 4, SMALL_TILE_MIN_L = 10, SMALL_TILE_MAX_L = 17;
 
-// Plan for 2^L elements.  The tuned digit cap applies to plain table-mode transforms.  A
-// transform whose first pass multiplies by a coset shift or reads a shorter source keeps that
-// pass at up to MAX_D bits: the first pass builds per-pencil shift tables, and the cost of
-// that set-up grows with the number of pencils.  Recompute mode (roots rebuilt per pencil) and
-// the batched form (one shared-memory pencil kernel for every pass) ignore the cap.
-inline Plan make_plan(u32 L, bool wide_first = false, bool ignore_cap = false) {
+// Plan for 2^L elements.  The tuned digit cap applies to plain table-mode transforms.  Recompute mode
+// (roots rebuilt per pencil) and the batched form (one shared-memory pencil kernel for every
+// pass) ignore it, and so does a transform in one_pass (L <= MAX_D), which multiplies by a coset
+// shift or reads another vector as it goes.
+inline Plan make_plan(u32 L, bool one_pass = false, bool ignore_cap = false) {
     Plan p{};
-    const u32 cap = ignore_cap ? MAX_D : digit_cap(L);
-    if (!wide_first && !ignore_cap && L >= SMALL_TILE_MIN_L && L <= SMALL_TILE_MAX_L) {
+    const u32 cap = ignore_cap || one_pass ? MAX_D : digit_cap(L);
+    if (!one_pass && !ignore_cap && L >= SMALL_TILE_MIN_L && L <= SMALL_TILE_MAX_L) {
         // register passes of at most 2^6 points, the last one of 2^4 with the small tile
         const u32 c = cap < WARP_MAX_D ? cap : WARP_MAX_D;
         split_digits(p, 0, L - SMALL_TILE, c);
@@ -732,21 +731,31 @@ inline Plan make_plan(u32 L, bool wide_first = false, bool ignore_cap = false) {
         p.lo[p.np++] = 0;
         return p;
     }
-    const u32 first_cap = wide_first ? (cap > MAX_D ? cap : MAX_D) : cap;
-    if (L <= first_cap) {
+    if (L <= cap) {
         p.np = 1;
         p.D[0] = L;
         p.lo[0] = 0;
         return p;
     }
-    if (!wide_first || first_cap == cap) {
-        split_digits(p, 0, L, cap);
-        return p;
-    }
-    p.D[0] = first_cap;
-    p.lo[0] = L - first_cap;
-    split_digits(p, 1, L - first_cap, cap);
+    split_digits(p, 0, L, cap);
     return p;
+}
+
+// whether an element of src may lie where v has another one, so that a pass from src to v by more
+// than one CTA would read overwritten elements
+inline bool tangled(const View &v, const View &src) {
+    auto range = [](const View &x, const char *&lo, const char *&hi) {
+        const u64 first = contiguous(x) ? x.off : 0, count = contiguous(x) ? x.len : x.whole;
+        lo = reinterpret_cast<const char *>(x.base) + first * 32;
+        hi = lo + count * 32;
+    };
+    const char *v0, *v1, *s0, *s1;
+    range(v, v0, v1);
+    range(src, s0, s1);
+    if (s1 <= v0 || v1 <= s0) return false;
+    const bool same = src.base == v.base && src.off == v.off &&
+                      (src.whole == v.whole || (contiguous(src) && contiguous(v)));
+    return !same;
 }
 
 std::atomic<uint64_t> g_attr_done{0};
@@ -915,7 +924,9 @@ cudaError_t run(const View &v, const View *src, u64 src_len, u32 L, const u32 *t
     // bytes (2^16 30.2 -> 27.9 us)
     if (L <= AHEAD_MAX_L) shoup = nullptr;
     profiler().begin(stream);
-    if (omegas == nullptr && (shift != nullptr || src != nullptr) && L >= PREP_MIN_L) {
+    // up to 2^MAX_D points one CTA can read the whole source before it writes
+    const bool one_pass = L < PREP_MIN_L || (L <= MAX_D && src != nullptr && tangled(v, *src));
+    if (omegas == nullptr && (shift != nullptr || src != nullptr) && !one_pass) {
         // a multi-pass table-mode plan: shift and zero-extend in one elementwise pass, then the
         // plain transform in place
         const u64 n = 1ull << L;
@@ -1141,7 +1152,7 @@ extern "C" cudaError_t zkp_ntt_batch_plan_create(const ZkpNttTask *tasks, unsign
             plan->solo.push_back({v, L, task.twiddle, task.shift_d, task.scale_d, task.shoup_d});
             continue;
         }
-        const ntt::Plan p = ntt::make_plan(L, task.shift_d != nullptr, /*ignore_cap=*/true);
+        const ntt::Plan p = ntt::make_plan(L, false, /*ignore_cap=*/true);
         for (u32 ph = 0; ph < p.np; ph++) {
             if (args.size() <= ph) {
                 args.emplace_back();
