@@ -88,17 +88,24 @@ cudaError_t zkp_ntt_roots_device(unsigned int *out_d, unsigned long long count, 
  *
  * Plan tuning (no counterpart in the reference): caps the digit width of the passes used for
  * transforms of 2^log_len elements (log_len 0: every size) at max_digit in [4, 12] (0 restores
- * the default 12).  Each pass transforms 2^D-element pencils in shared memory, D <= max_digit;
- * a smaller cap means more passes of smaller CTAs.  Plans made after the call use it. */
+ * the default 12).  A pass of D bits transforms 2^D-element pencils: in registers up to 6 bits, else
+ * in shared memory by one CTA a pencil.  Below 2^10 and from 2^18 to 2^20 elements the bits are split
+ * evenly into the fewest passes of at most max_digit; from 2^10 to 2^17 they are register passes of
+ * at most 6 bits (or max_digit if less) and a last one of 4; from 2^21 tensor-core passes of 4
+ * bits, with CTAs that fill an SM, and a last register pass of 5 bits where the cap allows it, else 4
+ * (the split of the smaller sizes for buffers that are not 32-byte aligned).  Plans made after the
+ * call use it. */
 cudaError_t zkp_ntt_set_max_digit(unsigned int log_len, unsigned int max_digit);
 /* CTA size (32, 64, 128 or 256 threads; 0 = 128) of the register passes of transforms of
- * 2^log_len elements (log_len 0: every size), set by the autotuner (no counterpart in the
- * reference, whose launch shapes follow max_threads_stage*_log).  Results do not depend on it. */
+ * 2^log_len elements (log_len 0: every size) but the last, whose CTA follows its tile; set by the
+ * autotuner (no counterpart in the reference, whose launch shapes follow max_threads_stage*_log).
+ * From 2^21 only a first pass of 1 to 3 bits is left of them, at sizes that need one.  Results do not depend on
+ * it. */
 cudaError_t zkp_ntt_set_block(unsigned int log_len, unsigned int threads);
 
 /* The digit widths, top digit first, of the sub-transform passes the current plan for
- * 2^log_len uses (at most max written); returns the number of passes (0 if log_len is 0 or
- * above 28). */
+ * 2^log_len uses over 32-byte aligned buffers (at most max written); returns the number of passes
+ * (0 if log_len is 0 or above 28). */
 unsigned int zkp_ntt_plan_digits(unsigned int log_len, unsigned int *digits, unsigned int max);
 
 /* Number of sub-transform passes + permutation passes the plan for 2^log_len uses. */

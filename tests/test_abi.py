@@ -49,3 +49,25 @@ def test_reference_stage_plan_helpers(zk):
     # GenPqOmegas::get_pq_len (core/src/ntt.rs:322-335) for 32-byte fields, caps (8, 8)
     assert zk.ntt.get_pq_len(16) == 1 << 7
     assert zk.ntt.get_pq_len(24) == 1 << 5
+
+
+def test_plan_digits_follow_the_documented_cap(zk):
+    """zkp_ntt_set_max_digit by size, as the header describes it (plans are host code)."""
+    lib = ctypes.CDLL(os.path.join(ROOT, "zkpoly-compiler_b200", "lib", "libntt.so"))
+
+    def digits(log_n, cap):
+        assert lib.zkp_ntt_set_max_digit(log_n, cap) == 0
+        buf = (ctypes.c_uint * 8)()
+        k = lib.zkp_ntt_plan_digits(log_n, buf, 8)
+        assert lib.zkp_ntt_set_max_digit(log_n, 0) == 0
+        return [buf[i] for i in range(k)]
+    for log_n in range(1, 29):
+        for cap in range(4, 13):
+            d = digits(log_n, cap)
+            assert sum(d) == log_n and max(d) <= cap, (log_n, cap, d)
+            if 10 <= log_n <= 17:
+                assert max(d) <= 6 and d[-1] == 4
+            elif log_n >= 21:
+                assert d[-1] in (4, 5) and d[-2] == 4 and d == digits(log_n, 4 if cap == 4 else 5)
+            else:
+                assert len(d) == -(-log_n // cap) and max(d) - min(d) <= 1

@@ -516,3 +516,15 @@ def test_coset_from_its_own_buffer(zk, orc, log_out, where):
                            orc.to_mont(orc.int_to_limbs(7)))
     zk.ntt.coset_ntt(out, coef)
     assert np.array_equal(out.numpy_u64(), expect)
+
+
+def test_tuner_times_a_plan_once(zk, monkeypatch):
+    """Digit caps that leave a size's plan as it is are not candidates of their own."""
+    monkeypatch.setattr(zk.tuner, "_save", lambda: None)
+    saved = {k: dict(v) for k, v in zk.tuner._load().get(zk.tuner._device_key(), {}).items()}
+    try:
+        times = zk.tuner.tune_ntt(log_ns=[12, 18], candidates=(4, 5, 6, 8, 12), apply=False)["ms"]
+        assert sorted(times) == ["12:4", "18:12", "18:4", "18:5", "18:6"]
+    finally:
+        zk.tuner._load()[zk.tuner._device_key()] = saved
+        zk.tuner.apply_ntt_plans()

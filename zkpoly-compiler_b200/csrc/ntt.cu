@@ -4,13 +4,14 @@
 // recompute_ntt.cuh:23-438) behind the same C ABI (core/src/ntt/src/ntt.h:5-16).
 //
 // Algorithm (n = 2^L).  The index bits are split into digits of at most 12 bits, top digit
-// first.  Pass p takes every "pencil" of 2^D elements that differ only in digit p (bits
+// first (passes of at most 6 bits run in registers, below, and from 2^21 points passes of 4 bits on
+// the tensor cores, ntt_umma.cuh; this describes the general pass).  Pass p takes every "pencil" of 2^D elements that differ only in digit p (bits
 // [lo, lo + D)), runs a radix-2 DIF sub-transform on it in shared memory (its output lands
 // bit-reversed inside the digit), and, when lower digits remain, multiplies element k of the
 // sub-transform by the four-step twist w_N^(c*k), where c is the pencil's value of the lower
 // digits and N = 2^(lo + D).  After the last digit the whole vector is in bit-reversed order;
-// a final in-place permutation pass swaps i <-> rev(i).  For L <= 12 one CTA does the whole
-// transform and writes natural order directly.
+// a final in-place permutation pass swaps i <-> rev(i), fused with the last pass where that is of
+// at most 5 bits.  In one pass (L <= 12) a CTA does the whole transform and writes natural order.
 //
 // Every pass reads and writes the same pencil, so all passes run in place on the caller's
 // buffer with no scratch memory.  Intermediate values stay in [0, 2m) (lazy Montgomery);
@@ -661,8 +662,8 @@ struct Plan {
 };
 
 // Per-size cap on the digit width (the sub-transform size 2^D of a pass), set by the tuner
-// through zkp_ntt_set_max_digit; 0 means MAX_D.  A smaller cap means more passes but smaller
-// CTAs, several of which share an SM (one loads or stores while another computes).
+// through zkp_ntt_set_max_digit; 0 means MAX_D.  In the shared-memory passes a smaller cap means more
+// passes but smaller CTAs, several of which share an SM (one loads or stores while another computes).
 std::atomic<u32> g_max_digit[29];
 
 inline u32 digit_cap(u32 L) {

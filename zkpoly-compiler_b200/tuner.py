@@ -139,9 +139,13 @@ def tune_ntt(log_ns=range(14, 25), candidates=(8, 9, 10, 11, 12), apply: bool = 
         x = ScalarArray(gen.fr(79, 1 << L))
         tw = ntt.twiddle_table(L)
         run = (lambda: ntt.ntt(x)) if path == "shoup" else (lambda: ntt.ssip_ntt(x, tw))
-        best = None
+        best, plans = None, set()
         for d in candidates:
             check(lib.zkp_ntt_set_max_digit(L, d), "zkp_ntt_set_max_digit")
+            plan = tuple(ntt.plan_digits(L))
+            if plan in plans:  # the cap makes no difference at this size
+                continue
+            plans.add(plan)
             t = _time(run, reps=10 if L < 20 else 3)
             times[f"{L}:{d}"] = t
             if best is None or t < best[1]:
