@@ -69,7 +69,10 @@ cudaError_t zkp_ntt_shoup_table(const unsigned int *twiddle_d, unsigned int log_
  * passes of transforms from 2^18 points multiply by its entries, 207 multiply instructions per
  * twiddle product instead of the Montgomery product's 256, identical results.  Smaller transforms
  * and the tensor-core passes read the Montgomery table, whose entries are half as long; twiddle is
- * always needed.  shoup_d = NULL gives zkp_ntt_ex / zkp_coset_lde. */
+ * always needed.  shoup_d = NULL gives zkp_ntt_ex / zkp_coset_lde.  zkp_ntt_wants_shoup: 1 for the sizes
+ * at which a table is worth its 64 bytes a root: below 2^18 it is not read, from 2^21 only by the
+ * register passes around the tensor-core ones (2^22 the same time without it, 2^24 0.4 % more). */
+int zkp_ntt_wants_shoup(unsigned int log_len);
 cudaError_t zkp_ntt_ex_shoup(PolyPtr x, const unsigned int *twiddle, const unsigned int *shoup_d,
                              unsigned int log_len, const unsigned int *shift_d, const unsigned int *scale_d,
                              cudaStream_t stream);

@@ -528,3 +528,20 @@ def test_tuner_times_a_plan_once(zk, monkeypatch):
     finally:
         zk.tuner._load()[zk.tuner._device_key()] = saved
         zk.tuner.apply_ntt_plans()
+
+
+def test_shoup_tables_only_where_they_are_worth_it(zk, orc):
+    """The library's own transforms build no Shoup table at sizes that do not read one."""
+    zk.ntt.shoup_table.cache_clear()
+    for log_n, tables in ((1, 0), (12, 0), (17, 0), (18, 1), (21, 1)):
+        a = orc.gen_fr(370 + log_n, 1 << log_n)
+        x = to_dev(zk, a)
+        zk.ntt.ntt(x)
+        assert zk.ntt.shoup_table.cache_info().currsize == tables, log_n
+        assert np.array_equal(x.numpy_u64(), orc.best_fft(a, orc.root_of_unity(log_n), log_n))
+    zk.ntt.shoup_table.cache_clear()
+    x = to_dev(zk, orc.gen_fr(380, 1 << 16))
+    zk.ntt.intt(x)
+    zk.ntt.NttBatch([(x, "ntt"), (to_dev(zk, orc.gen_fr(381, 1 << 8)), "coset")]).run()
+    zk.ntt.coset_ntt(zk.ScalarArray.zeros(1 << 17), x)
+    assert zk.ntt.shoup_table.cache_info().currsize == 0

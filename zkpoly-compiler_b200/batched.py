@@ -87,7 +87,7 @@ class MixedWorkload:
             self.build_plain_same_tables()
         for x, L, kind in zip(self.ntt_bufs, self.ntt_logs, self.ntt_kinds):
             inv = kind == "intt"
-            tw, sh = ntt.twiddle_table(L, inv), ntt.shoup_table(L, inv)
+            tw, sh = ntt.twiddle_table(L, inv), ntt.wanted_shoup(L, inv)
             if kind == "ntt":
                 ntt.ntt_ex(x, tw, None, None, stream, shoup=sh)
             elif kind == "intt":

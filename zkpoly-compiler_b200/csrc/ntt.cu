@@ -1050,6 +1050,10 @@ extern "C" cudaError_t zkp_coset_lde_shoup(PolyPtr out, ConstPolyPtr in, const u
     return ntt::run(vo, &vi, in.len, log_out, twiddle, nullptr, shift_d, nullptr, stream, shoup_d);
 }
 
+extern "C" int zkp_ntt_wants_shoup(unsigned int log_len) {
+    return log_len > ntt::AHEAD_MAX_L && log_len < ntt::UM_MIN_L ? 1 : 0;
+}
+
 // Shoup-product throughput probe (the twiddle product of the register passes): every thread
 // runs two independent chains of `iters` products x = x * w by fixed factors.
 __global__ void __launch_bounds__(256) shoup_probe_kernel(u32 iters, u32 *out) {

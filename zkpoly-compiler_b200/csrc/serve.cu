@@ -101,7 +101,7 @@ class Arena {
 struct SizeConsts {
     u32 *inv_tw = nullptr;   // inverse roots, 2^(k-1) entries
     u32 *fwd_tw = nullptr;   // forward roots of the extended size, 2^(k+ext-1) entries
-    u32 *inv_sh = nullptr;   // Shoup tables of the two (16 words per root)
+    u32 *inv_sh = nullptr;   // Shoup tables of the two (16 words per root), where zkp_ntt_wants_shoup
     u32 *fwd_sh = nullptr;
     u32 *ninv = nullptr;     // n^-1
     u32 *zh_inv = nullptr;   // 2^ext values of 1/Z_H on the coset
@@ -682,8 +682,8 @@ extern "C" cudaError_t zkp_serve_create(const ZkpServeConfig *cfg, const unsigne
         const u64 n = 1ull << k;
         e = cudaMalloc(&c.inv_tw, (n / 2) * 32);
         if (e == cudaSuccess) e = cudaMalloc(&c.fwd_tw, (n << ext) / 2 * 32);
-        if (e == cudaSuccess) e = cudaMalloc(&c.inv_sh, (n / 2) * 64);
-        if (e == cudaSuccess) e = cudaMalloc(&c.fwd_sh, (n << ext) / 2 * 64);
+        if (e == cudaSuccess && zkp_ntt_wants_shoup(k)) e = cudaMalloc(&c.inv_sh, (n / 2) * 64);
+        if (e == cudaSuccess && zkp_ntt_wants_shoup(k + ext)) e = cudaMalloc(&c.fwd_sh, (n << ext) / 2 * 64);
         if (e == cudaSuccess) e = cudaMalloc(&c.ninv, 32);
         if (e == cudaSuccess) e = cudaMalloc(&c.zh_inv, (32u << ext));
         if (e != cudaSuccess) break;
@@ -694,8 +694,8 @@ extern "C" cudaError_t zkp_serve_create(const ZkpServeConfig *cfg, const unsigne
         zkh::Fe wf = zkh::fr_root_of_unity(k + ext, false);
         if (e == cudaSuccess) e = cudaMemcpy(tmp, wf.l, 32, cudaMemcpyHostToDevice);
         if (e == cudaSuccess) e = zkp_ntt_roots_device(c.fwd_tw, (n << ext) / 2, tmp, 0);
-        if (e == cudaSuccess) e = zkp_ntt_shoup_table(c.inv_tw, k, c.inv_sh, 0);
-        if (e == cudaSuccess) e = zkp_ntt_shoup_table(c.fwd_tw, k + ext, c.fwd_sh, 0);
+        if (e == cudaSuccess && c.inv_sh) e = zkp_ntt_shoup_table(c.inv_tw, k, c.inv_sh, 0);
+        if (e == cudaSuccess && c.fwd_sh) e = zkp_ntt_shoup_table(c.fwd_tw, k + ext, c.fwd_sh, 0);
         if (e == cudaSuccess) e = cudaDeviceSynchronize();
         zkh::Fe ninv = zkh::inv(F, zkh::from_u64(F, n));
         if (e == cudaSuccess) e = cudaMemcpy(c.ninv, ninv.l, 32, cudaMemcpyHostToDevice);

@@ -52,6 +52,7 @@ SIGNATURES = {
                                               c_void_p, c_void_p]),
         "zkp_ntt_num_passes": (ctypes.c_uint, [ctypes.c_uint]),
         "zkp_ntt_status": (cudaError_t, []),
+        "zkp_ntt_wants_shoup": (ctypes.c_int, [ctypes.c_uint]),
         "zkp_ntt_wait_probe": (cudaError_t, [PolyPtr, c_void_p, ctypes.c_uint, ctypes.c_uint, c_void_p]),
         "zkp_ntt_plan_digits": (ctypes.c_uint, [ctypes.c_uint, c_void_p, ctypes.c_uint]),
         "zkp_ntt_set_max_digit": (cudaError_t, [ctypes.c_uint, ctypes.c_uint]),

@@ -173,25 +173,34 @@ def shoup_table(log_n: int, inverse: bool = False, device: str = "cuda") -> torc
     return tab
 
 
+@functools.lru_cache(maxsize=None)
+def _wants_shoup(log_n: int) -> bool:
+    return bool(_lib().zkp_ntt_wants_shoup(log_n))
+
+
+def wanted_shoup(log_n: int, inverse: bool = False) -> torch.Tensor | None:
+    """shoup_table(log_n, inverse) at the sizes whose transforms are faster with it, else None."""
+    return shoup_table(log_n, inverse) if _wants_shoup(log_n) else None
+
+
 def n_inv(log_n: int, device: str = "cuda") -> torch.Tensor:
     return scalar_const(pow(1 << log_n, -1, field.FR_MODULUS), device)
 
 
 # ------------------------------------------------------------------ compiler-level compositions
 def ntt(x: ScalarArray, stream=None) -> None:
-    """Forward NTT at the natural root of the size (NTT(w)); the register passes multiply by the
-    Shoup table of the root table (same values as ssip_ntt with the root table alone)."""
+    """Forward NTT at the natural root of the size (NTT(w)), with the Shoup table of the root table where
+    that is worth its memory (same values as ssip_ntt with the root table alone)."""
     log_n = _log2_exact(x.len)
     if log_n == 0:
         return
-    ntt_ex(x, twiddle_table(log_n, False), stream=stream, shoup=shoup_table(log_n, False))
+    ntt_ex(x, twiddle_table(log_n, False), stream=stream, shoup=wanted_shoup(log_n))
 
 
 def intt(x: ScalarArray, stream=None) -> None:
     """INTT = NTT(w^-1) then * n^-1 (intt_mending.rs:11-70), the scale fused into the last pass."""
     log_n = _log2_exact(x.len)
-    ntt_ex(x, twiddle_table(log_n, True), None, n_inv(log_n), stream,
-           shoup=shoup_table(log_n, True) if log_n >= 1 else None)
+    ntt_ex(x, twiddle_table(log_n, True), None, n_inv(log_n), stream, shoup=wanted_shoup(log_n, True))
 
 
 def coset_ntt(out: ScalarArray, coef: ScalarArray, shift: int = field.GENERATOR, stream=None) -> None:
@@ -199,7 +208,7 @@ def coset_ntt(out: ScalarArray, coef: ScalarArray, shift: int = field.GENERATOR,
     multiply by shift^i, NTT at the extended size, all fused (poly_coef.rs:252-255 Extend +
     distribute_powers.cuh:5-21 + NTT)."""
     log_n = _log2_exact(out.len)
-    coset_lde(out, coef, twiddle_table(log_n, False), scalar_const(shift), stream, shoup=shoup_table(log_n, False))
+    coset_lde(out, coef, twiddle_table(log_n, False), scalar_const(shift), stream, shoup=wanted_shoup(log_n))
 
 
 # ------------------------------------------------------------------ batched form
@@ -221,9 +230,9 @@ class NttBatch:
             tw = twiddle_table(log_n, inverse)
             sh = scalar_const(shift) if kind == "coset" else None
             sc = n_inv(log_n) if inverse else None
-            st = shoup_table(log_n, inverse)
+            st = wanted_shoup(log_n, inverse)
             self._keep += [x, tw, sh, sc, st]
-            arr[i] = ZkpNttTask(x.poly_ptr(), tw.values.data_ptr(), log_n, _ptr(sh), _ptr(sc), st.data_ptr())
+            arr[i] = ZkpNttTask(x.poly_ptr(), tw.values.data_ptr(), log_n, _ptr(sh), _ptr(sc), _ptr(st))
         self._plan = ctypes.c_void_p()
         self._destroy = lib.zkp_ntt_batch_plan_destroy  # kept: module globals may be gone at exit
         check(lib.zkp_ntt_batch_plan_create(ctypes.cast(arr, ctypes.c_void_p), len(tasks),

@@ -302,11 +302,12 @@ class Lowering:
         return replace(v, device="gpu", addr=self._dev_const[v.addr].data_ptr())
 
     def shoup_for(self, tw: Var, log_n: int) -> int:
-        """Shoup table of a full root table constant (built once, like the root table itself)."""
+        """Shoup table of a full root table constant (built once, like the root table itself), or 0 where
+        there is none or it is not worth its memory."""
         from . import ntt
         from .scalar import ScalarArray
         if tw.space != SPACE_ABS or tw.len != (1 << log_n) // 2 or tw.whole != tw.len or tw.rotate or tw.offset \
-                or log_n < 1:
+                or log_n < 1 or not load(ntt.LIB).zkp_ntt_wants_shoup(log_n):
             return 0
         if tw.addr not in self._shoup:
             words = self._tensors.get(tw.addr)
