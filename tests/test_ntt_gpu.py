@@ -545,3 +545,23 @@ def test_shoup_tables_only_where_they_are_worth_it(zk, orc):
     zk.ntt.NttBatch([(x, "ntt"), (to_dev(zk, orc.gen_fr(381, 1 << 8)), "coset")]).run()
     zk.ntt.coset_ntt(zk.ScalarArray.zeros(1 << 17), x)
     assert zk.ntt.shoup_table.cache_info().currsize == 0
+
+
+@pytest.mark.parametrize("log_n", [21, 22, 23])
+@pytest.mark.parametrize("fill", ["zero", "first", "last", "middle", "few", "every 16th"])
+def test_ntt_radix16_mostly_zero(zk, orc, log_n, fill):
+    """Zeros through the tensor-core passes, whose sign flip stores a zero as 2r: outputs are canonical."""
+    n = 1 << log_n
+    a = np.zeros((n, 4), dtype=np.uint64)
+    at = {"zero": [], "first": [0], "last": [n - 1], "middle": [n // 2 + 5], "few": list(range(8)),
+          "every 16th": list(range(0, n, 16))}[fill]
+    a[at] = orc.gen_fr(390, len(at)) if at else a[at]
+    x = to_dev(zk, a)
+    zk.ntt.ntt(x)
+    assert np.array_equal(x.numpy_u64(), orc.best_fft(a, orc.root_of_unity(log_n), log_n))
+    zk.ntt.intt(x)
+    assert np.array_equal(x.numpy_u64(), a)
+    if fill == "few":
+        g = orc.to_mont(orc.int_to_limbs(7))
+        zk.ntt.coset_ntt(x, to_dev(zk, a[:8]))
+        assert np.array_equal(x.numpy_u64(), orc.coset_ntt(a[:8], 3, log_n, g))

@@ -134,7 +134,7 @@ ZK_DI void um_st(u32 *p, const Fr &x) {
                  : "memory");
 }
 
-// a + b and a - b + 2m without a fold: below 4m for a, b <= 2m, so still 256 bits
+// a + b and a - b + 2m without a fold: at most 4m for a, b <= 2m, so still 256 bits
 ZK_DI Fr um_add_raw(const Fr &a, const Fr &b) {
     Fr r;
     r.v[0] = add_cc(a.v[0], b.v[0]);
@@ -301,7 +301,13 @@ __global__ void __launch_bounds__(UM_GROUPS * 128, 1) ntt_umma_kernel(const Pass
             Fr x = um_combine(cs);
             if (k != 0) {
                 x = Fr::mul(x, r);
-                if (((c * k) << esh) >= half) {  // w^(n/2) = -1
+                // w^(n/2) = -1.  2r - 0 is 2r itself: these passes store and take the closed range [0, 2r]
+                // (a sum of two is at most 4r and folds to at most 2r).  The last pass, in registers,
+                // canonicalises [0, 2r) only, and meets no more: its outputs are a + b and a - b with a the
+                // first element of a butterfly block, which is the pencil's element 0 plus and minus
+                // others, never multiplied.  That one came from c = 0, is not flipped and so below 2r,
+                // and a +- b folded is below 2r if a is and b is at most 2r.
+                if (((c * k) << esh) >= half) {
                     Fr m2;
 #pragma unroll
                     for (int i = 0; i < 8; i++) m2.v[i] = FrParams::m2(i);
