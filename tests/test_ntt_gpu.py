@@ -565,3 +565,22 @@ def test_ntt_radix16_mostly_zero(zk, orc, log_n, fill):
         g = orc.to_mont(orc.int_to_limbs(7))
         zk.ntt.coset_ntt(x, to_dev(zk, a[:8]))
         assert np.array_equal(x.numpy_u64(), orc.coset_ntt(a[:8], 3, log_n, g))
+
+
+def test_batch_of_large_tasks_captured(zk, orc):
+    """Batch tasks of the tensor-core sizes beside a small one, in a stream capture and replayed."""
+    import torch
+    g = orc.to_mont(orc.int_to_limbs(7))
+    sizes = ((21, "ntt"), (22, "intt"), (21, "coset"), (10, "ntt"))
+    vecs = [orc.gen_fr(400 + i, 1 << L) for i, (L, _) in enumerate(sizes)]
+    xs = [to_dev(zk, v) for v in vecs]
+    batch = zk.ntt.NttBatch([(x, kind) for x, (_, kind) in zip(xs, sizes)])
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=torch.cuda.Stream()):
+        batch.run()
+    graph.replay()
+    for x, v, (L, kind) in zip(xs, vecs, sizes):
+        expect = {"ntt": lambda: orc.best_fft(v, orc.root_of_unity(L), L), "intt": lambda: orc.intt(v, L),
+                  "coset": lambda: orc.coset_ntt(v, L, L, g)}[kind]()
+        assert np.array_equal(x.numpy_u64(), expect), (L, kind)
+    zk.ntt.status()
