@@ -10,6 +10,7 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -62,7 +63,11 @@ def build_one(name: str, force: bool = False, verbose: bool = False) -> str:
 
 
 def build_all(force: bool = False, verbose: bool = False):
-    out = [build_one(n, force, verbose) for n in LIBS]
+    # side by side, then what links against them
+    first = [n for n in LIBS if n != "libzkp_runtime.so"]
+    with ThreadPoolExecutor(max_workers=len(first)) as pool:
+        out = list(pool.map(lambda n: build_one(n, force, verbose), first))
+    out.append(build_one("libzkp_runtime.so", force, verbose))
     # fused kernels the hot path uses, generated from their graphs (fused.py)
     sys.path.insert(0, os.path.dirname(HERE))
     import importlib
