@@ -1050,6 +1050,8 @@ def emit(args, zk, rank, world, n_msm, n_ntt, ntt_ms, msm_ms, step_ms, pass_ms, 
             "ntt_passes": {"digits": digits, "fr_mults": ntt_mults, "ms": pass_total,
                            "fr_mults_per_s": ntt_mults / (pass_total / 1e3),
                            "frac": (ntt_mults / (pass_total / 1e3)) / shoup_per_s,
+                           "note": "credits the radix-2 transform's products, more than are executed: not a "
+                                   "utilisation",
                            "peak": "shoup_mul_peak_per_s"},
         },
         "e2e": {"value": world * n_msm / e2e_msm_s if e2e_msm_s == e2e_msm_s else None, "unit": "points/s",
