@@ -146,9 +146,9 @@ void zkp_ntt_batch_plan_destroy(ZkpNttBatchPlan *plan);
  * work has run: transforms of the context refuse with cudaErrorTimeout until zkp_ntt_status, called
  * after a synchronisation, has returned it (and cleared it).  cudaSuccess: no wait ran out. */
 cudaError_t zkp_ntt_status(void);
-/* Test support: the first tensor-core pass of a transform of x whose waits give up after `polls` polls (0:
- * at once); vector, table and length as the tensor-core passes need them. */
-cudaError_t zkp_ntt_wait_probe(PolyPtr x, const unsigned int *twiddle, unsigned int log_len, unsigned int polls,
+/* Test support: the first tensor-core pass of a transform of x whose waits give up after `limit_ns`
+ * nanoseconds (0: at once); vector, table and length as the tensor-core passes need them. */
+cudaError_t zkp_ntt_wait_probe(PolyPtr x, const unsigned int *twiddle, unsigned int log_len, unsigned int limit_ns,
                                cudaStream_t stream);
 
 /* Benchmark support: throughput probe of the Shoup twiddle product (blocks x 256 threads x

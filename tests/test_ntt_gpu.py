@@ -468,7 +468,7 @@ def test_wait_that_runs_out_is_reported(zk, orc):
     x, tw = to_dev(zk, a), zk.ntt.twiddle_table(log_n)
     stream = torch.cuda.current_stream().cuda_stream
     zk.ntt.status()
-    assert lib.zkp_ntt_wait_probe(x.poly_ptr(), tw.values.data_ptr(), log_n, 1 << 16, stream) == 0
+    assert lib.zkp_ntt_wait_probe(x.poly_ptr(), tw.values.data_ptr(), log_n, 10**9, stream) == 0
     torch.cuda.synchronize()
     zk.ntt.status()
     assert lib.zkp_ntt_wait_probe(x.poly_ptr(), tw.values.data_ptr(), log_n, 0, stream) == 0

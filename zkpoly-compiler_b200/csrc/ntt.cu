@@ -898,13 +898,13 @@ cudaError_t prepare_umma() {
     ZK_TRY(status_word(true, &word));
     return ensure_smem_attr(ntt_umma_kernel, (int)UM_SMEM, done);
 }
-cudaError_t launch_umma(const PassArgs &a, cudaStream_t stream, u32 polls = UM_POLLS) {
+cudaError_t launch_umma(const PassArgs &a, cudaStream_t stream, u32 limit_ns = UM_WAIT_NS) {
     ZK_TRY(prepare_umma());
     u32 *word = nullptr;
     ZK_TRY(status_word(true, &word));
     const u32 items = 1u << (a.L - UM_D - 7);
     const u32 grid = items < (u32)num_sms() ? items : (u32)num_sms();
-    ntt_umma_kernel<<<grid, UM_GROUPS * 128, UM_SMEM, stream>>>(a, items, polls, word);
+    ntt_umma_kernel<<<grid, UM_GROUPS * 128, UM_SMEM, stream>>>(a, items, limit_ns, word);
     return cudaGetLastError();
 }
 
@@ -1296,7 +1296,7 @@ extern "C" cudaError_t zkp_ntt_status(void) {
 }
 
 extern "C" cudaError_t zkp_ntt_wait_probe(PolyPtr x, const unsigned int *twiddle, unsigned int log_len,
-                                          unsigned int polls, cudaStream_t stream) {
+                                          unsigned int limit_ns, cudaStream_t stream) {
     View v;
     ZK_CHECK_ARG(log_len <= 28 && x.len == (1ull << log_len) && make_view(x, &v));
     ZK_CHECK_ARG(ntt::umma_ok(log_len, v, twiddle));
@@ -1306,7 +1306,7 @@ extern "C" cudaError_t zkp_ntt_wait_probe(PolyPtr x, const unsigned int *twiddle
     a.L = log_len;
     a.D = ntt::UM_D;
     a.lo = log_len - ntt::UM_D;
-    return ntt::launch_umma(a, stream, polls);
+    return ntt::launch_umma(a, stream, limit_ns);
 }
 
 extern "C" cudaError_t zkp_ntt_set_max_digit(unsigned int log_len, unsigned int max_digit) {

@@ -43,10 +43,10 @@ constexpr u32 UM_BAR = UM_A + UM_GROUPS * UM_A_BYTES;  // one mbarrier a group, 
 constexpr u32 UM_SMEM = UM_BAR + 64;
 // D = S32, A and B unsigned bytes, both K-major, N = 128, M = 128
 constexpr u32 UM_IDESC = (2u << 4) | ((UM_COLS >> 3) << 17) | ((UM_ROWS >> 4) << 24);
-// A wait for the tensor core (some microseconds) gives up after this many polls of an mbarrier, each
-// of at most UM_POLL_NS: about a second.  Its group then stores nothing more, waits once more for what is in
-// flight, sets the context's status word (zkp_ntt_status) and leaves.
-constexpr u32 UM_POLLS = 1u << 16, UM_POLL_NS = 16384;
+// A wait for the tensor core (some microseconds) gives up after a second, and whatever the clock says
+// after UM_POLLS polls of an mbarrier.  Its group then stores nothing more, waits once more for what is
+// in flight, sets the context's status word (zkp_ntt_status) and leaves.
+constexpr u32 UM_WAIT_NS = 1000000000u, UM_POLLS = 1u << 24;
 
 ZK_DI u32 um_smem_addr(const void *p) { return (u32)__cvta_generic_to_shared(p); }
 // shared-memory matrix descriptor: no swizzle, K-major; core matrices of 8 rows x 16 bytes,
@@ -65,17 +65,27 @@ ZK_DI void um_mma(u32 tmem, u64 a, u64 b, bool accumulate) {
 ZK_DI void um_commit(u32 bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
-ZK_DI bool um_wait(u32 bar, u32 parity, u32 polls) {
-    for (u32 i = 0; i < polls; i++) {
+ZK_DI u64 um_clock_ns() {
+    u64 t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
+// limit 0: gives up at once
+ZK_DI bool um_wait(u32 bar, u32 parity, u32 limit_ns) {
+    u64 start = 0;
+    for (u32 i = 0; limit_ns && i < UM_POLLS; i++) {
         u32 done;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
             "selp.b32 %0, 1, 0, p;\n\t}\n"
             : "=r"(done)
-            : "r"(bar), "r"(parity), "r"(UM_POLL_NS)
+            : "r"(bar), "r"(parity)
             : "memory");
         if (done) return true;
+        const u64 now = um_clock_ns();
+        if (i == 0) start = now;
+        if (now - start >= limit_ns) break;
     }
     return false;
 }
@@ -208,7 +218,7 @@ ZK_DI void um_pencil(u64 item, u32 row, u32 lo, u32 log_h, u64 &c, u64 &h) {
 // The twiddle product is the Montgomery one also for callers with a Shoup table: these passes wait
 // for loads more than for the multiply pipe, and its root is 32 bytes, not 64 (2^24 2.92 -> 2.83 ms,
 // 2^22 0.752 -> 0.738).
-__global__ void __launch_bounds__(UM_GROUPS * 128, 1) ntt_umma_kernel(const PassArgs a, u32 items, u32 polls,
+__global__ void __launch_bounds__(UM_GROUPS * 128, 1) ntt_umma_kernel(const PassArgs a, u32 items, u32 limit_ns,
                                                                        u32 *status) {
     extern __shared__ __align__(1024) unsigned char um_sm[];
     const u32 tid = threadIdx.x, g = tid >> 7, row = tid & 127;
@@ -275,9 +285,9 @@ __global__ void __launch_bounds__(UM_GROUPS * 128, 1) ntt_umma_kernel(const Pass
         return true;
     };
     auto finish = [&]() {
-        if (!um_wait(bar, parity, polls)) {
+        if (!um_wait(bar, parity, limit_ns)) {
             late = true;
-            um_wait(bar, parity, UM_POLLS);  // still in flight: reads A, writes TMEM
+            um_wait(bar, parity, UM_WAIT_NS);  // still in flight: reads A, writes TMEM
         }
         late = __any_sync(0xffffffffu, late);
         parity ^= 1;
