@@ -24,7 +24,7 @@
 // the digits that vary.  All words are sorted by, least significant first, where they have few varying
 // digits (FEW_DIGITS) or long runs are left after two such rounds.
 // 2^20 rows of random elements take 0.48 ms, a range table of either sign 0.45 (1.14 where all words had
-// to settle it, 0.92 with library sorts), 2^19 or 100 small values among random ones 0.85 / 0.76 (1.51 /
+// to settle it, 0.92 with library sorts), 2^19 or 100 small values among random ones 0.80 / 0.76 (1.51 /
 // 1.55, 0.98 / 1.16).
 #pragma once
 #include <cooperative_groups.h>
@@ -401,6 +401,11 @@ __global__ void __launch_bounds__(CTA, 1) permute_kernel(const Args a) {
         for (u32 i = gt; i < n; i += gs) a.word[s][cur][i] = a.run[s][a.idx[s][cur][i]];
         const u32 most = max(runs0, runs1) - 1;
         sort_digits(most ? 0xffffffffu >> __clz(most) : 0u);
+        if (top0 <= 31 && top1 <= 31) {  // the word held all the bits that were left: no ties
+            for (u32 i = gt; i < n; i += gs) k[i] = a.keys[s][a.idx[s][cur][i]];
+            grid.sync();
+            break;
+        }
     }
     // ---- run starts of the input take a table entry each (any of equal entries)
     const Key *A = a.sorted[0], *T = a.sorted[1];
